@@ -772,21 +772,23 @@ int launch(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t stre
 }
 
 // Tensor maps are pure functions of (pointer, rows, columns, box rows): encoding one costs about a microsecond of host
-// time, and a fused call needs up to four, so each entry point keeps the maps of its last few operand sets.
+// time, and a fused call needs up to four, so each entry point keeps the maps of its last few operand sets. A map is copied
+// out by the call that finds or makes it: the next operand's miss may take over the slot it came from.
 struct MapKey {
   const void* ptr; uint64_t rows, cols; uint32_t box;
   bool operator==(const MapKey& o) const { return ptr == o.ptr && rows == o.rows && cols == o.cols && box == o.box; }
 };
 class MapCache {
  public:
-  const CUtensorMap* get(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box) {
+  bool get(CUtensorMap& out, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box) {
     const MapKey k{ptr, rows, cols, box};
-    for (int i = 0; i < kSlots; ++i) if (valid_[i] && keys_[i] == k) return &maps_[i];
+    for (int i = 0; i < kSlots; ++i) if (valid_[i] && keys_[i] == k) { out = maps_[i]; return true; }
     const int i = next_; next_ = (next_ + 1) % kSlots;
     valid_[i] = false;
-    if (!makeMap(&maps_[i], ptr, rows, cols, box)) return nullptr;
+    if (!makeMap(&maps_[i], ptr, rows, cols, box)) return false;
     keys_[i] = k; valid_[i] = true;
-    return &maps_[i];
+    out = maps_[i];
+    return true;
   }
  private:
   static constexpr int kSlots = 16;
@@ -836,12 +838,10 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   Shape sh{};
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
-  const CUtensorMap* ma = cache.get(A, uint64_t(M), uint64_t(K), kBM);
-  const CUtensorMap* mb = ma ? cache.get(B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) : nullptr;
-  const CUtensorMap* mc = mb ? cache.get(C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32) : nullptr;
-  if (!ma || !mb || !mc) return 1;
   Maps maps{};
-  maps.a = *ma; maps.b = *mb; maps.aLocal = maps.a; maps.c = *mc;
+  if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
+      !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;
+  maps.aLocal = maps.a;
   p.C = static_cast<__nv_bfloat16*>(C);
   p.ldc = epilogue == kEpiSwiglu ? N / 2 : N;
   p.status = status;
@@ -906,14 +906,12 @@ int purlin_tp_ag_gemm(PurlinTpContext* c, const void* xLocal, const void* W, voi
   p.localA = static_cast<const __nv_bfloat16*>(xLocal);
   p.C = static_cast<__nv_bfloat16*>(out); p.ldc = epilogue == kEpiSwiglu ? N / 2 : N;
   // the host cannot know the device epoch (graph replays advance it): pass the maps of both gather buffers
-  const CUtensorMap* m0 = c->maps.get(c->peers[c->rank] + c->gatherOff[0], uint64_t(M), uint64_t(K), kBM);
-  const CUtensorMap* m1 = m0 ? c->maps.get(c->peers[c->rank] + c->gatherOff[1], uint64_t(M), uint64_t(K), kBM) : nullptr;
-  const CUtensorMap* ml = m1 ? c->maps.get(xLocal, uint64_t(M / c->world), uint64_t(K), kBM) : nullptr;
-  const CUtensorMap* mb = ml ? c->maps.get(W, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) : nullptr;
-  const CUtensorMap* mc = mb ? c->maps.get(out, uint64_t(M), uint64_t(p.ldc), 32) : nullptr;
-  if (!mc) return 1;
   Maps maps{};
-  maps.a = *m0; maps.a1 = *m1; maps.aLocal = *ml; maps.b = *mb; maps.c = *mc;
+  if (!c->maps.get(maps.a, c->peers[c->rank] + c->gatherOff[0], uint64_t(M), uint64_t(K), kBM) ||
+      !c->maps.get(maps.a1, c->peers[c->rank] + c->gatherOff[1], uint64_t(M), uint64_t(K), kBM) ||
+      !c->maps.get(maps.aLocal, xLocal, uint64_t(M / c->world), uint64_t(K), kBM) ||
+      !c->maps.get(maps.b, W, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
+      !c->maps.get(maps.c, out, uint64_t(M), uint64_t(p.ldc), 32)) return 1;
   p.gatherParityBytes = c->gatherOff[1] - c->gatherOff[0];
   for (int q = 0; q < c->world; ++q) {
     p.gatherBuf[q] = reinterpret_cast<__nv_bfloat16*>(c->peers[q] + c->gatherOff[0]);
@@ -935,11 +933,9 @@ int purlin_tp_gemm_rs(PurlinTpContext* c, const void* A, const void* W, void* ou
   p.status = reinterpret_cast<uint32_t*>(lb + 256); p.timeoutNs = c->timeoutNs;
   p.C = static_cast<__nv_bfloat16*>(out); p.ldc = N;
   p.partialParityStride = c->partialParityStride;
-  const CUtensorMap* ma = c->maps.get(A, uint64_t(M), uint64_t(K), kBM);
-  const CUtensorMap* mb = ma ? c->maps.get(W, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) : nullptr;
-  if (!mb) return 1;
   Maps maps{};
-  maps.a = *ma; maps.aLocal = maps.a; maps.b = *mb;
+  if (!c->maps.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !c->maps.get(maps.b, W, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas))) return 1;
+  maps.aLocal = maps.a;
   for (int q = 0; q < c->world; ++q) {
     p.partialBuf[q] = reinterpret_cast<__nv_bfloat16*>(c->peers[q] + c->partialOff);
     p.tileReady[q] = reinterpret_cast<uint64_t*>(c->peers[q] + c->tileReadyOff);

@@ -68,3 +68,17 @@ def test_repeated_calls_are_bitwise_stable():
     first = gemm(a, w).clone()
     for _ in range(5):
         assert torch.equal(gemm(a, w), first)
+
+
+def test_one_activation_against_more_weights_than_the_map_cache_holds():
+    # the tensor map of `a` is found in the cache while the weight's is made: every product has to see its own operands
+    from purlin_b200.ops.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a = torch.randint(-2, 3, (256, 128), generator=g, device="cuda").to(torch.bfloat16)
+    ws = [torch.randint(-1, 2, (256, 128), generator=g, device="cuda").to(torch.bfloat16) for _ in range(20)]
+    outs = [torch.empty(256, 256, device="cuda", dtype=torch.bfloat16) for _ in ws]
+    for _ in range(2):
+        for w, out in zip(ws, outs):
+            gemm(a, w, out)
+    for w, out in zip(ws, outs):
+        assert torch.equal(out.float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())

@@ -15,9 +15,9 @@
 //             released when its rows are on their way. Receiver CTAs of the same kernel wait on those chunk flags
 //             and copy every staged row to its expert rows (local HBM traffic): the permute is that address
 //             computation. Rows for this rank's own experts skip the staging area.
-//   combine   pusher CTAs on the experts' GPU form, for every staged row, the gate-weighted sum of its expert
-//             outputs (fp32) and store ONE row into the token's home GPU, chunk flags as above; finisher CTAs on
-//             the home GPU add the rows of a token's destinations as their chunks arrive.
+//   combine   pusher CTAs on the experts' GPU form, for every row staged by another rank, the gate-weighted sum of its
+//             expert outputs (fp32) and store ONE row into the token's home GPU, chunk flags as above; finisher CTAs on
+//             the home GPU add these rows, as their chunks arrive, to the token's expert rows on this GPU.
 //
 // Buffer reuse needs no extra handshake as long as dispatch and combine alternate on one stream (they are two halves
 // of a layer): a rank writes into a peer's staging or combine buffers only after it has seen that peer's counts of the
@@ -60,7 +60,8 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kDispatchCtasPerSm = 2;   // the dispatch is bound by memory latency and light on registers: two CTAs of eight warps per SM
-constexpr int kCombineCtasPerSm = 1;    // the weighted sums keep 8 x 32 bytes per lane in flight and need the registers
+constexpr int kCombineCtasPerSm = 1;    // with peers; the weighted sums keep 8 x 32 bytes per lane in flight
+constexpr int kCombineCtasPerSmAlone = 2;   // a world of one: all CTAs read expert rows, which is bound by bytes in flight
 constexpr int kMaxExperts = 512;
 constexpr int kChunkRows = 64;          // rows per flag
 constexpr int kRecvRows = 16;           // rows per receiver item of the dispatch (a part of a chunk)
@@ -191,6 +192,7 @@ PURLIN_D void copyRow(unsigned char* dst, const unsigned char* src, int vecs, in
 __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(const __grid_constant__ MoeParams p) {
   __shared__ int32_t rowBase[kMaxExperts];      // first row of (this rank, expert e) inside the destination's buffer
   __shared__ int32_t colTotal[kMaxExperts];     // rows of expert e over all ranks
+  __shared__ int32_t upTo[kMaxExperts], blockSum[kMaxExperts / 32];
   __shared__ int32_t sendCount[kMaxRanks], recvFrom[kMaxRanks];
   __shared__ int bad, nextItem;
   const uint64_t epoch = sig::ldRelaxedSys(p.epoch) + 1;
@@ -204,51 +206,55 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
   if (outOfOrder && tid == 0) { bad = 1; reportBad(p, 9, 0); }
 
   // 1. publish this rank's counts on every rank (flagged stores; the flag is released after the data)
-  if (blockIdx.x == 0 && !outOfOrder) {
+  if (blockIdx.x == 0 && !outOfOrder && W > 1) {
     for (int q = 0; q < W; ++q)
       for (int e = tid; e < stride; e += blockDim.x) p.countsAll[q][size_t(p.rank) * stride + e] = p.localCounts[e];
     __syncthreads();
     if (tid < W) sig::stReleaseSys(p.flags[tid] + p.rank, epoch);
   }
-  // 2. everyone's counts are here
+  // 2. everyone's counts are here (a world of one has them from its own plan)
   int okI = outOfOrder ? 0 : 1;
-  if (!outOfOrder && tid < W) okI = waitFlag(p, p.flags[p.rank] + tid, epoch, 1, tid) ? 1 : 0;
+  if (!outOfOrder && W > 1 && tid < W) okI = waitFlag(p, p.flags[p.rank] + tid, epoch, 1, tid) ? 1 : 0;
   bool ok = __syncthreads_and(okI) != 0;
-  // 3. where my rows go: expert-major on the destination, sources in rank order inside an expert
-  const uint32_t* all = p.countsAll[p.rank];
-  int before = 0;
-  for (int e = tid; ok && e < p.experts; e += blockDim.x) {
-    int tot = 0;
+  // 3. where my rows go: expert-major on the destination, sources in rank order inside an expert. The running sums over the
+  // experts are scans (32 experts per warp step): every CTA needs them before its first row, and one thread adding 256
+  // counters in turn took several microseconds of every call.
+  const uint32_t* all = W > 1 ? p.countsAll[p.rank] : p.localCounts;
+  for (int e0 = warp * 32; ok && e0 < p.experts; e0 += kWarps * 32) {
+    const int e = e0 + lane;
+    int tot = 0, before = 0;
     for (int s = 0; s < W; ++s) { const int c = int(all[size_t(s) * stride + e]); tot += c; if (s < p.rank) before += c; }
+    int sum = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
     colTotal[e] = tot;
+    rowBase[e] = before;
+    upTo[e] = sum;                                  // inclusive, inside the block of 32
+    if (lane == 31) blockSum[e0 / 32] = sum;
   }
   if (ok && tid < W) { sendCount[tid] = int(p.localCounts[p.experts + tid]); recvFrom[tid] = int(all[size_t(tid) * stride + p.experts + p.rank]); }
   __syncthreads();
-  for (int e = tid; ok && e < p.experts; e += blockDim.x) {
-    // (with experts <= blockDim.x a thread owns one expert, so `before` belongs to e; with more it is recomputed)
-    int b = 0;
-    if (p.experts > int(blockDim.x)) { for (int s = 0; s < p.rank; ++s) b += int(all[size_t(s) * stride + e]); } else b = before;
-    const int first = e / p.expertsPerRank * p.expertsPerRank;
-    for (int e2 = first; e2 < e; ++e2) b += colTotal[e2];
-    rowBase[e] = b;
-  }
+  auto rowsBefore = [&](int e) {                    // rows of all experts below e
+    int v = upTo[e] - colTotal[e];
+    for (int k = 0; k < e / 32; ++k) v += blockSum[k];
+    return v;
+  };
+  auto rowsOnRank = [&](int r) {                    // rows that rank r receives
+    const int last = (r + 1) * p.expertsPerRank - 1;
+    return rowsBefore(last) + colTotal[last] - rowsBefore(r * p.expertsPerRank);
+  };
+  for (int e = tid; ok && e < p.experts; e += blockDim.x) rowBase[e] += rowsBefore(e) - rowsBefore(e / p.expertsPerRank * p.expertsPerRank);
   // Capacity is judged on the whole count matrix, which every rank holds: if any destination would receive more rows
   // than its buffer has, every rank sees it, every rank reports it and nobody stores a row.
   if (ok && tid < W) {
-    long total = 0;
-    for (int e = tid * p.expertsPerRank; e < (tid + 1) * p.expertsPerRank; ++e) total += long(colTotal[e]);
-    if (total > long(p.capacityRows)) { bad = 1; reportBad(p, 2, uint32_t(tid)); }
+    if (rowsOnRank(tid) > p.capacityRows) { bad = 1; reportBad(p, 2, uint32_t(tid)); }
     if (sendCount[tid] > p.maxTokens || recvFrom[tid] > p.maxTokens) { bad = 1; reportBad(p, 3, uint32_t(tid)); }
   }
   __syncthreads();
   if (blockIdx.x == 0 && ok) {
     // what this rank receives: rows per local expert and their total
     for (int e = tid; e < p.expertsPerRank; e += blockDim.x) p.recvCounts[e] = bad ? 0 : colTotal[p.rank * p.expertsPerRank + e];
-    if (tid == 0) {
-      int total = 0;
-      for (int e = 0; e < p.expertsPerRank; ++e) total += colTotal[p.rank * p.expertsPerRank + e];
-      p.recvCounts[p.expertsPerRank] = bad ? 0 : total;
-    }
+    if (tid == 0) p.recvCounts[p.expertsPerRank] = bad ? 0 : rowsOnRank(p.rank);
   }
   const int vecs = p.hiddenBytes / 32;
   const size_t rowBytes = size_t(p.hiddenBytes);
@@ -301,61 +307,72 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
         }
       }
     } else {
-      // 4b. receiver: every row that belongs on this rank goes to its expert rows (local traffic). Rows of this rank's
-      // own tokens come straight from x; a peer's rows are copied out of the staging area as its chunks land.
-      int item = 0, want = grab(p.work + 1);
-      for (int c = 0; c < p.maxChunks && ok; ++c) {
-        for (int ss = 0; ss < W && ok; ++ss) {
-          const int s = (p.rank + W - ss) % W;          // own rows first, then the rank that serves this one first
-          const int count = s == p.rank ? sendCount[s] : recvFrom[s];
+      // 4b. receiver: every row that belongs on this rank goes to its expert rows (local traffic): the row is read once and
+      // written to each of them.
+      auto fanOut = [&](const unsigned char* src, int row, int begin, int end) {   // lanes 0..7 hold the rows; 32-byte pieces [begin, end)
+        unsigned char* dst[8];
+        unsigned mask = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = __shfl_sync(0xffffffffu, row, k);
+          const bool valid = r >= 0 && r < p.capacityRows;
+          dst[k] = p.recvBuf + size_t(valid ? r : 0) * rowBytes;
+          if (valid) mask |= 1u << k;
+        }
+        for (int i = begin + lane; i < end; i += 32 * 8) {
+          Vec32 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) if (i + u * 32 < end) v[u] = ld32(src + size_t(i + u * 32) * 32);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if ((mask >> k) & 1u) {
+#pragma unroll
+              for (int u = 0; u < 8; ++u) if (i + u * 32 < end) st32(dst[k] + size_t(i + u * 32) * 32, v[u]);
+            }
+        }
+      };
+      // Rows of this rank's own tokens come straight from x. They are one list of 1 KiB pieces, cut evenly over the receivers'
+      // warps, whatever the number of rows. Handed out in items of 16 rows, 4096 rows were 256 items for 296 CTAs and 16
+      // rows kept one SM busy. One B200, top-8: 4096 x 7168 of 256 experts 139 -> 101 us (5.2 TB/s), 128 x 7168 of 32
+      // experts 71 -> 10 us (the scans above included).
+      {
+        const int receivers = int(gridDim.x) - senders, me = int(blockIdx.x) - senders;
+        const int perRow = (vecs + 31) / 32;
+        const int64_t pieces = int64_t(sendCount[p.rank]) * perRow, nw = int64_t(receivers) * kWarps, w = int64_t(warp) * receivers + me;
+        int64_t u = pieces * w / nw;
+        const int64_t stop = pieces * (w + 1) / nw;
+        while (u < stop) {
+          const int pp = int(u / perRow), first = int(u % perRow);
+          const int n = int(min(int64_t(perRow - first), stop - u));
+          const int t = p.sendList[size_t(p.rank) * p.maxTokens + pp];
+          int row;
+          const int rec = recordOf(t, p.rank, row);
+          // the combine reads the record like a peer's
+          if (first == 0 && lane < kMetaWords) p.meta[p.rank][(size_t(p.rank) * p.maxTokens + pp) * kMetaWords + lane] = rec;
+          fanOut(p.x + size_t(t) * rowBytes, row, first * 32, min((first + n) * 32, vecs));
+          u += n;
+        }
+      }
+      // A peer's rows are copied out of the staging area as its chunks land. A receiver's item is a part of a chunk (kRecvRows
+      // rows, two per warp): a whole chunk per CTA made the last chunk to land a 50 us tail.
+      int item = 0, want = W > 1 ? grab(p.work + 1) : 0;
+      for (int c = 0; c < p.maxChunks && ok && W > 1; ++c) {
+        for (int ss = 1; ss < W && ok; ++ss) {
+          const int s = (p.rank + W - ss) % W;          // the rank that serves this one first comes first
+          const int count = recvFrom[s];
           if (c * kChunkRows >= count) continue;
-          // A receiver's item is a part of a chunk (kRecvRows rows, two per warp): a whole chunk per CTA left most CTAs
-          // without work (4096 local rows are 64 chunks for 296 CTAs) and made the last chunk to land a 50 us tail.
           for (int part = 0; part < kChunkRows / kRecvRows && ok; ++part) {
             const int begin = c * kChunkRows + part * kRecvRows;
             if (begin >= count) break;
             if (item++ != want) continue;
-            if (s != p.rank) {
-              int good = 1;
-              if (tid == 0) good = waitFlag(p, dispatchFlag(p, p.rank, s, c), epoch, 3, s) ? 1 : 0;
-              ok = __syncthreads_and(good) != 0;
-              if (!ok) break;
-            }
+            int good = 1;
+            if (tid == 0) good = waitFlag(p, dispatchFlag(p, p.rank, s, c), epoch, 3, s) ? 1 : 0;
+            ok = __syncthreads_and(good) != 0;
+            if (!ok) break;
             const int end = min(begin + kRecvRows, count);
             for (int pp = begin + warp; pp < end; pp += kWarps) {
               const size_t at = size_t(s) * p.maxTokens + pp;
-              int row;
-              const unsigned char* src;
-              if (s == p.rank) {
-                const int t = p.sendList[size_t(s) * p.maxTokens + pp];
-                const int rec = recordOf(t, s, row);
-                if (lane < kMetaWords) p.meta[s][at * kMetaWords + lane] = rec;      // the combine reads it like a peer's
-                src = p.x + size_t(t) * rowBytes;
-              } else {
-                row = lane < 8 ? p.meta[p.rank][at * kMetaWords + lane] : -1;
-                src = p.stage[p.rank] + at * rowBytes;
-              }
-              // the row is read once and written to each of its expert rows
-              unsigned char* dst[8];
-              unsigned mask = 0;
-  #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const int r = __shfl_sync(0xffffffffu, row, k);
-                const bool valid = r >= 0 && r < p.capacityRows;
-                dst[k] = p.recvBuf + size_t(valid ? r : 0) * rowBytes;
-                if (valid) mask |= 1u << k;
-              }
-              for (int i = lane; i < vecs; i += 32 * 8) {
-                Vec32 v[8];
-  #pragma unroll
-                for (int u = 0; u < 8; ++u) if (i + u * 32 < vecs) v[u] = ld32(src + size_t(i + u * 32) * 32);
-  #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  if ((mask >> k) & 1u) {
-  #pragma unroll
-                    for (int u = 0; u < 8; ++u) if (i + u * 32 < vecs) st32(dst[k] + size_t(i + u * 32) * 32, v[u]);
-                  }
-              }
+              fanOut(p.stage[p.rank] + at * rowBytes, lane < 8 ? p.meta[p.rank][at * kMetaWords + lane] : -1, 0, vecs);
             }
             want = grab(p.work + 1);
           }
@@ -386,10 +403,10 @@ PURLIN_D uint32_t packBf16x2(float lo, float hi) {
 // out = sum of w[k] * rows[k] over the first n of R rows (fp32 accumulate). 32-byte accesses, P positions of every row
 // in flight per lane: R x P = 8 loads of 32 bytes, whatever the number of rows, because the sum is latency-bound
 // otherwise (16 in flight spilled).
-// n is the same in every lane, so the branches are uniform and the arrays stay in registers. rowBytes % 32 == 0.
+// 32-byte pieces [begin, vecs32). n is the same in every lane, so the branches are uniform and the arrays stay in registers. rowBytes % 32 == 0.
 template <int R, int P>
-PURLIN_D void weightedSum(unsigned char* out, const unsigned char* const (&rows)[8], const float (&w)[8], int n, int vecs32, int lane) {
-  for (int i = lane; i < vecs32; i += 32 * P) {
+PURLIN_D void weightedSum(unsigned char* out, const unsigned char* const (&rows)[8], const float (&w)[8], int n, int begin, int vecs32, int lane) {
+  for (int i = begin + lane; i < vecs32; i += 32 * P) {
     Vec32 v[P][R];
 #pragma unroll
     for (int h = 0; h < P; ++h)
@@ -416,13 +433,13 @@ PURLIN_D void weightedSum(unsigned char* out, const unsigned char* const (&rows)
   }
 }
 // the rows of a sum arrive in arbitrary lanes; few rows take many positions each, many rows few
-PURLIN_D void weightedSumAny(unsigned char* out, const unsigned char* const (&rows)[8], const float (&w)[8], int n, int vecs32, int lane) {
-  if (n <= 2) weightedSum<2, 4>(out, rows, w, n, vecs32, lane);
-  else if (n <= 4) weightedSum<4, 2>(out, rows, w, n, vecs32, lane);
-  else weightedSum<8, 1>(out, rows, w, n, vecs32, lane);
+PURLIN_D void weightedSumAny(unsigned char* out, const unsigned char* const (&rows)[8], const float (&w)[8], int n, int begin, int vecs32, int lane) {
+  if (n <= 2) weightedSum<2, 4>(out, rows, w, n, begin, vecs32, lane);
+  else if (n <= 4) weightedSum<4, 2>(out, rows, w, n, begin, vecs32, lane);
+  else weightedSum<8, 1>(out, rows, w, n, begin, vecs32, lane);
 }
 
-__global__ void __launch_bounds__(kThreads, kCombineCtasPerSm) combineKernel(const __grid_constant__ MoeParams p) {
+__global__ void __launch_bounds__(kThreads, kCombineCtasPerSmAlone) combineKernel(const __grid_constant__ MoeParams p) {
   __shared__ int32_t recvFrom[kMaxRanks];
   __shared__ int bad, nextItem;
   const uint64_t epoch = sig::ldRelaxedSys(p.epoch + 1) + 1;
@@ -439,9 +456,9 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSm) combineKernel(con
   const bool ok = __syncthreads_and(!bad && sig::ldRelaxedGpu32(p.status) == 0u) != 0;   // one answer for the whole CTA: the roles below hold barriers
   const int vecs32 = p.hiddenBytes / 32;
   const size_t rowBytes = size_t(p.hiddenBytes);
-  const int senders = p.senders < int(gridDim.x) ? p.senders : int(gridDim.x) - 1;
+  const int senders = W == 1 ? 0 : (p.senders < int(gridDim.x) ? p.senders : int(gridDim.x) - 1);
   if (ok && int(blockIdx.x) < senders) {
-    // A. pusher: for every row staged here by rank s, the gate-weighted sum of its expert outputs goes home as ONE row.
+    // A. pusher: for every row staged here by another rank s, the gate-weighted sum of its expert outputs goes home as ONE row.
     // Items (one chunk of one source) are handed out through a counter in chunk order: the pushers end together, and the
     // chunks complete in the order in which the finishers at home need them (a static split of 232 items over 98 CTAs
     // had the last pusher end at 313 us and the first at 187 us, and left a third of the finishers' work for the end).
@@ -453,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSm) combineKernel(con
     };
     int item = 0, want = grab();
     for (int c = 0; c < p.maxChunks; ++c) {
-      for (int ss = 0; ss < W; ++ss) {
+      for (int ss = 0; ss + 1 < W; ++ss) {
         const int s = (p.rank + 1 + ss) % W;
         if (c * kChunkRows >= recvFrom[s]) continue;
         if (item++ != want) continue;
@@ -475,40 +492,68 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSm) combineKernel(con
             w[j] = __int_as_float(__shfl_sync(0xffffffffu, rec, 8 + from));
             rows[j] = p.outBuf + size_t(j < n ? r : 0) * rowBytes;
           }
-          weightedSumAny(p.cbuf[s] + (size_t(p.rank) * p.maxTokens + pp) * rowBytes, rows, w, n, vecs32, lane);
+          weightedSumAny(p.cbuf[s] + (size_t(p.rank) * p.maxTokens + pp) * rowBytes, rows, w, n, 0, vecs32, lane);
         }
         want = grab();                  // (its first barrier also orders the rows before the flag)
         if (tid == 0) sig::stReleaseSys(combineFlag(p, s, p.rank, c), epoch);
       }
     }
   } else if (ok) {
-    // B. finisher: a token's result is the sum of one row per destination GPU, added as their chunks arrive
+    // B. finisher: a token's result is the gate-weighted sum of its expert rows on this rank, read where the experts wrote
+    // them, and of one finished row per other destination GPU, added as their chunks arrive. Bound by the read of the expert
+    // rows; this rank's own share does not go through the return buffer, where a pusher would write it as a bf16 row to be
+    // read again. One B200, top-8: 4096 x 7168 189 -> 110 us (4.8 TB/s), 128 x 7168 119 -> 11 us.
     const int nFin = int(gridDim.x) - senders, me = int(blockIdx.x) - senders;
-    for (int t = me * kWarps + warp; t < p.tokens; t += nFin * kWarps) {
-      int d = -1 - lane, pos = -1;
+    auto finish = [&](int t, int begin, int end) {     // 32-byte pieces [begin, end) of token t
+      int d = -1 - lane, pos = -1, ownRow = -1;
+      float weight = 1.f;
       if (lane < p.topk) {
         const int e = p.topkIdx[size_t(t) * p.topk + lane];
         pos = p.pos[size_t(t) * p.topk + lane];
         if (e >= 0 && e < p.experts && pos >= 0) d = e / p.expertsPerRank;
+        if (d == p.rank) {
+          ownRow = p.meta[p.rank][(size_t(p.rank) * p.maxTokens + pos) * kMetaWords + lane];
+          weight = __int_as_float(p.meta[p.rank][(size_t(p.rank) * p.maxTokens + pos) * kMetaWords + 8 + lane]);
+        }
       }
       const unsigned same = __match_any_sync(0xffffffffu, d);
-      const bool leader = d >= 0 && (__ffs(same) - 1) == lane;
+      const bool remote = d >= 0 && d != p.rank && (__ffs(same) - 1) == lane;
       int good = 1;
-      if (leader) good = waitFlag(p, combineFlag(p, p.rank, d, pos / kChunkRows), epoch, 4, d) ? 1 : 0;
-      if (!__all_sync(0xffffffffu, good)) break;
+      if (remote) good = waitFlag(p, combineFlag(p, p.rank, d, pos / kChunkRows), epoch, 4, d) ? 1 : 0;
+      if (!__all_sync(0xffffffffu, good)) return false;
       __syncwarp();
-      const unsigned leaders = __ballot_sync(0xffffffffu, leader) & 0xffu;
-      const int n = __popc(leaders);
+      const bool own = ownRow >= 0 && ownRow < p.capacityRows;
+      const unsigned parts = __ballot_sync(0xffffffffu, own || remote) & 0xffu;
+      const uint64_t at = own ? uint64_t(reinterpret_cast<uintptr_t>(p.outBuf + size_t(ownRow) * rowBytes))
+                              : uint64_t(reinterpret_cast<uintptr_t>(p.cbuf[p.rank] + (size_t(remote ? d : 0) * p.maxTokens + (remote ? pos : 0)) * rowBytes));
+      const int n = __popc(parts);
       const unsigned char* rows[8];
       float w[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int from = j < n ? int(__fns(leaders, 0, j + 1)) : 0;
-        const int dk = __shfl_sync(0xffffffffu, d, from), pk = __shfl_sync(0xffffffffu, pos, from);
-        rows[j] = p.cbuf[p.rank] + (size_t(j < n ? dk : 0) * p.maxTokens + (j < n ? pk : 0)) * rowBytes;
-        w[j] = 1.f;
+        const int from = j < n ? int(__fns(parts, 0, j + 1)) : 0;
+        rows[j] = reinterpret_cast<const unsigned char*>(uintptr_t(__shfl_sync(0xffffffffu, at, from)));
+        w[j] = __shfl_sync(0xffffffffu, weight, from);
       }
-      weightedSumAny(p.y + size_t(t) * rowBytes, rows, w, n, vecs32, lane);
+      weightedSumAny(p.y + size_t(t) * rowBytes, rows, w, n, begin, end, lane);
+      return true;
+    };
+    if (W == 1) {
+      // nothing to wait for: the output is one list of 1 KiB pieces, cut evenly over the warps of the grid
+      const int perRow = (vecs32 + 31) / 32;
+      const int64_t pieces = int64_t(p.tokens) * perRow, nw = int64_t(nFin) * kWarps, wi = int64_t(warp) * nFin + me;
+      int64_t u = pieces * wi / nw;
+      const int64_t stop = pieces * (wi + 1) / nw;
+      while (u < stop) {
+        const int t = int(u / perRow), first = int(u % perRow);
+        const int m = int(min(int64_t(perRow - first), stop - u));
+        finish(t, first * 32, min((first + m) * 32, vecs32));
+        u += m;
+      }
+    } else {
+      // in token order over the warps, which is about the order in which the chunks arrive
+      for (int t = me * kWarps + warp; t < p.tokens; t += nFin * kWarps)
+        if (!finish(t, 0, vecs32)) break;
     }
   }
   __syncthreads();
@@ -714,11 +759,11 @@ int purlin_moe_combine(PurlinMoeContext* c, void* y, int tokens, const int32_t* 
   MoeParams p{};
   fillCommon(p, c, tokens);
   p.y = static_cast<unsigned char*>(y);
-  const int grid = smCount() * kCombineCtasPerSm;
-  // The pushers read every expert output row, the finishers add at most `world` rows per token, and it is the finishers
-  // that end last: measured at 4 GPUs (4096 tokens, hidden 7168, top-8 of 256), 80 pushers of 148 CTAs 343 us, 98 pushers
-  // 366 us, 110 pushers 392 us.
-  p.senders = blocks > 0 ? std::min(blocks, grid - 1) : std::max(grid * 54 / 100, 1);
+  const int grid = smCount() * (c->world == 1 ? kCombineCtasPerSmAlone : kCombineCtasPerSm);
+  // With the own share pushed too, 80 pushers of 148 CTAs were the best at 4 GPUs (4096 tokens, hidden 7168, top-8 of 256:
+  // 343 us; 98 pushers 366 us, 110 pushers 392 us): the finishers end last. The pushers now have (W - 1) / W of that work and
+  // the finishers the rest, so their number shrinks with it (bytes per CTA as measured; not timed again on several GPUs).
+  p.senders = blocks > 0 ? std::min(blocks, grid - 1) : std::max(grid * 54 * (c->world - 1) / (100 * c->world), 1);
   combineKernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { setError(std::string("combine launch: ") + cudaGetErrorString(e)); return 1; }

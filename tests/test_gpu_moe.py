@@ -17,6 +17,15 @@ def test_moe_world_of_one():
     assert not fails, fails
 
 
+@pytest.mark.parametrize("tokens,hidden,experts,topk", [(1, 16, 32, 1), (1, 7168, 32, 8), (3, 1040, 64, 3), (300, 528, 512, 8), (2371, 48, 256, 2)])
+def test_exchange_pieces(tokens, hidden, experts, topk):
+    # rows are cut into 1 KiB pieces over all warps: one piece in all, a remainder of a piece, fewer and more pieces than warps
+    sys.path.insert(0, HERE)
+    from moe_worker import run
+    fails = run(0, 1, torch.device("cuda", 0), tokens=tokens, hidden=hidden, experts=experts, topk=topk, iters=2)
+    assert not fails, fails
+
+
 @pytest.mark.multigpu
 def test_moe_all_gpus():
     n = torch.cuda.device_count()

@@ -40,6 +40,7 @@
 #include "purlin/atom.cuh"
 #include "purlin/constants.hpp"
 #include "purlin/gemm.h"
+#include "purlin/gemm_skinny.cuh"
 #include "purlin/layout.hpp"
 #include "purlin/tc_sm100.cuh"
 #include "purlin/telemetry.hpp"
@@ -798,6 +799,67 @@ class MapCache {
   int next_ = 0;
 };
 
+// ---- few rows of activations (or of weights): gemm_skinny.cuh ----
+int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* status, cudaStream_t stream) {
+  const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
+  if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
+  skinny::Params p{};
+  // Few rows of W against many rows of X (a router): the operands change places and the output row is the MMA's row.
+  const bool tokenRows = epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens;
+  if (tokenRows) { std::swap(A, B); std::swap(M, N); }
+  p.N = N; p.K = K; p.tokens = M; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
+  p.status = status;
+  p.timeoutNs = 2ull * 1000 * 1000 * 1000;
+  p.tokenBox = M <= 16 ? 16 : 32;
+  p.passTokens = std::min(int(roundUp(size_t(M), size_t(p.tokenBox))), skinny::kMaxTokens);
+  // up to 128 columns two CTAs share an SM (128 columns: 3 stages of 32 KiB each)
+  const int stageBytes = skinny::kWBytes + p.passTokens * skinny::kK * 2;
+  const int perSm = p.passTokens <= 128 ? 2 : 1;
+  const int budget = (perSm == 2 ? 113 : 227) * 1024 - 1024 - skinny::kBarrierBytes;
+  p.stages = std::min(budget / stageBytes, skinny::kMaxStages);
+  for (p.tmemCols = 32; p.tmemCols < p.passTokens; p.tmemCols *= 2) {}
+  // Split k until the CTAs fill three quarters of the places on the GPU and a part keeps at least four k-blocks. Measured,
+  // 1 x 8192 x 3584: one CTA per tile 20.1 us, two 14.4, four 14.2, eight 18.2; 64 x 8192 x 28672: 142.6 / 87.4 / 79.1 /
+  // 90.5 us. At most 15 clusters of eight fit on the GPU at once, so eight are used for no more tiles than that.
+  const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
+  const long slots = long(smCount()) * perSm;
+  int split = 1;
+  while (split < (tiles <= 15 ? skinny::kMaxSplit : 4) && long(tiles) * split * 4 < slots * 3 && kBlocks >= 8 * split) split *= 2;
+  skinny::Maps maps{};
+  if (!cache.get(maps.w, B, uint64_t(N), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
+  const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;
+  auto kernel = tokenRows ? skinny::skinnyGemmKernel<skinny::kTokenRows>
+              : epilogue == kEpiSwiglu ? skinny::skinnyGemmKernel<skinny::kWeightRowsSwiglu> : skinny::skinnyGemmKernel<skinny::kWeightRows>;
+  static std::mutex mu;
+  static bool optedIn[64][3] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) { setError("GEMM launch: no current device"); return 1; }
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    bool& done = optedIn[device][mode];
+    if (!done && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess) { setError("cannot opt in to 227 KiB of shared memory"); return 1; }
+    done = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(split); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(unsigned(tiles * split)); cfg.blockDim = dim3(skinny::kThreads);
+  cfg.dynamicSmemBytes = size_t(p.stages) * stageBytes + skinny::kBarrierBytes + 1024; cfg.stream = stream;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
+  if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
+  return 0;
+}
+
+// Where the few-rows kernel is the better one (one B200, us, it / the tiles of this file): always up to 64 rows (64 x 57344 x
+// 8192 153 / 165, 48 x 4096 x 4096 14 / 22); up to 128 rows while W has too few rows to give every SM a tile of its own and k is
+// worth splitting (128 x 8192 x 7168 31.5 / 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 14336 x
+// 4096 28.2 / 27.4 and 128 x 264 x 72 7.4 / 5.3); few rows of W (4096 x 32 x 7168 11 / 75).
+bool useSkinny(int M, int N, int K, int epilogue) {
+  if (M > skinny::kMaxTokens / 2) return epilogue == kEpiStore && N <= skinny::kMaxTokens;
+  return M <= 64 || (N <= 8192 && K >= 1024);
+}
+
 }  // namespace
 
 struct PurlinTpContext {
@@ -838,6 +900,7 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   Shape sh{};
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
+  if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, status, static_cast<cudaStream_t>(stream));
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
       !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;

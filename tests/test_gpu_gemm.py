@@ -82,3 +82,38 @@ def test_one_activation_against_more_weights_than_the_map_cache_holds():
             gemm(a, w, out)
     for w, out in zip(ws, outs):
         assert torch.equal(out.float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+def _small_integers(m, n, k, seed):
+    # every partial sum is exact in fp32, whatever the order, so the bf16 result is one value
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    a = torch.randint(-2, 3, (m, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randint(-1, 2, (n, k), generator=g, device="cuda").to(torch.bfloat16)
+    return a, w
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 136, 72), (15, 264, 200), (16, 1024, 64), (17, 128, 520), (33, 640, 1024), (64, 4096, 4096),
+                                    (65, 2048, 1096), (96, 384, 2048), (128, 1024, 4096)])
+def test_few_rows_are_exact_on_small_integers(m, n, k):
+    # tiles of 128 weight rows with and without a remainder, one to eight k-splits, one column up to a full pass
+    from purlin_b200.ops.gemm import gemm
+    a, w = _small_integers(m, n, k, 11)
+    assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 8, 64), (300, 32, 1024), (4096, 64, 512), (1000, 256, 136), (257, 248, 72)])
+def test_few_weight_rows_are_exact_on_small_integers(m, n, k):
+    # a router's shape: the tokens are the rows of the tile
+    from purlin_b200.ops.gemm import gemm
+    a, w = _small_integers(m, n, k, 12)
+    assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("m,i,k", [(1, 16, 72), (16, 80, 128), (100, 3584, 512), (300, 528, 200), (777, 1024, 256), (1000, 7168, 64)])
+def test_swiglu_at_odd_sizes(m, i, k):
+    from purlin_b200.ops.gemm import gemm_swiglu, interleave_gate_up
+    a, wg, wu = _rand(m, k, 3), _rand(i, k, 4, 0.05), _rand(i, k, 5, 0.05)
+    out = gemm_swiglu(a, interleave_gate_up(wg, wu)).float()
+    ref = torch.nn.functional.silu(a.float() @ wg.float().t()) * (a.float() @ wu.float().t())
+    # one rounding to bf16 (2^-9 relative) on top of fp32 sums; the absolute term covers cancellation at K <= 512 of unit values
+    assert ((out - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()

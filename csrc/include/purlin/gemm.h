@@ -16,6 +16,12 @@ enum { PURLIN_EPI_STORE = 0, PURLIN_EPI_SWIGLU = 1 };
 int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int bn,
                      uint32_t* status, void* stream);
 
+/* The same product per group of rows: expert e owns counts[e] consecutive rows of A and C and rows [e * N, (e + 1) * N)
+ * of B. counts: device words, read by the kernel (no host synchronisation); rows: rows of A and C, an upper bound of the sum
+ * of the counts. likelyRows: rows a group is expected to have (a hint for speed; any counts are computed). */
+int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, int experts, int N, int K, const int32_t* counts,
+                             int likelyRows, int epilogue, void* stream);
+
 typedef struct PurlinTpContext PurlinTpContext;
 
 /* Bytes of symmetric memory one rank needs for the fused kernels at these maximum shapes:

@@ -40,6 +40,7 @@
 #include "purlin/atom.cuh"
 #include "purlin/constants.hpp"
 #include "purlin/gemm.h"
+#include "purlin/gemm_ragged.cuh"
 #include "purlin/gemm_skinny.cuh"
 #include "purlin/layout.hpp"
 #include "purlin/tc_sm100.cuh"
@@ -799,19 +800,27 @@ class MapCache {
   int next_ = 0;
 };
 
+struct GroupedArgs {
+  int experts = 1;                    // groups of rows; 1 with counts == nullptr: a plain GEMM
+  const int32_t* counts = nullptr;    // device: rows of every group
+  int likelyRows = 0;                 // rows a group is expected to have
+};
+
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
-int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* status, cudaStream_t stream) {
+int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
   if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
   skinny::Params p{};
   // Few rows of W against many rows of X (a router): the operands change places and the output row is the MMA's row.
-  const bool tokenRows = epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens;
+  const bool tokenRows = !g.counts && epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens;
   if (tokenRows) { std::swap(A, B); std::swap(M, N); }
-  p.N = N; p.K = K; p.tokens = M; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
+  p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status;
   p.timeoutNs = 2ull * 1000 * 1000 * 1000;
-  p.tokenBox = M <= 16 ? 16 : 32;
-  p.passTokens = std::min(int(roundUp(size_t(M), size_t(p.tokenBox))), skinny::kMaxTokens);
+  // one pass has to hold a group's rows (a second pass reads W again): a group of average size has twice the room
+  const int room = std::min(g.counts ? 2 * g.likelyRows + 16 : M, M);
+  p.tokenBox = room <= 16 ? 16 : 32;
+  p.passTokens = std::min(int(roundUp(size_t(room), size_t(p.tokenBox))), skinny::kMaxTokens);
   // up to 128 columns two CTAs share an SM (128 columns: 3 stages of 32 KiB each)
   const int stageBytes = skinny::kWBytes + p.passTokens * skinny::kK * 2;
   const int perSm = p.passTokens <= 128 ? 2 : 1;
@@ -824,9 +833,9 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
   const long slots = long(smCount()) * perSm;
   int split = 1;
-  while (split < (tiles <= 15 ? skinny::kMaxSplit : 4) && long(tiles) * split * 4 < slots * 3 && kBlocks >= 8 * split) split *= 2;
+  while (split < (long(tiles) * g.experts <= 15 ? skinny::kMaxSplit : 4) && long(tiles) * g.experts * split * 4 < slots * 3 && kBlocks >= 8 * split) split *= 2;
   skinny::Maps maps{};
-  if (!cache.get(maps.w, B, uint64_t(N), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
+  if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
   const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;
   auto kernel = tokenRows ? skinny::skinnyGemmKernel<skinny::kTokenRows>
               : epilogue == kEpiSwiglu ? skinny::skinnyGemmKernel<skinny::kWeightRowsSwiglu> : skinny::skinnyGemmKernel<skinny::kWeightRows>;
@@ -843,7 +852,7 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(split); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(unsigned(tiles * split)); cfg.blockDim = dim3(skinny::kThreads);
+  cfg.gridDim = dim3(unsigned(tiles * split), unsigned(g.experts)); cfg.blockDim = dim3(skinny::kThreads);
   cfg.dynamicSmemBytes = size_t(p.stages) * stageBytes + skinny::kBarrierBytes + 1024; cfg.stream = stream;
   cfg.attrs = attr; cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
@@ -858,6 +867,75 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
 bool useSkinny(int M, int N, int K, int epilogue) {
   if (M > skinny::kMaxTokens / 2) return epilogue == kEpiStore && N <= skinny::kMaxTokens;
   return M <= 64 || (N <= 8192 && K >= 1024);
+}
+
+// ---- any number of rows of activations: gemm_ragged.cuh ----
+int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
+  const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
+  if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
+  if (g.experts > ragged::kMaxExperts) { setError("grouped GEMM: at most 512 experts"); return 1; }
+  auto kernel = epilogue == kEpiSwiglu ? ragged::raggedGemmKernel<true> : ragged::raggedGemmKernel<false>;
+  static std::mutex mu;
+  static int pairsOf[64][2] = {};      // CTA pairs the device can hold at once (0: not asked yet)
+  int device = 0, pairs = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) { setError("GEMM launch: no current device"); return 1; }
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.blockDim = dim3(ragged::kThreads);
+  constexpr int stageBytes = 2 * ragged::kABytes + ragged::kMaxCols / 2 * ragged::kBK * 2;
+  constexpr int fixedBytes = 1024 + ragged::kStagingBytes + ragged::kBarrierBytes + ragged::kTableBytes;
+  constexpr int stages = (kSmemLimit - fixedBytes) / stageBytes < ragged::kMaxStages ? (kSmemLimit - fixedBytes) / stageBytes : ragged::kMaxStages;
+  cfg.dynamicSmemBytes = size_t(stages) * stageBytes + fixedBytes;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    int& known = pairsOf[device][epilogue == kEpiSwiglu ? 1 : 0];
+    if (!known) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess) { setError("cannot opt in to 227 KiB of shared memory"); return 1; }
+      int n = 0;
+      cfg.gridDim = dim3(unsigned(smCount() / 2 * 2));
+      known = smCount() / 2;
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) known = std::min(known, n);
+    }
+    pairs = known;
+  }
+  ragged::Params p{};
+  p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.experts = g.experts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
+  p.stages = stages; p.status = status; p.timeoutNs = 2ull * 1000 * 1000 * 1000;
+  const int wTiles = (N + ragged::kTileRows - 1) / ragged::kTileRows;
+  int items = INT32_MAX;
+  p.tileCols = ragged::kMaxCols; p.xBox = 32;
+  if (!g.counts) {
+    // The cut that leaves the pairs least idle. A tile takes about as long as its columns, in steps of 64, and 57 more do
+    // (measured per wave at K = 8192: 256 columns 90 us, 224 89 us, 192 72.5 us, 160 71.5 us); half tiles in the last wave
+    // take about 0.85 of a whole one.
+    auto cost = [](int cols) { return double((cols + 63) / 64 * 64 + 57); };
+    double best = -1;
+    for (int cols : {256, 192, 128}) {
+      const long full = M / cols, rem = M % cols ? 1 : 0, tiles = (full + rem) * wTiles, rest = tiles % pairs;
+      const double tail = rest == 0 ? 0. : 2 * rest <= pairs ? 0.85 : 1.;
+      const double average = (double(full) * cost(cols) + double(rem) * cost(M % cols)) / double(full + rem);
+      const double time = tiles > pairs ? (double(tiles / pairs) + tail) * average : (tiles == pairs ? 1. : tail) * cost(full ? cols : M % cols);
+      if (best < 0 || time < best * 0.99) { best = time; p.tileCols = cols; items = int(std::min<long>(2 * tiles, INT32_MAX)); }
+    }
+    p.xBox = p.tileCols / 2;
+  }
+  ragged::Maps maps{};
+  if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), ragged::kBM) ||
+      !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.xBox))) return 1;
+  cfg.gridDim = dim3(unsigned(std::min(pairs, items) * 2)); cfg.stream = stream;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
+  if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
+  return 0;
+}
+
+// Rows that are no multiple of 512 go through the ragged kernel once its 512 x 256 tiles give five eighths of the CTA pairs
+// work (one B200, us, it / the tiles of this file: 1000 x 14336 x 8192 177 / 222, 1000 x 8192 x 7168 83 / 104, 5000 x 4096 x
+// 4096 126 / 158, 1500 x 4096 x 4096 41 / 62; with fewer tiles 700 x 4096 x 4096 51 / 31, 300 x 8192 x 7168 61 / 56).
+bool useRagged(int M, int N) {
+  const long tiles = long((M + ragged::kMaxCols - 1) / ragged::kMaxCols) * ((N + ragged::kTileRows - 1) / ragged::kTileRows);
+  return M % (4 * kBM) != 0 && tiles * 16 >= long(smCount()) * 5;
 }
 
 }  // namespace
@@ -900,7 +978,8 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   Shape sh{};
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
-  if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, status, static_cast<cudaStream_t>(stream));
+  if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+  if (bn == 0 && useRagged(M, N)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
       !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;
@@ -912,6 +991,20 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   p.rank = 0; p.world = 1; p.blocksPerRank = p.tilesM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return epilogue == kEpiSwiglu ? launch<kEpiSwiglu, kCommNone>(maps, p, sh, s) : launch<kEpiStore, kCommNone>(maps, p, sh, s);
+}
+
+// Expert e owns counts[e] consecutive rows of A (and of C) and rows [e * N, (e + 1) * N) of B; rows beyond the sum of the
+// counts are neither read into a result nor written. Up to about 96 rows per expert the read of the weights is what takes
+// the time (few-rows kernel, every expert's weights once); above, the tensor pipe.
+int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, int experts, int N, int K, const int32_t* counts, int likelyRows,
+                             int epilogue, void* stream) {
+  NvtxRange range(epilogue == kEpiSwiglu ? "groupedGemmSwiglu" : "groupedGemm", size_t(rows) * size_t(N) * 2);
+  if (rows <= 0 || N <= 0 || K <= 0 || experts <= 0 || !counts) { setError("grouped GEMM: dimensions must be positive and counts given"); return 1; }
+  if (K % 8 || N % 8) { setError("N and K must be multiples of 8"); return 1; }
+  static thread_local MapCache cache;
+  GroupedArgs g;
+  g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);
+  return (g.likelyRows <= 96 ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 size_t purlin_tp_workspace_bytes(int world, int M, int kAg, int nRs) { return tpLayout(world, M, kAg, nRs).total; }

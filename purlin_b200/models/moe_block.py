@@ -3,7 +3,7 @@
     logits = x @ w_router.T                                  (tcgen05 GEMM)
     route: softmax + top-k                                   (one kernel)
     dispatch: tokens -> their experts' GPUs, expert-major    (one kernel over peer memory)
-    experts: SwiGLU MLP per local expert on its rows         (tcgen05 GEMMs on contiguous row ranges)
+    experts: SwiGLU MLP per local expert on its rows         (two grouped tcgen05 GEMMs over contiguous row ranges)
     combine: gate-weighted sum of the top-k outputs          (one kernel over peer memory)
 
 DeepSeek-V3-like shapes are the defaults of the benchmark: hidden 7168, 256 experts (32 per GPU at 8 GPUs), top-8.
@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from ..ops.gemm import gemm, gemm_swiglu, interleave_gate_up
+from ..ops.gemm import gemm, grouped_gemm, interleave_gate_up
 from ..parallel.expert_parallel import ExpertParallelContext
 
 
@@ -42,13 +42,11 @@ class ExpertParallelMoE:
         logits = gemm(x, self.w_router).float()
         self.ep.route(logits)
         recv, counts = self.ep.dispatch(x)
-        offs = [0] + torch.cumsum(counts[: self.ep.experts_per_rank], 0).tolist()   # one host read per layer: row ranges of the experts
         outb = self.ep.out_rows()
-        for e in range(self.ep.experts_per_rank):
-            a, b = offs[e], offs[e + 1]
-            if b > a:
-                h = gemm_swiglu(recv[a:b], self.w_gu[e], self._h[a:b])
-                gemm(h, self.w_down[e], outb[a:b])
+        # one launch per projection; the row counts stay on the device (rows per expert when every rank brings as many tokens)
+        average = -(-t * self.topk * self.ep.world // self.experts)
+        h = grouped_gemm(recv, self.w_gu, counts, average, self._h, swiglu=True)
+        grouped_gemm(h, self.w_down, counts, average, outb)
         return self.ep.combine(t, out)
 
     __call__ = forward

@@ -23,6 +23,7 @@ def _lib():
     if not _declared:
         vp, i = C.c_void_p, C.c_int
         lib.purlin_gemm_bf16.argtypes = [vp, vp, vp, i, i, i, i, i, vp, vp]
+        lib.purlin_gemm_grouped_bf16.argtypes = [vp, vp, vp, i, i, i, i, vp, i, i, vp]
         _declared = True
     return lib
 
@@ -70,5 +71,25 @@ def gemm_swiglu(a: torch.Tensor, w_gu: torch.Tensor, out: Optional[torch.Tensor]
     lib = _lib()
     rc = lib.purlin_gemm_bf16(a.data_ptr(), w_gu.data_ptr(), out.data_ptr(), m, n, k, EPI_SWIGLU, bn, None,
                               torch.cuda.current_stream().cuda_stream)
+    _native.check(lib, rc)
+    return out
+
+
+def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_rows: int, out: torch.Tensor, swiglu: bool = False) -> torch.Tensor:
+    """``out[rows of e] = a[rows of e] @ w[e].T`` (or the SwiGLU form) for every expert e, in one launch: expert e owns
+    ``counts[e]`` consecutive rows of ``a [rows, K]`` and ``w[e] [N, K]``. ``counts`` (int32) stays on the device; rows beyond
+    the sum of the counts are left alone. ``likely_rows`` says how many rows an expert is expected to have."""
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or counts.dtype != torch.int32:
+        raise TypeError("the grouped GEMM takes bf16 operands and int32 counts")
+    if not (a.is_cuda and w.is_cuda and out.is_cuda and counts.is_cuda):
+        raise ValueError("operands must be CUDA tensors")
+    if not (a.is_contiguous() and w.is_contiguous() and out.is_contiguous() and counts.is_contiguous()):
+        raise ValueError("operands must be contiguous")
+    experts, n, k = w.shape
+    if a.shape[1] != k or out.shape != (a.shape[0], n // 2 if swiglu else n) or counts.numel() < experts:
+        raise ValueError("a is [rows, K], w is [experts, N, K], out is [rows, N or N / 2] and counts has an entry per expert")
+    lib = _lib()
+    rc = lib.purlin_gemm_grouped_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], experts, n, k, counts.data_ptr(), likely_rows,
+                                      EPI_SWIGLU if swiglu else EPI_STORE, torch.cuda.current_stream().cuda_stream)
     _native.check(lib, rc)
     return out

@@ -117,3 +117,37 @@ def test_swiglu_at_odd_sizes(m, i, k):
     ref = torch.nn.functional.silu(a.float() @ wg.float().t()) * (a.float() @ wu.float().t())
     # one rounding to bf16 (2^-9 relative) on top of fp32 sums; the absolute term covers cancellation at K <= 512 of unit values
     assert ((out - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 264, 72), (257, 14336, 72), (513, 8192, 136), (777, 8200, 328), (1000, 14336, 64), (2049, 4104, 72),
+                                    (2368, 8192, 64)])
+def test_ragged_rows_are_exact_on_small_integers(m, n, k):
+    # row counts that are no multiple of a tile: narrow remainder tiles, half tiles in the last wave, more than one wave
+    from purlin_b200.ops.gemm import gemm
+    a, w = _small_integers(m, n, k, 13)
+    assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("likely", [1, 40, 96, 97, 400])
+@pytest.mark.parametrize("counts", [[0, 1, 0, 31, 33, 0], [300, 0, 129, 1, 256, 515], [0, 0, 0, 0, 0, 700], [0, 0, 0, 0, 0, 0]])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_grouped_gemm(likely, counts, swiglu):
+    # `likely` picks the kernel and the columns of a pass; any counts have to come out right, and rows beyond them stay as they were
+    from purlin_b200.ops.gemm import grouped_gemm
+    n, k, rows = 544, 136, sum(counts) + 37
+    a, _ = _small_integers(rows, 8, k, 14)
+    w = torch.stack([_small_integers(1, n, k, 20 + e)[1] for e in range(len(counts))])
+    out = torch.full((rows, n // 2 if swiglu else n), 7.0, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w, torch.tensor(counts, dtype=torch.int32, device="cuda"), likely, out, swiglu=swiglu)
+    first = 0
+    for e, c in enumerate(counts):
+        ref = a[first:first + c].float() @ w[e].float().t()
+        got = out[first:first + c].float()
+        if swiglu:
+            v = ref.view(c, n // 32, 2, 16)
+            ref = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(c, n // 2)
+            assert ((got - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+        else:
+            assert torch.equal(got, ref.to(torch.bfloat16).float())
+        first += c
+    assert (out[first:] == 7).all()

@@ -125,6 +125,19 @@ def test_default_policies(worlds):
             run_case(ew, coll, nbytes=n, dtype=0, pol=None, reps=1)
 
 
+@pytest.mark.parametrize("world", [2, 4, 8])
+def test_default_grids_fit_and_ranks_travel_with_the_launch(worlds, world):
+    # sizes in both regimes, every collective: the shared grid has to fit on one GPU, and short plans go as kernel parameters
+    ew = worlds(world, 4 << 20)
+    for n in (32, 4096 + 32, 3 * (1 << 20) // world // 32 * 32, 5 * (1 << 20)):
+        for coll in (AR, AG, RS, A2A):
+            run_case(ew, coll, nbytes=n, dtype=4, pol=None)
+    for scale in (4096, 1 << 21):
+        for coll in (AGV, RSV):
+            run_case(ew, coll, sizes=_sizes(world, 3, scale=scale, zero_every=3), dtype=0, pol=None)
+        run_case(ew, A2AV, sizes=[_sizes(world, 60 + r, scale=scale, zero_every=4) for r in range(world)], dtype=0, pol=None)
+
+
 def test_absent_rank_times_out_and_context_recovers():
     # A rank that never launches: the others' bounded waits give up, the host reads a status, and after
     # clearing it the same contexts run a correct collective. Nothing traps, faults or spins forever.

@@ -37,6 +37,9 @@ void* purlin_moe_out_buffer(PurlinMoeContext* ctx);    /* [capacityRows, hidden]
  * topkIdx / topkWeight / slot [tokens, topk] are device outputs the context keeps using until the next route or plan. */
 int purlin_moe_route(PurlinMoeContext* ctx, const float* logits, int tokens, int normalize, int32_t* topkIdx, float* topkWeight,
                      int32_t* slot, void* stream);
+/* The same from bf16 logits, as a router GEMM writes them. */
+int purlin_moe_route_bf16(PurlinMoeContext* ctx, const void* logits, int tokens, int normalize, int32_t* topkIdx, float* topkWeight,
+                          int32_t* slot, void* stream);
 /* The plan alone, for routing the caller computed itself: slot = position of each (token, expert) pair among this rank's
  * rows of that expert; internally one send-list position per (token, destination GPU). Expert ids outside
  * [0, experts) are reported through the status word and their pairs dropped. */

@@ -22,14 +22,14 @@ __device__ __forceinline__ float sanitizeLogit(float x) {
 }
 
 // One warp routes one token. Lane k (k < topk) returns the k-th choice in `expert` / `weight`; other lanes get -1 / 0.
-// VPL = experts / 32 values per lane.
-template <int VPL>
-__device__ __forceinline__ void routeToken(const float* __restrict__ row, int experts, int topk, int normalize, int lane,
+// VPL = experts / 32 values per lane. Logit: float, or a 16-bit type that converts to it.
+template <int VPL, class Logit>
+__device__ __forceinline__ void routeToken(const Logit* __restrict__ row, int experts, int topk, int normalize, int lane,
                                            int& expert, float& weight) {
   float v[VPL];
   float mx = -FLT_MAX;
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) { v[i] = sanitizeLogit(row[i * 32 + lane]); mx = fmaxf(mx, v[i]); }
+  for (int i = 0; i < VPL; ++i) { v[i] = sanitizeLogit(static_cast<float>(row[i * 32 + lane])); mx = fmaxf(mx, v[i]); }
 #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;

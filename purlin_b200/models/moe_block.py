@@ -39,8 +39,7 @@ class ExpertParallelMoE:
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         t = x.shape[0]
-        logits = gemm(x, self.w_router).float()
-        self.ep.route(logits)
+        self.ep._route_bf16(gemm(x, self.w_router))
         recv, counts = self.ep.dispatch(x)
         outb = self.ep.out_rows()
         # one launch per projection; the row counts stay on the device (rows per expert when every rank brings as many tokens)

@@ -40,6 +40,7 @@ def _lib():
         lib.purlin_moe_out_buffer.restype = vp
         lib.purlin_moe_out_buffer.argtypes = [vp]
         lib.purlin_moe_route.argtypes = [vp, vp, i, i, vp, vp, vp, vp]
+        lib.purlin_moe_route_bf16.argtypes = [vp, vp, i, i, vp, vp, vp, vp]
         lib.purlin_moe_dispatch.argtypes = [vp, vp, i, vp, vp, vp, vp, i, vp]
         lib.purlin_moe_combine.argtypes = [vp, vp, i, vp, vp, vp, i, vp]
         _declared = True
@@ -93,6 +94,12 @@ class ExpertParallelContext:
                                        self.topk_weight.data_ptr(), self.slot.data_ptr(), self.stream())
         _native.check(self.lib, rc)
         return self.topk_idx[:t], self.topk_weight[:t]
+
+    def _route_bf16(self, logits: torch.Tensor):
+        """``route`` for the bf16 logits that a router GEMM has just written: the same values without a pass that widens them."""
+        rc = self.lib.purlin_moe_route_bf16(self.ctx, logits.data_ptr(), logits.shape[0], 1, self.topk_idx.data_ptr(),
+                                            self.topk_weight.data_ptr(), self.slot.data_ptr(), self.stream())
+        _native.check(self.lib, rc)
 
     def plan(self, topk_idx: torch.Tensor, topk_weight: torch.Tensor):
         """Adopts routing the caller computed: int32 ``topk_idx`` and fp32 ``topk_weight`` of shape [tokens, topk]."""

@@ -11,7 +11,7 @@ from typing import Optional
 
 import torch
 
-from .. import _native
+from .. import _native, _stream
 
 EPI_STORE, EPI_SWIGLU = 0, 1
 _declared = False
@@ -45,7 +45,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, b
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     lib = _lib()
     rc = lib.purlin_gemm_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, EPI_STORE, bn, None,
-                              torch.cuda.current_stream().cuda_stream)
+                              _stream(None))
     _native.check(lib, rc)
     return out
 
@@ -70,7 +70,7 @@ def gemm_swiglu(a: torch.Tensor, w_gu: torch.Tensor, out: Optional[torch.Tensor]
         out = torch.empty(m, n // 2, dtype=torch.bfloat16, device=a.device)
     lib = _lib()
     rc = lib.purlin_gemm_bf16(a.data_ptr(), w_gu.data_ptr(), out.data_ptr(), m, n, k, EPI_SWIGLU, bn, None,
-                              torch.cuda.current_stream().cuda_stream)
+                              _stream(None))
     _native.check(lib, rc)
     return out
 
@@ -90,6 +90,6 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_
         raise ValueError("a is [rows, K], w is [experts, N, K], out is [rows, N or N / 2] and counts has an entry per expert")
     lib = _lib()
     rc = lib.purlin_gemm_grouped_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], experts, n, k, counts.data_ptr(), likely_rows,
-                                      EPI_SWIGLU if swiglu else EPI_STORE, torch.cuda.current_stream().cuda_stream)
+                                      EPI_SWIGLU if swiglu else EPI_STORE, _stream(None))
     _native.check(lib, rc)
     return out

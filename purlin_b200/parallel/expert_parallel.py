@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from .. import _native
+from .. import _native, _stream
 from .symmetric import allocate_symmetric, RawBuffer as _RawBuffer
 
 _declared = False
@@ -69,7 +69,7 @@ class ExpertParallelContext:
             base = (self._owner.data_ptr() + 1023) // 1024 * 1024
             self._hdl, peer_ptrs = None, [base]
         ptrs = (C.c_uint64 * self.world)(*peer_ptrs)
-        self.stream = lambda: torch.cuda.current_stream().cuda_stream
+        self.stream = lambda: _stream(None)
         self.ctx = self.lib.purlin_moe_create(self.rank, self.world, ptrs, max_tokens, hidden, experts, topk, self.capacity_rows,
                                               timeout_ms * 1_000_000, self.stream())
         if not self.ctx:

@@ -34,17 +34,19 @@ class EmulatedWorld:
                 if not h:
                     raise RuntimeError("purlin: " + _native.last_error(self.lib))
                 self.ctxs.append(h)
+        self._ptrs = C.c_void_p * world
+        self._ctx_arr = self._ptrs(*self.ctxs)
 
     def run(self, collective: int, srcs: Sequence[torch.Tensor], dsts: Sequence[torch.Tensor], nbytes: int = 0,
             sizes=None, dtype: int = 0, op: int = 0, mode: int = 0, policy=None, absent: int = -1):
         w = self.world
-        ctx_arr = (C.c_void_p * w)(*self.ctxs)
-        src_arr = (C.c_void_p * w)(*[t.data_ptr() if t.numel() else None for t in srcs])
-        dst_arr = (C.c_void_p * w)(*[t.data_ptr() if t.numel() else None for t in dsts])
+        # (an empty tensor's data_ptr is 0, the null pointer)
+        src_arr = self._ptrs(*[t.data_ptr() for t in srcs])
+        dst_arr = self._ptrs(*[t.data_ptr() for t in dsts])
         flat = None
         if sizes is not None:
             flat = _native.size_array([x for row in sizes for x in row] if isinstance(sizes[0], (list, tuple)) else sizes)
-        rc = self.lib.purlin_emu_collective(ctx_arr, w, collective, src_arr, dst_arr, nbytes, flat, dtype, op, mode,
+        rc = self.lib.purlin_emu_collective(self._ctx_arr, w, collective, src_arr, dst_arr, nbytes, flat, dtype, op, mode,
                                             C.byref(policy) if policy is not None else None, absent, self.stream)
         _native.check(self.lib, rc)
 
@@ -72,6 +74,7 @@ class EmulatedWorld:
         for h in self.ctxs:
             self.lib.purlin_context_destroy(h, self.stream)
         self.ctxs = []
+        self._ctx_arr = None
 
     def __del__(self):
         try:

@@ -806,13 +806,29 @@ struct GroupedArgs {
   int likelyRows = 0;                 // rows a group is expected to have
 };
 
+// Which GEMMs the few-rows kernel takes, each line with one B200's times in us, it / the other tiles. Few rows of W (a router)
+// with a long k: 4096 x 32 x 7168 11 / 75; with a short k the sum over the partial tiles costs more than it saves (1656 x 208
+// x 112 14.4 / 12.2 a call).
+bool fewWeightRows(int M, int N, int K, int epilogue) { return epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens && K >= 2048; }
+bool useSkinny(int M, int N, int K, int epilogue) {
+  if (fewWeightRows(M, N, K, epilogue)) return true;
+  // always up to 64 rows: 64 x 57344 x 8192 153 / 165, 48 x 4096 x 4096 14 / 22
+  if (M <= 64) return true;
+  // up to 128 while W has too few rows to give every SM a tile of its own and k is worth splitting: 128 x 8192 x 7168 31.5 /
+  // 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 14336 x 4096 28.2 / 27.4, 128 x 264 x 72 7.4 / 5.3
+  if (M <= 128) return N <= 8192 && K >= 1024;
+  // up to 256 where the tiles are few and k is long: 256 x 4096 x 4096 21.2 / 25.1, 256 x 8192 x 7168 40.4 / 42.4, 140 x 8192 x
+  // 4096 21.1 / 22.6; but 200 x 14336 x 8192 74.9 / 67.5, 200 x 264 x 72 9.2 / 5.3
+  return M <= skinny::kMaxTokens && N >= 4096 && N <= 8192 && K >= 4096;
+}
+
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
 int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
   if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
   skinny::Params p{};
   // Few rows of W against many rows of X (a router): the operands change places and the output row is the MMA's row.
-  const bool tokenRows = !g.counts && epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens;
+  const bool tokenRows = !g.counts && fewWeightRows(M, N, K, epilogue);
   if (tokenRows) { std::swap(A, B); std::swap(M, N); }
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status;
@@ -860,14 +876,7 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   return 0;
 }
 
-// Where the few-rows kernel is the better one (one B200, us, it / the tiles of this file): always up to 64 rows (64 x 57344 x
-// 8192 153 / 165, 48 x 4096 x 4096 14 / 22); up to 128 rows while W has too few rows to give every SM a tile of its own and k is
-// worth splitting (128 x 8192 x 7168 31.5 / 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 14336 x
-// 4096 28.2 / 27.4 and 128 x 264 x 72 7.4 / 5.3); few rows of W (4096 x 32 x 7168 11 / 75).
-bool useSkinny(int M, int N, int K, int epilogue) {
-  if (M > skinny::kMaxTokens / 2) return epilogue == kEpiStore && N <= skinny::kMaxTokens;
-  return M <= 64 || (N <= 8192 && K >= 1024);
-}
+constexpr int kFewGroupRows = 12;
 
 // ---- any number of rows of activations: gemm_ragged.cuh ----
 int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
@@ -994,8 +1003,10 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
 }
 
 // Expert e owns counts[e] consecutive rows of A (and of C) and rows [e * N, (e + 1) * N) of B; rows beyond the sum of the
-// counts are neither read into a result nor written. Up to about 96 rows per expert the read of the weights is what takes
-// the time (few-rows kernel, every expert's weights once); above, the tensor pipe.
+// counts are neither read into a result nor written. The kernel on CTA pairs streams the weights as fast as the few-rows
+// kernel, because a pair's loads run on into its next tile; with a handful of rows per expert the few-rows kernel is ahead, it
+// has a CTA per 128 weight rows (32 experts, gate-up 4096 x 7168 + down 7168 x 2048, us, pairs / few rows: 1 row 306 / 283, 4
+// rows 435 / 425, 16 rows 456 / 462, 32 rows 463 / 473, 64 rows 466 / 543).
 int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, int experts, int N, int K, const int32_t* counts, int likelyRows,
                              int epilogue, void* stream) {
   NvtxRange range(epilogue == kEpiSwiglu ? "groupedGemmSwiglu" : "groupedGemm", size_t(rows) * size_t(N) * 2);
@@ -1004,7 +1015,7 @@ int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, in
   static thread_local MapCache cache;
   GroupedArgs g;
   g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);
-  return (g.likelyRows <= 96 ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, nullptr, static_cast<cudaStream_t>(stream));
+  return (g.likelyRows <= kFewGroupRows ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 size_t purlin_tp_workspace_bytes(int world, int M, int kAg, int nRs) { return tpLayout(world, M, kAg, nRs).total; }

@@ -93,7 +93,7 @@ def _small_integers(m, n, k, seed):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 136, 72), (15, 264, 200), (16, 1024, 64), (17, 128, 520), (33, 640, 1024), (64, 4096, 4096),
-                                    (65, 2048, 1096), (96, 384, 2048), (128, 1024, 4096)])
+                                    (65, 2048, 1096), (96, 384, 2048), (128, 1024, 4096), (129, 4096, 4096), (255, 4104, 4160)])
 def test_few_rows_are_exact_on_small_integers(m, n, k):
     # tiles of 128 weight rows with and without a remainder, one to eight k-splits, one column up to a full pass
     from purlin_b200.ops.gemm import gemm
@@ -101,7 +101,7 @@ def test_few_rows_are_exact_on_small_integers(m, n, k):
     assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
 
 
-@pytest.mark.parametrize("m,n,k", [(129, 8, 64), (300, 32, 1024), (4096, 64, 512), (1000, 256, 136), (257, 248, 72)])
+@pytest.mark.parametrize("m,n,k", [(129, 8, 2048), (300, 32, 4096), (4096, 64, 2056), (1000, 256, 2112), (257, 248, 7168)])
 def test_few_weight_rows_are_exact_on_small_integers(m, n, k):
     # a router's shape: the tokens are the rows of the tile
     from purlin_b200.ops.gemm import gemm
@@ -128,7 +128,7 @@ def test_ragged_rows_are_exact_on_small_integers(m, n, k):
     assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
 
 
-@pytest.mark.parametrize("likely", [1, 40, 96, 97, 400])
+@pytest.mark.parametrize("likely", [1, 8, 12, 13, 400])
 @pytest.mark.parametrize("counts", [[0, 1, 0, 31, 33, 0], [300, 0, 129, 1, 256, 515], [0, 0, 0, 0, 0, 700], [0, 0, 0, 0, 0, 0]])
 @pytest.mark.parametrize("swiglu", [False, True])
 def test_grouped_gemm(likely, counts, swiglu):

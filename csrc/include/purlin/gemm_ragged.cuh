@@ -23,8 +23,11 @@ constexpr int kBM = 128, kBK = 64, kMaxCols = 256;
 constexpr int kABytes = kBM * kBK * 2;
 constexpr int kTileRows = 512;                  // rows of W per tile: 2 accumulators x 2 CTAs x 128
 constexpr int kAccStride = 256, kTmemCols = 512;
-constexpr int kEpiWarps = 4, kThreads = 32 * (2 + kEpiWarps);
-constexpr int kStagingBytes = kEpiWarps * 2 * 2048;   // two 32 x 32 bf16 tiles per epilogue warp
+// Four epilogue warps per accumulator: with both accumulators of a tile in use the epilogue is exposed, and eight warps halve it
+// (four / eight warps, one B200: 3000 x 7168 x 2048 77.5 / 73.3 us, 1500 x 4096 x 4096 SwiGLU 51.1 / 46.9, 32 experts of 1024
+// rows 1748 + 1151 / 1631 + 1130).
+constexpr int kEpiWarps = 8, kThreads = 32 * (2 + kEpiWarps);
+constexpr int kStagingBytes = kEpiWarps * 2048;       // a 32 x 32 bf16 tile per epilogue warp
 constexpr int kBarrierBytes = 256;
 constexpr int kMaxExperts = 512;
 constexpr int kTableBytes = 2 * (kMaxExperts + 1) * 4;
@@ -75,7 +78,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
-    for (int a = 0; a < 2; ++a) { tc::mbarInit(tmemFullBar(a), 1); tc::mbarInit(tmemEmptyBar(a), kEpiWarps * 2); }
+    for (int a = 0; a < 2; ++a) { tc::mbarInit(tmemFullBar(a), 1); tc::mbarInit(tmemEmptyBar(a), kEpiWarps); }   // 4 warps in each CTA
     *abortWord = 0;
     tc::mbarFenceInit();
     tc::tmaPrefetchDescriptor(&maps.w);
@@ -213,16 +216,17 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     constexpr int kPitch = kOut * 2;                           // bytes of a token's row in the staging tile
     const int quarter = warp & 3;                              // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
     const int outCols = SWIGLU ? p.N / 2 : p.N;
-    uint32_t use0 = 0, use1 = 0, chunkCount = 0;
+    const int a = (warp - 2) / 4;                              // this warp's accumulator
+    const uint32_t buf = stagingAll + uint32_t(warp - 2) * 2048u;
+    uint32_t use = 0;
     bool ok = true;
     for (int it = pairIdx; it < numItems && ok; it += numPairs) {
       const Item m = itemOf(it);
-#pragma unroll 1
-      for (int a = 0; a < m.accs && ok; ++a) {
-        ok = tc::mbarWait(tmemFullBar(a), (a ? use1 : use0) & 1, abortWord, p.timeoutNs);
+      if (a < m.accs) {
+        ok = tc::mbarWait(tmemFullBar(a), use & 1, abortWord, p.timeoutNs);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { if (lane == 0) skinny::recordTimeout(p.status, 5, it, a); break; }
-        if (a) ++use1; else ++use0;
+        ++use;
         tc::fenceAfterThreadSync();
         const uint32_t taddr = tmemBase + (uint32_t(quarter * 32) << 16) + uint32_t(a) * kAccStride;
         const int wRow = m.w0 + a * 2 * kBM + int(ctaRank) * kBM + quarter * 32;     // of lane 0
@@ -231,7 +235,6 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
 
         // 32 columns (tokens) of this warp's 32 rows of W -> rows of C
         auto drain = [&](const uint32_t (&r)[32], int c) {
-          const uint32_t buf = stagingAll + uint32_t(quarter * 2 + (chunkCount++ & 1)) * 2048u;
           if constexpr (SWIGLU) {
             // lanes 0-15 hold gate, 16-31 up, of the same 16 output columns: the lower half finishes tokens t and t + 1, the
             // upper half t + 2 and t + 3; then neighbouring lanes pair up so that each writes two columns of one token
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]) : "r"(buf + uint32_t(row * kPitch + piece * 16)) : "memory");
             if (colOk && c + row < m.count) st16(out + size_t(c + row) * p.ldc + piece * 8, v);
           }
-          // (two buffers in turn: the warp is past the reads of a buffer, by the other chunk's __syncwarp, before it is filled again)
+          __syncwarp();                                        // the tile has been read before the next chunk fills it
         };
         uint32_t ra[32], rb[32];
         tc::tmemLoad32(taddr, ra);

@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     tc::tmaPrefetchDescriptor(&maps.x);
   }
   if (warp == 1) { tc::tmemAllocPair(tc::smemAddr(words), kTmemCols); tc::tmemRelinquishPair(); }
+  tc::gridDependencyWait();                                    // from here on memory that earlier kernels write may be read
   if (warp == 2) {
     // rows and tiles of every expert, as running sums: 32 experts per step
     int rows0 = 0, items0 = 0;
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   __syncthreads();
   tc::clusterSync();                                           // the pair's barriers exist before any remote arrival
   tc::fenceAfterThreadSync();
+  tc::gridLaunchDependents();
   const uint32_t tmemBase = *tmemBaseWord;
   const uint32_t leaderBars = tc::mapToCta(barBase, 0), peerBars = tc::mapToCta(barBase, 1);
   const int numTiles = itemStart[p.experts], rest = numTiles % numPairs;

@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
     tc::tmaPrefetchDescriptor(&maps.x);
   }
   if (warp == 1) { tc::tmemAlloc(tc::smemAddr(words), uint32_t(p.tmemCols)); tc::tmemRelinquish(); }
+  tc::gridDependencyWait();                                   // from here on memory that earlier kernels write may be read
   if (warp == 2) {
     int first = 0, rows = p.tokens;
     if (p.counts) {
@@ -210,6 +211,8 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
     }
     __syncwarp();
     tc::clusterSync();                                        // every partial tile of the cluster is in shared memory
+    // Only now may the next kernel take the free places: earlier, its CTAs would crowd the SMs that this one leaves empty.
+    tc::gridLaunchDependents();
     // ---- the sum: CTA `part` finishes its share of the tokens, 8 output columns per thread ----
     if (MODE == kTokenRows && *abortWord == 0) {
       // row r of the tile, 8 of its columns per thread; neighbouring lanes read neighbouring rows

@@ -84,6 +84,14 @@ template <int N> PURLIN_D void bulkWaitGroupRead() { asm volatile("cp.async.bulk
 // at most N of this thread's groups may still be in flight at all (their global writes included)
 template <int N> PURLIN_D void bulkWaitGroup() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
 
+// ---- programmatic dependent launch ----
+// A kernel launched with the attribute may start while the kernel before it on the stream still runs: its set-up (barriers,
+// TMEM, descriptors) then costs nothing. Everything that touches memory another kernel reads or writes comes after
+// gridDependencyWait(), which returns once the kernels before it have finished and their writes are visible.
+PURLIN_D void gridDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// lets the next kernel on the stream start its own set-up as soon as every CTA of this one has got here
+PURLIN_D void gridLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- CTA pairs (cluster of two): the pair shares one 256-row MMA; CTA 0 issues it ----
 PURLIN_D uint32_t clusterCtaRank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 // address of the same shared-memory offset inside CTA `rank` of the cluster

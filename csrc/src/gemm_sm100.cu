@@ -14,7 +14,7 @@
 //                                        a third fewer operand bytes per flop, and consecutive MMAs alternate between
 //                                        the accumulators while they share the B operand, which the tensor pipe rewards
 //                                        (measured on B200: +13 % over back-to-back MMAs into one accumulator)
-//   warps 2-5   epilogue       tcgen05.ld -> registers -> fused epilogue -> global / peer memory
+//   warps 2-5   epilogue       (2-9 in the plain GEMM with two accumulators, four for each) tcgen05.ld -> registers -> fused epilogue -> global / peer memory
 //   warps 6-9   communication  (all-gather variant) push this rank's activation rows into every peer's buffer
 //
 // Variants (template COMM):
@@ -55,8 +55,9 @@ constexpr int kBM = 128, kBK = 64, kMaxBN = 256;
 constexpr int kAccStride = 256;                // TMEM columns between the two accumulators
 constexpr int kTmemCols = 512;
 constexpr int kABytes = kBM * kBK * 2;         // 16 KiB
-constexpr int kEpiWarps = 4, kCommWarps = 4;
-constexpr int kThreadsPlain = 32 * (2 + kEpiWarps);
+enum { kEpiStore = 0, kEpiSwiglu = 1 };
+enum { kCommNone = 0, kCommAG = 1, kCommRS = 2 };
+constexpr int kEpiWarps = 4, kCommWarps = 4;    // warps that drain one accumulator of a CTA; pushing warps
 constexpr int kThreadsComm = 32 * (2 + kEpiWarps + kCommWarps);
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kBarrierBytes = 256;
@@ -65,11 +66,13 @@ constexpr int kMaxStages = 8;
 // 128-byte swizzle), filled from its TMEM lanes and drained row-contiguously: by a TMA store, by coalesced stores into
 // a peer's memory, or by the owner's sum over the peers' partial tiles.
 constexpr int kStageTileBytes = 32 * 128;
-constexpr int kStageTiles = 4;                  // per warp: up to three TMA stores in flight while the fourth tile is filled
-constexpr int kStagingBytes = kEpiWarps * kStageTiles * kStageTileBytes;   // 64 KiB
-
-enum { kEpiStore = 0, kEpiSwiglu = 1 };
-enum { kCommNone = 0, kCommAG = 1, kCommRS = 2 };
+constexpr int kStageTilesAll = 16;              // of a CTA: four per warp (three TMA stores in flight while the fourth is filled), two with eight warps
+constexpr int kStagingBytes = kStageTilesAll * kStageTileBytes;   // 64 KiB
+// With two accumulators per tile the epilogue is exposed (the next tile's MMAs need both), so the plain GEMM gives each
+// accumulator four epilogue warps of its own; with one per tile it hides under the next tile's MMAs (four / eight warps, one
+// B200: 2048 x 4096 x 2048 34.5 / 32.5 us, 8192 x 2048 x 1024 SwiGLU 38.1 / 36.0, 1024 x 14336 x 8192 SwiGLU 184.5 / 182.5).
+template <int COMM, int ACCS> constexpr int epilogueWarps() { return COMM == kCommNone && ACCS == 2 ? 2 * kEpiWarps : kEpiWarps; }
+template <int COMM, int ACCS> constexpr int threadsOf() { return COMM == kCommAG ? kThreadsComm : 32 * (2 + epilogueWarps<COMM, ACCS>()); }
 
 struct Params {
   int M, N, K, bn, stages;             // bn: columns of a tile (one MMA); a tile is ACCS x CTAS x 128 rows tall
@@ -224,7 +227,7 @@ PURLIN_D void itemOf(const Params& p, int i, int& tile, int& first, int& count) 
 // byte of B crosses L2 -> shared memory once per 256 rows instead of once per 128.
 // ACCS = 2 (pairs only): the tile is 2 x 256 rows tall; each k-block of B meets two blocks of A, one per accumulator.
 template <int EPI, int COMM, int CTAS, int ACCS>
-__global__ void __launch_bounds__(COMM == kCommAG ? kThreadsComm : kThreadsPlain, 1)
+__global__ void __launch_bounds__(threadsOf<COMM, ACCS>(), 1)
 gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) {
   extern __shared__ unsigned char smemRaw[];
   const uint32_t rawAddr = tc::smemAddr(smemRaw);
@@ -395,9 +398,12 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
         }
       }
     }
-  } else if (warp < 2 + kEpiWarps) {
+  } else if (warp < 2 + epilogueWarps<COMM, ACCS>()) {
     // ------------------------------- epilogue -------------------------------
     const int quarter = warp & 3;                // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
+    constexpr bool kOwnAcc = epilogueWarps<COMM, ACCS>() > kEpiWarps;      // this warp drains one accumulator of every tile
+    constexpr int kStageTiles = kStageTilesAll / epilogueWarps<COMM, ACCS>();
+    const int group = kOwnAcc ? (warp - 2) / kEpiWarps : 0;
     uint32_t accIt = 0;
     uint32_t use0 = 0, use1 = 0;
     uint32_t tileCount = 0;                      // staging tiles this warp has filled: they rotate through its buffers
@@ -410,7 +416,7 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
       const int n0 = nBlk * p.bn;
 
 #pragma unroll 1
-      for (int ai = 0; ai < accCount && ok; ++ai) {
+      for (int ai = group; ai < (kOwnAcc ? min(accCount, group + 1) : accCount) && ok; ++ai) {
       const int a = ACCS == 1 ? int(accIt & 1) : ai;      // accumulator slot
       const int mBlk = (rowBlk * ACCS + accFirst + ai) * CTAS + int(ctaRank);   // this CTA's 128-row block of the accumulator
       const int rowInTile = quarter * 32 + lane;
@@ -739,7 +745,7 @@ cudaLaunchAttribute overlapAttribute() {
 template <int EPI, int COMM, int CTAS, int ACCS>
 int launchImpl(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t stream) {
   auto kernel = gemmKernel<EPI, COMM, CTAS, ACCS>;
-  constexpr int threads = COMM == kCommAG ? kThreadsComm : kThreadsPlain;
+  constexpr int threads = threadsOf<COMM, ACCS>();
   // shared-memory opt-in and cluster occupancy belong to the device's copy of the kernel: resolve them once per device
   static int perDevice[64];
   static bool seen[64] = {};

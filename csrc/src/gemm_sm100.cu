@@ -1011,7 +1011,7 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
   if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
-  if (bn == 0 && useRagged(M, N)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+  if (bn == 0 && !switches().singleCta && !switches().oneAcc && useRagged(M, N)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
       !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;

@@ -463,7 +463,9 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
       else if (COMM == kCommRS) outRow0 = p.C + size_t(rowInShard - lane) * p.ldc;
       else outRow0 = p.C + size_t(row0) * p.ldc;
       const int rowsValid = COMM == kCommRS ? 32 : (p.M - row0 < 32 ? p.M - row0 : 32);    // rows of this warp inside the output
-      const int nChunks = p.bn / 32;
+      // chunks of 32 accumulator columns that hold output: none past the last column (a tile of 256 over 64 columns has two), none
+      // in a warp whose rows all lie past the last row
+      const int nChunks = rowsValid <= 0 ? 0 : min(p.bn / 32, (outBound - outCol0 + kOut - 1) / kOut);
 
       // 32 accumulator columns of this lane's row -> bf16 (activated) -> chunk `slot` of the staging tile
       const uint32_t stagingWarp = stagingAll + uint32_t(warp - 2) * uint32_t(kStageTiles * kStageTileBytes);
@@ -490,9 +492,10 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
       };
 
       // Software pipeline over the accumulator: the TMEM load of the next 32 columns is in flight while the current ones
-      // are converted and staged; every kPerTile chunks a staging tile is full and is drained.
+      // are converted and staged; every kPerTile chunks a staging tile is full and is drained. Every staging tile that is
+      // filled commits one bulk group, an empty one if it leaves by plain stores: the wait below counts groups.
       uint32_t ra[32], rb[32];
-      tc::tmemLoad32(taddr, ra);
+      if (nChunks > 0) tc::tmemLoad32(taddr, ra);
 #pragma unroll 1
       for (int c0 = 0; c0 < nChunks; c0 += kPerTile) {
         const uint32_t buf = stagingWarp + (tileCount % uint32_t(kStageTiles)) * kStageTileBytes;
@@ -519,7 +522,6 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
         }
         // ---- drain the tile: output columns [oc, oc + cols) of the warp's 32 rows ----
         const int oc = outCol0 + (c0 / kPerTile) * 64, cols = filled * kOut;
-        if (oc >= outBound || rowsValid <= 0) continue;
         if constexpr (COMM != kCommRS) {
           // a whole tile (or one whose unused columns fall outside the matrix, where the store is clipped) leaves by TMA
           if (cols == 64 || oc + cols >= outBound) {
@@ -528,6 +530,7 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
             if (lane == 0) { tc::tmaStore2d(&maps.c, oc, row0, buf); tc::bulkCommitGroup(); }
             continue;
           }
+          if (lane == 0) tc::bulkCommitGroup();
         }
         __syncwarp();
         const int rowInGroup = lane >> 3, piece = lane & 7;

@@ -151,3 +151,25 @@ def test_grouped_gemm(likely, counts, swiglu):
             assert torch.equal(got, ref.to(torch.bfloat16).float())
         first += c
     assert (out[first:] == 7).all()
+
+
+@pytest.mark.parametrize("m", [512, 1024, 4096])
+@pytest.mark.parametrize("n,bn", [(8, 0), (32, 0), (64, 0), (72, 0), (128, 0), (264, 0), (320, 0), (1000, 0), (448, 224), (320, 160), (192, 96), (72, 32)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_tiles_wider_than_the_output_are_exact_on_small_integers(m, n, bn, swiglu):
+    # The staging tiles of the epilogue rotate: columns past the output take none, a tile that leaves by plain stores counts like
+    # one that leaves by TMA. Several calls with a short k, so that the epilogues follow each other closely.
+    from purlin_b200.ops.gemm import gemm, gemm_swiglu
+    n = (n + 31) // 32 * 32 if swiglu else n
+    a, w = _small_integers(m, n, 72, 15)
+    ref = a.float() @ w.float().t()
+    if swiglu:
+        v = ref.view(m, n // 32, 2, 16)
+        ref = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(m, n // 2)
+    for _ in range(4):
+        out = torch.full(ref.shape, 7.0, device="cuda", dtype=torch.bfloat16)
+        (gemm_swiglu if swiglu else gemm)(a, w, out, bn=bn)
+        if swiglu:
+            assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+        else:
+            assert torch.equal(out.float(), ref.to(torch.bfloat16).float())

@@ -97,6 +97,8 @@ class ExpertParallelContext:
 
     def _route_bf16(self, logits: torch.Tensor):
         """``route`` for the bf16 logits that a router GEMM has just written: the same values without a pass that widens them."""
+        if logits.dtype != torch.bfloat16 or not logits.is_contiguous() or logits.dim() != 2 or logits.shape[1] != self.experts:
+            raise ValueError("logits must be contiguous bf16 [tokens, experts]")      # the kernel reads `experts` columns of every row
         rc = self.lib.purlin_moe_route_bf16(self.ctx, logits.data_ptr(), logits.shape[0], 1, self.topk_idx.data_ptr(),
                                             self.topk_weight.data_ptr(), self.slot.data_ptr(), self.stream())
         _native.check(self.lib, rc)

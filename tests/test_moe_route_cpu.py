@@ -65,3 +65,13 @@ def test_usable_values_win_over_masked_ones():
     nan_row[0, 5] = float("nan")
     idx, _ = route_host(nan_row, topk)
     assert 5 not in idx[0].tolist()
+
+
+@pytest.mark.parametrize("logits", [torch.zeros(4, 16, dtype=torch.bfloat16), torch.zeros(4, 64, dtype=torch.bfloat16), torch.zeros(4, 32),
+                                    torch.zeros(32, 4, dtype=torch.bfloat16).t(), torch.zeros(32, dtype=torch.bfloat16)])
+def test_bf16_routing_refuses_logits_that_the_kernel_would_misread(logits):
+    # a router with fewer rows than there are experts must not become a read past its logits; nothing native is reached
+    from types import SimpleNamespace
+    from purlin_b200.parallel.expert_parallel import ExpertParallelContext
+    with pytest.raises(ValueError, match="contiguous bf16"):
+        ExpertParallelContext._route_bf16(SimpleNamespace(experts=32, lib=None), logits)

@@ -7,7 +7,9 @@
     combine: gate-weighted sum of the top-k outputs          (one kernel over peer memory)
 
 DeepSeek-V3-like shapes are the defaults of the benchmark: hidden 7168, 256 experts (32 per GPU at 8 GPUs), top-8.
-Weights are random N(0, 0.02) from a seed; there is no checkpoint loading here.
+Weights are random N(0, 0.02) from a seed; there is no checkpoint loading here. ``w_gu`` and ``w_down`` are best one contiguous
+tensor each, expert after expert: then the experts are two launches. A list of tensors, or a stack with gaps between the experts,
+is computed expert by expert.
 """
 from __future__ import annotations
 
@@ -15,7 +17,7 @@ from typing import Optional
 
 import torch
 
-from ..ops.gemm import gemm, grouped_gemm, interleave_gate_up
+from ..ops.gemm import gemm, gemm_swiglu, grouped_gemm, interleave_gate_up
 from ..parallel.expert_parallel import ExpertParallelContext
 
 
@@ -42,13 +44,31 @@ class ExpertParallelMoE:
         self.ep._route_bf16(gemm(x, self.w_router))
         recv, counts = self.ep.dispatch(x)
         outb = self.ep.out_rows()
-        # one launch per projection; the row counts stay on the device (rows per expert when every rank brings as many tokens)
-        average = -(-t * self.topk * self.ep.world // self.experts)
-        h = grouped_gemm(recv, self.w_gu, counts, average, self._h, swiglu=True)
-        grouped_gemm(h, self.w_down, counts, average, outb)
+        w_gu, w_down = self._in_one_block(self.w_gu), self._in_one_block(self.w_down)
+        if w_gu is not None and w_down is not None:
+            # one launch per projection; the row counts stay on the device (rows per expert when every rank brings as many tokens)
+            average = -(-t * self.topk * self.ep.world // self.experts)
+            h = grouped_gemm(recv, w_gu, counts, average, self._h, swiglu=True)
+            grouped_gemm(h, w_down, counts, average, outb)
+        else:
+            self._expert_by_expert(recv, counts, outb)
         return self.ep.combine(t, out)
 
     __call__ = forward
+
+    def _in_one_block(self, w):
+        """The weights of this rank's experts as one contiguous [experts, N, K], as the grouped GEMM reads them, or None: a list
+        with a tensor per expert, or a stack of which only the slices are contiguous."""
+        n = self.ep.experts_per_rank
+        return w[:n] if isinstance(w, torch.Tensor) and w.dim() == 3 and w.shape[0] >= n and w[:n].is_contiguous() else None
+
+    def _expert_by_expert(self, recv, counts, outb):
+        """The experts when their weights are not one block: two GEMMs each, for which the host has to read the row counts."""
+        offs = [0] + torch.cumsum(counts[: self.ep.experts_per_rank], 0).tolist()
+        for e in range(self.ep.experts_per_rank):
+            a, b = offs[e], offs[e + 1]
+            if b > a:
+                gemm(gemm_swiglu(recv[a:b], self.w_gu[e], self._h[a:b]), self.w_down[e], outb[a:b])
 
     def reference(self, x: torch.Tensor, all_gate=None, all_up=None, all_down=None) -> torch.Tensor:
         """fp32 PyTorch result for a world of one (all experts local)."""

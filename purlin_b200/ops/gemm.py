@@ -77,8 +77,9 @@ def gemm_swiglu(a: torch.Tensor, w_gu: torch.Tensor, out: Optional[torch.Tensor]
 
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_rows: int, out: torch.Tensor, swiglu: bool = False) -> torch.Tensor:
     """``out[rows of e] = a[rows of e] @ w[e].T`` (or the SwiGLU form) for every expert e, in one launch: expert e owns
-    ``counts[e]`` consecutive rows of ``a [rows, K]`` and ``w[e] [N, K]``. ``counts`` (int32) stays on the device; rows beyond
-    the sum of the counts are left alone. ``likely_rows`` says how many rows an expert is expected to have."""
+    ``counts[e]`` consecutive rows of ``a [rows, K]`` and ``w[e] [N, K]``; ``w`` is one contiguous tensor. ``counts`` (int32)
+    stays on the device; rows beyond the sum of the counts are left alone. ``likely_rows`` says how many rows an expert is
+    expected to have."""
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or counts.dtype != torch.int32:
         raise TypeError("the grouped GEMM takes bf16 operands and int32 counts")
     if not (a.is_cuda and w.is_cuda and out.is_cuda and counts.is_cuda):

@@ -76,3 +76,51 @@ def test_sharded_flat_parameter(fakes):
     g = sh.reduce_scatter_grad(average=True)
     assert torch.equal(g, torch.arange(sh.slice_elems, 2 * sh.slice_elems, dtype=torch.float32))   # (x + x) / 2
     assert fakes[-1][0] == "rs" and sh.status() == 0
+
+
+@pytest.mark.parametrize("layout", ["stack", "stack with more experts than are local", "list", "stack with gaps", "down as a list"])
+def test_moe_block_takes_expert_weights_in_one_block_or_one_by_one(monkeypatch, layout):
+    # the exchange and the GEMMs are replaced by plain torch on the CPU; the grouped GEMM's own demands on its operands are kept
+    from types import SimpleNamespace
+    from purlin_b200.models import moe_block
+    rows, hidden, inter, n = 24, 32, 16, 4
+    counts = torch.tensor([5, 0, 12, 3, 20], dtype=torch.int32)              # rows of the local experts, then their total
+    g = torch.Generator().manual_seed(3)
+    recv, outb = torch.randn(rows, hidden, generator=g), torch.full((rows, hidden), 7.0)
+    gu, down = torch.randn(n, 2 * inter, hidden, generator=g), torch.randn(n, hidden, inter, generator=g)
+
+    def product(a, w, out, swiglu):
+        v = a @ w.t()
+        if swiglu:
+            v = v.view(len(a), len(w) // 32, 2, 16)
+            v = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(len(a), len(w) // 2)
+        return out.copy_(v)
+
+    def grouped(a, w, counts, likely, out, swiglu=False):
+        assert isinstance(w, torch.Tensor) and w.dim() == 3 and w.is_contiguous() and len(w) == n
+        first = 0
+        for e in range(n):
+            product(a[first:first + counts[e]], w[e], out[first:first + counts[e]], swiglu)
+            first += int(counts[e])
+        return out
+
+    monkeypatch.setattr(moe_block, "gemm", lambda a, w, out=None: a if out is None else product(a, w, out, False))
+    monkeypatch.setattr(moe_block, "gemm_swiglu", lambda a, w, out: product(a, w, out, True), raising=False)
+    monkeypatch.setattr(moe_block, "grouped_gemm", grouped)
+    moe = object.__new__(moe_block.ExpertParallelMoE)
+    moe.ep = SimpleNamespace(experts_per_rank=n, world=1, _route_bf16=lambda logits: None, dispatch=lambda x: (recv, counts),
+                             out_rows=lambda: outb, combine=lambda t, out: outb)
+    moe.topk, moe.experts, moe.w_router, moe._h = 2, n, None, torch.zeros(rows, inter)
+    moe.w_gu, moe.w_down = gu, down
+    if layout == "stack with more experts than are local":
+        moe.w_gu, moe.w_down = torch.cat([gu, gu]), torch.cat([down, down])
+    elif layout == "list":
+        moe.w_gu, moe.w_down = list(gu), list(down)
+    elif layout == "stack with gaps":
+        moe.w_gu = torch.zeros(n, 2 * inter + 16, hidden)[:, : 2 * inter].copy_(gu)
+    elif layout == "down as a list":
+        moe.w_down = list(down)
+    y = moe(recv)
+    ref = torch.full((rows, hidden), 7.0)
+    grouped(grouped(recv, gu, counts, 1, torch.zeros(rows, inter), swiglu=True), down, counts, 1, ref)
+    assert torch.equal(y, ref)

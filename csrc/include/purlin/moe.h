@@ -45,13 +45,13 @@ int purlin_moe_route_bf16(PurlinMoeContext* ctx, const void* logits, int tokens,
  * [0, experts) are reported through the status word and their pairs dropped. */
 int purlin_moe_plan(PurlinMoeContext* ctx, const int32_t* topkIdx, const float* topkWeight, int tokens, int32_t* slot, void* stream);
 /* x [tokens, hidden] bf16 -> every chosen expert's GPU, in expert-major order in its receive buffer. topkIdx and slot are
- * the arrays of the last route / plan. sentRow [tokens, topk] (optional, may be null: the row of each pair inside its
+ * the arrays of the last route / plan; x may have more rows than were routed (they are not sent), not fewer. sentRow [tokens, topk] (optional, may be null: the row of each pair inside its
  * expert GPU's receive buffer) and recvCounts [experts / world + 1] (rows per local expert, then their total) are
  * outputs. `blocks` > 0 sets how many CTAs send (the rest of the grid receives); 0 picks a default. */
 int purlin_moe_dispatch(PurlinMoeContext* ctx, const void* x, int tokens, const int32_t* topkIdx, const int32_t* slot,
                         int32_t* sentRow, int32_t* recvCounts, int blocks, void* stream);
 /* y [tokens, hidden] = sum over the token's experts of gate weight x expert output row. The weights travelled with the
- * rows at dispatch; topkWeight and sentRow are accepted for symmetry and not read. */
+ * rows at dispatch; topkWeight and sentRow are accepted for symmetry and not read. At most the tokens that were sent. */
 int purlin_moe_combine(PurlinMoeContext* ctx, void* y, int tokens, const int32_t* topkIdx, const float* topkWeight,
                        const int32_t* sentRow, int blocks, void* stream);
 

@@ -51,6 +51,7 @@ struct PurlinMoeContext {
   const int32_t* topkIdx = nullptr;      // routing of the current layer (device pointers the caller owns)
   const float* topkWeight = nullptr;
   const int32_t* slot = nullptr;
+  int routed = 0, dispatched = 0;        // tokens of the last route or plan, and of the one the last dispatch sent
   uint64_t timeoutNs = 0;
   bool timing = false;                   // PURLIN_MOE_TIMING=1: the kernels stamp their phases (purlin_moe_timing)
 };
@@ -652,18 +653,18 @@ bool beginPlan(PurlinMoeContext* c, const int32_t* topkIdx, const float* topkWei
   p.counts = reinterpret_cast<uint32_t*>(lb + c->countsLocalOff);
   p.status = reinterpret_cast<uint32_t*>(lb + 256);
   if (cudaMemsetAsync(p.counts, 0, size_t(c->experts + c->world) * 4, s) != cudaSuccess) { setError("route: clearing the counters failed"); return false; }
-  c->topkIdx = topkIdx; c->topkWeight = topkWeight; c->slot = slot;
+  c->topkIdx = topkIdx; c->topkWeight = topkWeight; c->slot = slot; c->routed = tokens;
   return true;
 }
 
 template <class Logit>
 int routeOn(PurlinMoeContext* c, const Logit* logits, int tokens, int normalize, int32_t* topkIdx, float* topkWeight, int32_t* slot, cudaStream_t s) {
   if (tokens < 0 || tokens > c->maxTokens) { setError("route: more tokens than the context was created for"); return 1; }
-  if (tokens == 0) return 0;
   const int vpl = c->experts / 32;
-  if (vpl != 1 && vpl != 2 && vpl != 4 && vpl != 8 && vpl != 16) { setError("experts / 32 must be 1, 2, 4, 8 or 16"); return 1; }
+  if (tokens > 0 && vpl != 1 && vpl != 2 && vpl != 4 && vpl != 8 && vpl != 16) { setError("experts / 32 must be 1, 2, 4, 8 or 16"); return 1; }
   PlanParams p;
   if (!beginPlan(c, topkIdx, topkWeight, tokens, slot, s, p)) return 1;
+  if (tokens == 0) return 0;             // an empty layer all the same: the counters of the layer before are gone
   const int blocks = (tokens * 32 + kThreads - 1) / kThreads;
   switch (vpl) {
     case 1: routeKernel<1><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
@@ -784,6 +785,8 @@ int purlin_moe_dispatch(PurlinMoeContext* c, const void* x, int tokens, const in
   NvtxRange range("moeDispatch", size_t(tokens));
   if (tokens < 0 || tokens > c->maxTokens) { setError("dispatch: more tokens than the context was created for"); return 1; }
   if (!c->topkIdx || topkIdx != c->topkIdx || slot != c->slot) { setError("dispatch: the routing must come from purlin_moe_route or purlin_moe_plan on this context"); return 1; }
+  if (tokens < c->routed) { setError("dispatch: fewer tokens than were routed"); return 1; }      // the send lists name rows of x
+  c->dispatched = c->routed;
   MoeParams p{};
   fillCommon(p, c, tokens);
   p.x = static_cast<const unsigned char*>(x); p.sentRow = sentRow; p.recvCounts = recvCounts;
@@ -803,6 +806,7 @@ int purlin_moe_combine(PurlinMoeContext* c, void* y, int tokens, const int32_t* 
   (void)topkWeight; (void)sentRow;   // the gate weights travelled with the rows at dispatch
   if (tokens < 0 || tokens > c->maxTokens) { setError("combine: more tokens than the context was created for"); return 1; }
   if (!c->topkIdx || topkIdx != c->topkIdx) { setError("combine: the routing must be the one the matching dispatch used"); return 1; }
+  if (tokens > c->dispatched) { setError("combine: more tokens than the matching dispatch sent"); return 1; }   // nothing will come back for them
   MoeParams p{};
   fillCommon(p, c, tokens);
   p.y = static_cast<unsigned char*>(y);

@@ -26,6 +26,43 @@ def test_exchange_pieces(tokens, hidden, experts, topk):
     assert not fails, fails
 
 
+def test_layers_without_tokens_and_token_counts_that_do_not_match():
+    # a layer with no tokens sends none of the layer before it, and x and y have to fit what was routed
+    from purlin_b200.parallel.expert_parallel import ExpertParallelContext
+    dev = torch.device("cuda", 0)
+    tokens, hidden, experts, topk = 48, 64, 32, 2
+    ep = ExpertParallelContext(None, dev, max_tokens=64, hidden=hidden, experts=experts, topk=topk)
+    g = torch.Generator(device=dev).manual_seed(4)
+    x = torch.randn(tokens, hidden, generator=g, device=dev).to(torch.bfloat16)
+    logits = torch.randn(tokens, experts, generator=g, device=dev)
+    for n in (tokens, 0, tokens, 0, 1):
+        for empty_plan in (False, True):
+            if empty_plan and n == 0:
+                ep.plan(ep.topk_idx[:0], ep.topk_weight[:0])
+            else:
+                ep.route(logits[:n])
+            ep.recv_rows().fill_(3.0)
+            rows, counts = ep.dispatch(x[:n])
+            assert int(counts[:-1].sum()) == int(counts[-1]) == n * topk
+            assert (rows[n * topk:] == 3).all()
+            ep.out_rows().copy_(rows)
+            y = ep.combine(n)
+            ep.check()
+            assert y.shape == (n, hidden) and torch.allclose(y.float(), x[:n].float(), rtol=2 ** -7, atol=1e-6)    # the gate weights sum to one
+    ep.route(logits)
+    with pytest.raises(RuntimeError, match="fewer tokens than were routed"):
+        ep.dispatch(x[:8])
+    padded = torch.cat([x, x[:16]])
+    rows, counts = ep.dispatch(padded)                       # rows past the routed ones are allowed and not sent
+    assert int(counts[-1]) == tokens * topk
+    with pytest.raises(RuntimeError, match="more tokens than the matching dispatch sent"):
+        ep.combine(64)
+    ep.out_rows().copy_(rows)
+    assert torch.allclose(ep.combine(8).float(), x[:8].float(), rtol=2 ** -7, atol=1e-6)
+    ep.check()
+    ep.close()
+
+
 @pytest.mark.multigpu
 def test_moe_all_gpus():
     n = torch.cuda.device_count()

@@ -468,7 +468,11 @@ PURLIN_D void weightedSumAny(unsigned char* out, const unsigned char* const (&ro
   else weightedSum<8, 1>(out, rows, w, n, begin, vecs32, lane);
 }
 
-__global__ void __launch_bounds__(kThreads, kCombineCtasPerSmAlone) combineKernel(const __grid_constant__ MoeParams p) {
+// ALONE > 0: a world of one with top-k up to ALONE. Then there are no pushers and nothing to wait for, and what is left, reading
+// expert rows, is bound by the bytes in flight: two CTAs per SM at 128 registers, with one form of the sum (all three together
+// spill 476 bytes). ALONE = 0: with peers a CTA has an SM and its registers (250) to itself; held to 128 it spills 1540 bytes.
+template <int ALONE>
+__global__ void __launch_bounds__(kThreads, ALONE ? kCombineCtasPerSmAlone : kCombineCtasPerSm) combineKernel(const __grid_constant__ MoeParams p) {
   __shared__ int32_t recvFrom[kMaxRanks];
   __shared__ int bad, nextItem;
   const uint64_t epoch = sig::ldRelaxedSys(p.epoch + 1) + 1;
@@ -480,13 +484,13 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSmAlone) combineKerne
   // combine n follows dispatch n; a call out of order does nothing and is not counted
   const bool outOfOrder = sig::ldRelaxedSys(p.epoch) != epoch;
   if (outOfOrder && tid == 0) { bad = 1; reportBad(p, 10, 0); }
-  if (tid < W) recvFrom[tid] = int(p.countsAll[p.rank][size_t(tid) * stride + p.experts + p.rank]);
+  if (!ALONE && tid < W) recvFrom[tid] = int(p.countsAll[p.rank][size_t(tid) * stride + p.experts + p.rank]);
   __syncthreads();
   const bool ok = __syncthreads_and(!bad && sig::ldRelaxedGpu32(p.status) == 0u) != 0;   // one answer for the whole CTA: the roles below hold barriers
   const int vecs32 = p.hiddenBytes / 32;
   const size_t rowBytes = size_t(p.hiddenBytes);
-  const int senders = W == 1 ? 0 : (p.senders < int(gridDim.x) ? p.senders : int(gridDim.x) - 1);
-  if (ok && int(blockIdx.x) < senders) {
+  const int senders = ALONE ? 0 : (p.senders < int(gridDim.x) ? p.senders : int(gridDim.x) - 1);
+  if (!ALONE && ok && int(blockIdx.x) < senders) {
     // A. pusher: for every row staged here by another rank s, the gate-weighted sum of its expert outputs goes home as ONE row.
     // Items (one chunk of one source) are handed out through a counter in chunk order: the pushers end together, and the
     // chunks complete in the order in which the finishers at home need them (a static split of 232 items over 98 CTAs
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSmAlone) combineKerne
         }
       }
       const unsigned same = __match_any_sync(0xffffffffu, d);
-      const bool remote = d >= 0 && d != p.rank && (__ffs(same) - 1) == lane;
+      const bool remote = !ALONE && d >= 0 && d != p.rank && (__ffs(same) - 1) == lane;
       int good = 1;
       if (remote) good = waitFlag(p, combineFlag(p, p.rank, d, pos / kChunkRows), epoch, 4, d) ? 1 : 0;
       if (!__all_sync(0xffffffffu, good)) return false;
@@ -564,11 +568,13 @@ __global__ void __launch_bounds__(kThreads, kCombineCtasPerSmAlone) combineKerne
         rows[j] = reinterpret_cast<const unsigned char*>(uintptr_t(__shfl_sync(0xffffffffu, at, from)));
         w[j] = __shfl_sync(0xffffffffu, weight, from);
       }
-      weightedSumAny(p.y + size_t(t) * rowBytes, rows, w, n, begin, end, lane);
+      unsigned char* y = p.y + size_t(t) * rowBytes;
+      if constexpr (ALONE > 0) weightedSum<ALONE, 8 / ALONE>(y, rows, w, n, begin, end, lane);
+      else weightedSumAny(y, rows, w, n, begin, end, lane);
       return true;
     };
-    if (W == 1) {
-      // nothing to wait for: the output is one list of 1 KiB pieces, cut evenly over the warps of the grid
+    if constexpr (ALONE > 0) {
+      // the output is one list of 1 KiB pieces, cut evenly over the warps of the grid
       const int perRow = (vecs32 + 31) / 32;
       const int64_t pieces = int64_t(p.tokens) * perRow, nw = int64_t(nFin) * kWarps, wi = int64_t(warp) * nFin + me;
       int64_t u = pieces * wi / nw;
@@ -815,7 +821,8 @@ int purlin_moe_combine(PurlinMoeContext* c, void* y, int tokens, const int32_t* 
   // 343 us; 98 pushers 366 us, 110 pushers 392 us): the finishers end last. The pushers now have (W - 1) / W of that work and
   // the finishers the rest, so their number shrinks with it (bytes per CTA as measured; not timed again on several GPUs).
   p.senders = blocks > 0 ? std::min(blocks, grid - 1) : std::max(grid * 54 * (c->world - 1) / (100 * c->world), 1);
-  combineKernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  auto kernel = c->world > 1 ? combineKernel<0> : c->topk <= 2 ? combineKernel<2> : c->topk <= 4 ? combineKernel<4> : combineKernel<8>;
+  kernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { setError(std::string("combine launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;

@@ -5,6 +5,8 @@ import threading
 import time
 from pathlib import Path
 
+import pytest
+
 from purlin_b200 import _build
 
 
@@ -83,3 +85,17 @@ def test_concurrent_callers_build_once(tmp_path, monkeypatch):
     (src / "one.cpp").write_text("int one() { return 2; }\n")
     build()
     assert len(compiles) == 2, "changed contents rebuild"
+
+
+def test_the_combine_keeps_its_loads_in_registers(tmp_path):
+    # Every form of the MoE combine holds 8 x 32 bytes per lane in flight; a launch bound that it does not fit spills them.
+    import shutil
+    import subprocess
+    nvcc = _build._nvcc()
+    if not shutil.which(nvcc):
+        pytest.skip("no CUDA compiler")
+    res = subprocess.run([nvcc, *_build.NVCC_FLAGS, "-I", str(_build.CSRC / "include"), "-Xptxas", "-v", "-c",
+                          str(_build.CSRC / "src" / "moe.cu"), "-o", str(tmp_path / "moe.o")], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    reports = [part for part in res.stderr.split("Compiling entry function")[1:] if "combineKernel" in part.splitlines()[0]]
+    assert reports and all("0 bytes spill stores, 0 bytes spill loads" in part for part in reports), reports

@@ -88,21 +88,23 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   tc::gridDependencyWait();                                    // from here on memory that earlier kernels write may be read
   if (warp == 2) {
     // rows and tiles of every expert, as running sums: 32 experts per step
-    int rows0 = 0, items0 = 0;
+    const uint32_t limit = uint32_t(p.tokens);
+    uint32_t rows0 = 0;
+    int items0 = 0;
     for (int e0 = 0; e0 < p.experts; e0 += 32) {
       const int e = e0 + lane;
-      int r = e < p.experts ? (p.counts ? max(p.counts[e], 0) : p.tokens) : 0;
-      int sum = r;
+      uint32_t sum = e < p.experts ? (p.counts ? skinny::groupRowsOf(p.counts[e], limit) : limit) : 0u;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
-      const int first = min(rows0 + sum - r, p.tokens);
-      r = min(r, p.tokens - first);                                    // never past the buffers, whatever the counts say
+      for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum = skinny::addRows(sum, v, limit); }
+      const uint32_t before = __shfl_up_sync(0xffffffffu, sum, 1);
+      const int first = int(lane ? skinny::addRows(rows0, before, limit) : rows0), end = int(skinny::addRows(rows0, sum, limit));
+      const int r = end - first;
       const int n = r > 0 ? tilesOf(r) * wTiles : 0;
       int items = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, items, o); if (lane >= o) items += v; }
-      if (e < p.experts) { rowStart[e] = first; itemStart[e] = items0 + items - n; rowStart[e + 1] = first + r; itemStart[e + 1] = items0 + items; }
-      rows0 += __shfl_sync(0xffffffffu, sum, 31);
+      if (e < p.experts) { rowStart[e] = first; itemStart[e] = items0 + items - n; rowStart[e + 1] = end; itemStart[e + 1] = items0 + items; }
+      rows0 = skinny::addRows(rows0, __shfl_sync(0xffffffffu, sum, 31), limit);
       items0 += __shfl_sync(0xffffffffu, items, 31);
       __syncwarp();
     }

@@ -47,6 +47,11 @@ PURLIN_D void recordTimeout(uint32_t* status, uint32_t where, uint32_t a, uint32
   if (status && atomicCAS(status, 0u, uint32_t(kStatusTimeoutBarrier)) == 0u) { status[1] = where; status[2] = a; status[3] = b; __threadfence(); }
 }
 
+// Rows of a group and sums of them never count past the `limit` rows that there are, whatever the counts say: a count is cut to
+// [0, limit] and a sum stays at the limit (neither term is above it, so the unsigned sum cannot wrap).
+PURLIN_D uint32_t groupRowsOf(int32_t count, uint32_t limit) { return count > 0 ? min(uint32_t(count), limit) : 0u; }
+PURLIN_D uint32_t addRows(uint32_t a, uint32_t b, uint32_t limit) { return min(a + b, limit); }
+
 // (volatile keeps these loads behind the cluster barriers; they may overlap one another and the sums)
 PURLIN_D float4 ldCluster4(uint32_t addr) {
   float4 v;
@@ -130,14 +135,15 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
   if (warp == 1) { tc::tmemAlloc(tc::smemAddr(words), uint32_t(p.tmemCols)); tc::tmemRelinquish(); }
   tc::gridDependencyWait();                                   // from here on memory that earlier kernels write may be read
   if (warp == 2) {
-    int first = 0, rows = p.tokens;
+    const uint32_t limit = uint32_t(p.tokens);
+    uint32_t first = 0, rows = limit;
     if (p.counts) {
-      for (int e = lane; e < expert; e += 32) first += max(p.counts[e], 0);
+      for (int e = lane; e < expert; e += 32) first = addRows(first, groupRowsOf(p.counts[e], limit), limit);
 #pragma unroll
-      for (int o = 16; o; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
-      rows = min(max(p.counts[expert], 0), max(p.tokens - first, 0));    // never past the buffers, whatever the counts say
+      for (int o = 16; o; o >>= 1) first = addRows(first, __shfl_xor_sync(0xffffffffu, first, o), limit);
+      rows = min(groupRowsOf(p.counts[expert], limit), limit - first);
     }
-    if (lane == 0) { groupRows[0] = first; groupRows[1] = rows; }
+    if (lane == 0) { groupRows[0] = int(first); groupRows[1] = int(rows); }
   }
   tc::fenceBeforeThreadSync();
   __syncthreads();

@@ -173,3 +173,21 @@ def test_tiles_wider_than_the_output_are_exact_on_small_integers(m, n, bn, swigl
             assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
         else:
             assert torch.equal(out.float(), ref.to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("likely", [1, 400])
+@pytest.mark.parametrize("counts", [[100, 200, 30, 300], [0, 256, 1, 0], [300, 5, 5, 5], [10, -7, 20, -1], [2 ** 31 - 1] * 4, [255] + [2 ** 31 - 1] * 45, [1] * 300])
+def test_grouped_gemm_counts_never_lead_past_the_rows(likely, counts):
+    # counts that add up to more than the 256 rows, and past 2^31: groups are cut at the last row, later ones are empty
+    from purlin_b200.ops.gemm import grouped_gemm
+    rows, n, k = 256, 40, 72
+    a, w = _small_integers(rows, len(counts) * n, k, 16)
+    guard = torch.full((rows + 64, n), 7.0, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w.view(len(counts), n, k), torch.tensor(counts, dtype=torch.int32, device="cuda"), likely, guard[32:32 + rows])
+    ref, first = torch.full((rows, n), 7.0, device="cuda"), 0
+    for e, c in enumerate(counts):
+        end = min(first + max(c, 0), rows)
+        ref[first:end] = a[first:end].float() @ w[e * n:(e + 1) * n].float().t()
+        first = end
+    assert torch.equal(guard[32:32 + rows].float(), ref)
+    assert (guard[:32] == 7).all() and (guard[32 + rows:] == 7).all()

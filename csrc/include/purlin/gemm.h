@@ -11,7 +11,7 @@ extern "C" {
 enum { PURLIN_EPI_STORE = 0, PURLIN_EPI_SWIGLU = 1 };
 
 /* C[M,N] = A[M,K] * B[N,K]^T, bf16 row-major operands (K contiguous), fp32 accumulation, bf16 output.
- * PURLIN_EPI_SWIGLU: B's rows alternate 16 gate rows and 16 up rows; C is [M, N/2] = silu(gate) * up.
+ * PURLIN_EPI_SWIGLU: B's rows alternate 16 gate rows and 16 up rows (N a multiple of 32); C is [M, N/2] = silu(gate) * up.
  * bn: tile width (multiple of 16, at most 256); 0 lets the library choose. status: 4 device words or NULL. */
 int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int bn,
                      uint32_t* status, void* stream);

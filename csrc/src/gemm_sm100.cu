@@ -712,9 +712,17 @@ int ctasFor(int M, int rowsPerRank) {
 
 struct Shape { int ctas, accs; };
 
+// The SwiGLU epilogue takes the rows of W as 16 of gate and 16 of up in turn: half a group has no up rows of its own.
+bool epilogueFits(int N, int epilogue) {
+  if (epilogue != kEpiStore && epilogue != kEpiSwiglu) { setError("unknown epilogue"); return false; }
+  if (epilogue == kEpiSwiglu && N % 32) { setError("the SwiGLU epilogue needs N to be a multiple of 32"); return false; }
+  return true;
+}
+
 bool fillShape(Params& p, Shape& sh, int M, int N, int K, int epilogue, int bn, int rowsPerRank, int accsWanted = 0) {
   if (M <= 0 || N <= 0 || K <= 0) { setError("GEMM dimensions must be positive"); return false; }
   if (K % 8 || N % 8) { setError("N and K must be multiples of 8"); return false; }
+  if (!epilogueFits(N, epilogue)) return false;
   const int ctas = ctasFor(M, rowsPerRank);
   if (bn == 0) bn = chooseBn(M, N, epilogue);
   if (bn % 32 || bn < 32 || bn > kMaxBN) { setError("tile width must be a multiple of 32 up to 256"); return false; }
@@ -1038,6 +1046,8 @@ int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, in
   NvtxRange range(epilogue == kEpiSwiglu ? "groupedGemmSwiglu" : "groupedGemm", size_t(rows) * size_t(N) * 2);
   if (rows <= 0 || N <= 0 || K <= 0 || experts <= 0 || !counts) { setError("grouped GEMM: dimensions must be positive and counts given"); return 1; }
   if (K % 8 || N % 8) { setError("N and K must be multiples of 8"); return 1; }
+  if (!epilogueFits(N, epilogue)) return 1;
+  if (int64_t(experts) * N > INT32_MAX) { setError("grouped GEMM: the rows of all experts' weights must fit 32 bits"); return 1; }   // TMA row coordinates
   static thread_local MapCache cache;
   GroupedArgs g;
   g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);

@@ -89,6 +89,8 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_
     experts, n, k = w.shape
     if a.shape[1] != k or out.shape != (a.shape[0], n // 2 if swiglu else n) or counts.numel() < experts:
         raise ValueError("a is [rows, K], w is [experts, N, K], out is [rows, N or N / 2] and counts has an entry per expert")
+    if swiglu and n % 32:
+        raise ValueError("the SwiGLU epilogue needs N to be a multiple of 32 (16 rows of gate and 16 of up in turn)")
     lib = _lib()
     rc = lib.purlin_gemm_grouped_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], experts, n, k, counts.data_ptr(), likely_rows,
                                       EPI_SWIGLU if swiglu else EPI_STORE, _stream(None))

@@ -284,3 +284,23 @@ def test_fastcall_extension_passes_the_seven_scalars_unchanged():
     assert fast is not lib.purlin_call_fixed or os.environ.get("PURLIN_NO_FASTCALL")
     assert fast(0, 0, 0, 0, 64, 4, 0) == 1
     assert "null context" in _native.last_error(lib)
+
+
+@pytest.mark.parametrize("args,message", [((64, 4, 48, 64, 1), "multiple of 32"), ((64, 4, 40, 64, 1), "multiple of 32"), ((64, 4, 64, 64, 2), "unknown epilogue"),
+                                          ((64, 512, 1 << 23, 64, 0), "32 bits"), ((64, 4, 64, 60, 0), "multiples of 8"), ((0, 4, 64, 64, 0), "positive")])
+def test_grouped_gemm_refuses_sizes_it_would_compute_wrongly(args, message):
+    # host-side checks, before anything is launched: (rows, experts, N, K, epilogue)
+    from purlin_b200.ops.gemm import _lib
+    lib = _lib()
+    rows, experts, n, k, epilogue = args
+    counts = (C.c_int32 * experts)()
+    assert lib.purlin_gemm_grouped_bf16(0, 0, 0, rows, experts, n, k, C.addressof(counts), 16, epilogue, None) != 0
+    assert message in _native.last_error(lib)
+
+
+@pytest.mark.parametrize("n,epilogue,message", [(48, 1, "multiple of 32"), (64, 7, "unknown epilogue")])
+def test_gemm_refuses_half_a_group_of_gate_and_up_rows(n, epilogue, message):
+    from purlin_b200.ops.gemm import _lib
+    lib = _lib()
+    assert lib.purlin_gemm_bf16(0, 0, 0, 16, n, 64, epilogue, 0, None, None) != 0
+    assert message in _native.last_error(lib)

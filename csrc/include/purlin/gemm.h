@@ -18,9 +18,11 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
 
 /* The same product per group of rows: expert e owns counts[e] consecutive rows of A and C and rows [e * N, (e + 1) * N)
  * of B. counts: device words, read by the kernel (no host synchronisation); rows: rows of A and C, an upper bound of the sum
- * of the counts. likelyRows: rows a group is expected to have (a hint for speed; any counts are computed). */
+ * of the counts. likelyRows: rows a group is expected to have (a hint for speed; any counts are computed). status: 4 device
+ * words or NULL, {code, where, tile, k-block} of the first wait that took longer than timeoutNs (0: two seconds); what the
+ * kernel had not finished by then is not written. */
 int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, int experts, int N, int K, const int32_t* counts,
-                             int likelyRows, int epilogue, void* stream);
+                             int likelyRows, int epilogue, uint32_t* status, uint64_t timeoutNs, void* stream);
 
 typedef struct PurlinTpContext PurlinTpContext;
 

@@ -55,6 +55,11 @@ PURLIN_D bool mbarWait(uint32_t bar, uint32_t parity, volatile int* abortWord, u
   }
   return true;
 }
+// For the way out after a wait gave up: copies and MMAs that are under way end by themselves, so this one has only a limit.
+PURLIN_D void mbarDrain(uint32_t bar, uint32_t parity) {
+  const uint64_t start = sig::globalTimerNs();
+  while (!mbarTryWait(bar, parity) && sig::globalTimerNs() - start < 1000ull * 1000 * 1000) {}
+}
 
 // ---- TMA (tile mode, this CTA only) ----
 PURLIN_D void tmaLoad2d(uint32_t smemDst, const CUtensorMap* map, int x, int y, uint32_t bar) {

@@ -833,6 +833,7 @@ struct GroupedArgs {
   int experts = 1;                    // groups of rows; 1 with counts == nullptr: a plain GEMM
   const int32_t* counts = nullptr;    // device: rows of every group
   int likelyRows = 0;                 // rows a group is expected to have
+  uint64_t timeoutNs = 2ull * 1000 * 1000 * 1000;   // of every wait inside the kernel
 };
 
 // Which GEMMs the few-rows kernel takes, each line with one B200's times in us, it / the other tiles. Few rows of W (a router)
@@ -861,7 +862,7 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   if (tokenRows) { std::swap(A, B); std::swap(M, N); }
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status;
-  p.timeoutNs = 2ull * 1000 * 1000 * 1000;
+  p.timeoutNs = g.timeoutNs;
   // one pass has to hold a group's rows (a second pass reads W again): a group of average size has twice the room
   const int room = std::min(g.counts ? 2 * g.likelyRows + 16 : M, M);
   p.tokenBox = room <= 16 ? 16 : 32;
@@ -945,7 +946,7 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   }
   ragged::Params p{};
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.experts = g.experts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
-  p.stages = stages; p.status = status; p.timeoutNs = 2ull * 1000 * 1000 * 1000;
+  p.stages = stages; p.status = status; p.timeoutNs = g.timeoutNs;
   const int wTiles = (N + ragged::kTileRows - 1) / ragged::kTileRows;
   int items = INT32_MAX;
   p.tileCols = ragged::kMaxCols; p.xBox = 32;
@@ -1042,7 +1043,7 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
 // has a CTA per 128 weight rows (32 experts, gate-up 4096 x 7168 + down 7168 x 2048, us, pairs / few rows: 1 row 306 / 283, 4
 // rows 435 / 425, 16 rows 456 / 462, 32 rows 463 / 473, 64 rows 466 / 543).
 int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, int experts, int N, int K, const int32_t* counts, int likelyRows,
-                             int epilogue, void* stream) {
+                             int epilogue, uint32_t* status, uint64_t timeoutNs, void* stream) {
   NvtxRange range(epilogue == kEpiSwiglu ? "groupedGemmSwiglu" : "groupedGemm", size_t(rows) * size_t(N) * 2);
   if (rows <= 0 || N <= 0 || K <= 0 || experts <= 0 || !counts) { setError("grouped GEMM: dimensions must be positive and counts given"); return 1; }
   if (K % 8 || N % 8) { setError("N and K must be multiples of 8"); return 1; }
@@ -1051,7 +1052,8 @@ int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, in
   static thread_local MapCache cache;
   GroupedArgs g;
   g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);
-  return (g.likelyRows <= kFewGroupRows ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, nullptr, static_cast<cudaStream_t>(stream));
+  if (timeoutNs) g.timeoutNs = timeoutNs;
+  return (g.likelyRows <= kFewGroupRows ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, status, static_cast<cudaStream_t>(stream));
 }
 
 size_t purlin_tp_workspace_bytes(int world, int M, int kAg, int nRs) { return tpLayout(world, M, kAg, nRs).total; }

@@ -23,7 +23,7 @@ def _lib():
     if not _declared:
         vp, i = C.c_void_p, C.c_int
         lib.purlin_gemm_bf16.argtypes = [vp, vp, vp, i, i, i, i, i, vp, vp]
-        lib.purlin_gemm_grouped_bf16.argtypes = [vp, vp, vp, i, i, i, i, vp, i, i, vp]
+        lib.purlin_gemm_grouped_bf16.argtypes = [vp, vp, vp, i, i, i, i, vp, i, i, vp, C.c_uint64, vp]
         _declared = True
     return lib
 
@@ -75,11 +75,13 @@ def gemm_swiglu(a: torch.Tensor, w_gu: torch.Tensor, out: Optional[torch.Tensor]
     return out
 
 
-def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_rows: int, out: torch.Tensor, swiglu: bool = False) -> torch.Tensor:
+def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_rows: int, out: torch.Tensor, swiglu: bool = False,
+                 status_ptr: int = 0, timeout_ns: int = 0) -> torch.Tensor:
     """``out[rows of e] = a[rows of e] @ w[e].T`` (or the SwiGLU form) for every expert e, in one launch: expert e owns
     ``counts[e]`` consecutive rows of ``a [rows, K]`` and ``w[e] [N, K]``; ``w`` is one contiguous tensor. ``counts`` (int32)
     stays on the device; rows beyond the sum of the counts are left alone. ``likely_rows`` says how many rows an expert is
-    expected to have."""
+    expected to have. ``status_ptr``: four device words for the first wait inside the kernel that took longer than
+    ``timeout_ns`` (0: two seconds); rows that were not finished by then are left alone too."""
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or counts.dtype != torch.int32:
         raise TypeError("the grouped GEMM takes bf16 operands and int32 counts")
     if not (a.is_cuda and w.is_cuda and out.is_cuda and counts.is_cuda):
@@ -93,6 +95,6 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, likely_
         raise ValueError("the SwiGLU epilogue needs N to be a multiple of 32 (16 rows of gate and 16 of up in turn)")
     lib = _lib()
     rc = lib.purlin_gemm_grouped_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], experts, n, k, counts.data_ptr(), likely_rows,
-                                      EPI_SWIGLU if swiglu else EPI_STORE, _stream(None))
+                                      EPI_SWIGLU if swiglu else EPI_STORE, status_ptr or None, timeout_ns, _stream(None))
     _native.check(lib, rc)
     return out

@@ -191,3 +191,26 @@ def test_grouped_gemm_counts_never_lead_past_the_rows(likely, counts):
         first = end
     assert torch.equal(guard[32:32 + rows].float(), ref)
     assert (guard[:32] == 7).all() and (guard[32 + rows:] == 7).all()
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_a_wait_that_runs_out_reports_and_leaves_no_half_sums(swiglu):
+    # k so long that the wait for the accumulator outlasts its limit in some CTAs of a cluster: their peers must not add what is
+    # not a partial tile. A row piece is the product or untouched, the status says which wait it was, the next call is whole.
+    from purlin_b200.ops.gemm import grouped_gemm
+    rows, n, k = 8, 64, 1 << 21
+    a = torch.zeros(rows, k, device="cuda", dtype=torch.bfloat16)
+    a[:, ::4096] = 1
+    w = torch.full((1, n, k), 0.125, device="cuda", dtype=torch.bfloat16)
+    counts = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    width = n // 2 if swiglu else n
+    ref = torch.full((rows, width), 64.0 * 64.0 if swiglu else 64.0, device="cuda")      # 512 ones x 0.125; silu(64) = 64 in fp32
+    out = torch.full((rows, width), 7.0, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w, counts, rows, out, swiglu=swiglu, status_ptr=status.data_ptr(), timeout_ns=1)
+    torch.cuda.synchronize()
+    assert status[0].item() == 5 and status[1].item() in (1, 3, 5)
+    assert ((out == 7) | (out.float() == ref)).all()
+    status.zero_()
+    grouped_gemm(a, w, counts, rows, out, swiglu=swiglu, status_ptr=status.data_ptr())
+    assert status[0].item() == 0 and torch.equal(out.float(), ref)

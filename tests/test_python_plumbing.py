@@ -294,7 +294,7 @@ def test_grouped_gemm_refuses_sizes_it_would_compute_wrongly(args, message):
     lib = _lib()
     rows, experts, n, k, epilogue = args
     counts = (C.c_int32 * experts)()
-    assert lib.purlin_gemm_grouped_bf16(0, 0, 0, rows, experts, n, k, C.addressof(counts), 16, epilogue, None) != 0
+    assert lib.purlin_gemm_grouped_bf16(0, 0, 0, rows, experts, n, k, C.addressof(counts), 16, epilogue, None, 0, None) != 0
     assert message in _native.last_error(lib)
 
 

@@ -26,6 +26,7 @@ PurlinMoeContext* purlin_moe_create(int rank, int world, const uint64_t* peerPtr
 int purlin_moe_destroy(PurlinMoeContext* ctx, void* stream);
 int purlin_moe_status(PurlinMoeContext* ctx, uint32_t* out4, void* stream);
 int purlin_moe_clear_status(PurlinMoeContext* ctx, void* stream);
+uint32_t* purlin_moe_status_words(PurlinMoeContext* ctx);   /* the four device words themselves, for the experts' kernels to report into */
 /* Diagnostics (contexts created with PURLIN_MOE_TIMING=1): nanoseconds from the first CTA's start to {last sender end, last
  * receiver end, first sender end, 0} of the dispatches and {last pusher end, last finisher end, first pusher end, 0} of the
  * combines since the previous call of this function. Synchronises the stream. */

@@ -759,6 +759,7 @@ int purlin_moe_timing(PurlinMoeContext* c, uint64_t* out8, void* stream) {
 int purlin_moe_clear_status(PurlinMoeContext* c, void* stream) {
   return cudaMemsetAsync(static_cast<unsigned char*>(c->local) + 256, 0, 16, static_cast<cudaStream_t>(stream)) == cudaSuccess ? 0 : 1;
 }
+uint32_t* purlin_moe_status_words(PurlinMoeContext* c) { return reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(c->local) + 256); }
 void* purlin_moe_recv_buffer(PurlinMoeContext* c) { return c->peers[c->rank] + c->recvOff; }
 void* purlin_moe_out_buffer(PurlinMoeContext* c) { return c->peers[c->rank] + c->outOff; }
 

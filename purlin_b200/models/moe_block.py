@@ -48,8 +48,9 @@ class ExpertParallelMoE:
         if w_gu is not None and w_down is not None:
             # one launch per projection; the row counts stay on the device (rows per expert when every rank brings as many tokens)
             average = -(-t * self.topk * self.ep.world // self.experts)
-            h = grouped_gemm(recv, w_gu, counts, average, self._h, swiglu=True)
-            grouped_gemm(h, w_down, counts, average, outb)
+            report = {"status_ptr": self.ep.status_ptr, "timeout_ns": self.ep.timeout_ns}     # ep.check() covers the experts too
+            h = grouped_gemm(recv, w_gu, counts, average, self._h, swiglu=True, **report)
+            grouped_gemm(h, w_down, counts, average, outb, **report)
         else:
             self._expert_by_expert(recv, counts, outb)
         return self.ep.combine(t, out)

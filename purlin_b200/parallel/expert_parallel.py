@@ -35,6 +35,8 @@ def _lib():
         lib.purlin_moe_status.argtypes = [vp, C.POINTER(C.c_uint32), vp]
         lib.purlin_moe_clear_status.argtypes = [vp, vp]
         lib.purlin_moe_timing.argtypes = [vp, C.POINTER(u64), vp]
+        lib.purlin_moe_status_words.restype = vp
+        lib.purlin_moe_status_words.argtypes = [vp]
         lib.purlin_moe_recv_buffer.restype = vp
         lib.purlin_moe_recv_buffer.argtypes = [vp]
         lib.purlin_moe_out_buffer.restype = vp
@@ -74,6 +76,8 @@ class ExpertParallelContext:
                                               timeout_ms * 1_000_000, self.stream())
         if not self.ctx:
             raise RuntimeError("purlin: " + _native.last_error(self.lib))
+        # where kernels of the experts report a wait that ran out, so that check() sees it like one of the exchange's own
+        self.status_ptr, self.timeout_ns = self.lib.purlin_moe_status_words(self.ctx), timeout_ms * 1_000_000
         dev = self.device
         self.topk_idx = torch.empty(max_tokens, topk, dtype=torch.int32, device=dev)
         self.topk_weight = torch.empty(max_tokens, topk, dtype=torch.float32, device=dev)
@@ -152,7 +156,8 @@ class ExpertParallelContext:
             self.lib.purlin_moe_clear_status(self.ctx, self.stream())
             what = {2: "receive buffer capacity exceeded", 3: "more rows for one destination than the staging area holds",
                     7: "an expert id outside [0, experts)", 9: "dispatch called twice without a combine in between",
-                    10: "combine called without a matching dispatch"}.get(out[1], "bad plan") if out[0] == 6 else "a wait timed out"
+                    10: "combine called without a matching dispatch"}.get(out[1], "bad plan") if out[0] == 6 else \
+                "a wait inside a GEMM of the experts timed out" if out[0] == 5 else "a wait timed out"
             raise RuntimeError(f"purlin: MoE exchange failed: {what} (where {out[1]}, peer {out[2]})")
 
     def timing(self):

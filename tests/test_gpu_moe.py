@@ -63,6 +63,24 @@ def test_layers_without_tokens_and_token_counts_that_do_not_match():
     ep.close()
 
 
+def test_check_sees_a_wait_that_ran_out_in_the_experts_gemm():
+    # a grouped GEMM over a k so long that the wait for its accumulator outlasts a limit of 1 ns, reporting where the block's report
+    from purlin_b200.models.moe_block import ExpertParallelMoE
+    from purlin_b200.ops.gemm import grouped_gemm
+    moe = ExpertParallelMoE(hidden=128, intermediate=64, experts=32, topk=2, max_tokens=16, device="cuda:0")
+    x = torch.ones(16, 128, device="cuda", dtype=torch.bfloat16)
+    y = moe(x)
+    moe.ep.check()
+    a, w = torch.zeros(8, 1 << 21, device="cuda", dtype=torch.bfloat16), torch.zeros(1, 64, 1 << 21, device="cuda", dtype=torch.bfloat16)
+    out = torch.zeros(8, 64, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w, torch.tensor([8], dtype=torch.int32, device="cuda"), 8, out, status_ptr=moe.ep.status_ptr, timeout_ns=1)
+    with pytest.raises(RuntimeError, match="inside a GEMM of the experts timed out"):
+        moe.ep.check()
+    assert torch.equal(moe(x), y)                            # the report is cleared, the next layer runs
+    moe.ep.check()
+    moe.ep.close()
+
+
 @pytest.mark.multigpu
 def test_moe_all_gpus():
     n = torch.cuda.device_count()

@@ -96,7 +96,8 @@ def test_moe_block_takes_expert_weights_in_one_block_or_one_by_one(monkeypatch, 
             v = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(len(a), len(w) // 2)
         return out.copy_(v)
 
-    def grouped(a, w, counts, likely, out, swiglu=False):
+    def grouped(a, w, counts, likely, out, swiglu=False, status_ptr=4096, timeout_ns=77):
+        assert (status_ptr, timeout_ns) == (4096, 77)                        # the exchange's own words and limit
         assert isinstance(w, torch.Tensor) and w.dim() == 3 and w.is_contiguous() and len(w) == n
         first = 0
         for e in range(n):
@@ -108,7 +109,7 @@ def test_moe_block_takes_expert_weights_in_one_block_or_one_by_one(monkeypatch, 
     monkeypatch.setattr(moe_block, "gemm_swiglu", lambda a, w, out: product(a, w, out, True), raising=False)
     monkeypatch.setattr(moe_block, "grouped_gemm", grouped)
     moe = object.__new__(moe_block.ExpertParallelMoE)
-    moe.ep = SimpleNamespace(experts_per_rank=n, world=1, _route_bf16=lambda logits: None, dispatch=lambda x: (recv, counts),
+    moe.ep = SimpleNamespace(experts_per_rank=n, world=1, status_ptr=4096, timeout_ns=77, _route_bf16=lambda logits: None, dispatch=lambda x: (recv, counts),
                              out_rows=lambda: outb, combine=lambda t, out: outb)
     moe.topk, moe.experts, moe.w_router, moe._h = 2, n, None, torch.zeros(rows, inter)
     moe.w_gu, moe.w_down = gu, down

@@ -214,3 +214,41 @@ def test_a_wait_that_runs_out_reports_and_leaves_no_half_sums(swiglu):
     status.zero_()
     grouped_gemm(a, w, counts, rows, out, swiglu=swiglu, status_ptr=status.data_ptr())
     assert status[0].item() == 0 and torch.equal(out.float(), ref)
+
+
+def _swiglu_ref(a, w):
+    v = (a.float() @ w.float().t()).view(a.shape[0], w.shape[0] // 32, 2, 16)
+    return (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(a.shape[0], w.shape[0] // 2)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 7168, 8192), (33, 1024, 4096), (64, 14336, 2048), (16, 64, 8200), (128, 2080, 1032)])
+def test_few_rows_swiglu_with_the_k_range_split(m, n, k):
+    # gate and up are summed over a cluster of two to eight CTAs; both sums are exact, so what is left is one rounding to bf16
+    from purlin_b200.ops.gemm import gemm_swiglu
+    a, w = _small_integers(m, n, k, 17)
+    ref = _swiglu_ref(a, w)
+    assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("likely,n,k,counts", [
+    (1, 64, 4104, [100, 0, 515]), (1, 544, 1032, [33, 1, 0, 64, 200]),                # several passes of a cluster of eight, of four
+    (12, 160, 2048, [300, 40, 0, 41]),
+    (400, 96, 72, [7] * 33), (400, 64, 136, [0, 65, 1, 300] * 16), (400, 32, 72, [1, 0, 3, 2] * 128),      # 33, 64, 512 groups in the scan
+    (5, 32, 72, [1, 0, 3, 2] * 128)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_grouped_gemm_split_over_clusters_and_over_many_groups(likely, n, k, counts, swiglu):
+    from purlin_b200.ops.gemm import grouped_gemm
+    rows, experts = sum(counts) + 5, len(counts)
+    a, w = _small_integers(rows, experts * n, k, 18)
+    out = torch.full((rows, n // 2 if swiglu else n), 7.0, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w.view(experts, n, k), torch.tensor(counts, dtype=torch.int32, device="cuda"), likely, out, swiglu=swiglu)
+    ref, first = torch.full(out.shape, 7.0, device="cuda"), 0
+    for e, c in enumerate(counts):
+        ae, we = a[first:first + c], w[e * n:(e + 1) * n]
+        if c:
+            ref[first:first + c] = _swiglu_ref(ae, we) if swiglu else (ae.float() @ we.float().t()).to(torch.bfloat16).float()
+        first += c
+    if swiglu:
+        assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+    else:
+        assert torch.equal(out.float(), ref)

@@ -110,6 +110,24 @@ def test_moe_block_world_of_one_matches_fp32_reference():
     assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("tokens", [1, 7, 48, 120])
+def test_moe_block_decode_batches_match_the_fp32_reference(tokens):
+    # up to a dozen rows per expert the few-rows kernel computes the experts, above it the one on CTA pairs (15 rows at 120 tokens)
+    from purlin_b200.models.moe_block import ExpertParallelMoE
+    moe = ExpertParallelMoE(hidden=1024, intermediate=512, experts=32, topk=4, max_tokens=120, device="cuda:0", capacity_factor=1.0)
+    g = torch.Generator(device="cuda:0").manual_seed(tokens)
+    x = torch.randn(tokens, 1024, generator=g, device="cuda:0").to(torch.bfloat16)
+    y = moe(x)
+    moe.ep.check()
+    ref = moe.reference(x)
+    assert (y.float() - ref).abs().max().item() <= 3e-2 * ref.abs().max().item() + 2e-3
+    stacked = moe.w_gu, moe.w_down
+    moe.w_gu, moe.w_down = list(moe.w_gu), list(moe.w_down)                       # expert by expert: the same products
+    assert ((moe(x).float() - y.float()).abs() <= 2 ** -6 * y.float().abs() + 2 ** -7 * ref.abs().max()).all()
+    moe.w_gu, moe.w_down = stacked
+    moe.ep.close()
+
+
 def test_route_kernel_is_total_and_matches_the_host_restatement():
     """Rows of NaN, +inf, -inf and rows with fewer than top-k usable logits: the kernel must return k distinct experts
     inside [0, experts) with finite weights, equal to the host restatement of the same arithmetic."""

@@ -157,16 +157,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
 #pragma unroll
   for (int q = 0; q < kMaxSplit; ++q) peer[q] = uint32_t(q) < split ? tc::mapToCta(base, uint32_t(q)) : 0u;
 
-  // A wait that gave up is everybody's business: the partial tile of this CTA is not what its peers would add. They learn of it
-  // through their own abort words, written before the cluster barrier after which they are read.
-  auto giveUp = [&](uint32_t where, int kb) {
-    recordTimeout(p.status, where, tile, kb);
-    const uint32_t word = tc::smemAddr(words + 1);
-    for (uint32_t q = 0; q < split; ++q) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(tc::mapToCta(word, q)), "r"(1) : "memory");
-  };
-
   uint32_t st = 0, ph = 0;                                    // ring position and phase of the producer / the MMA issuer
-  uint32_t issued = 0;                                        // stages the producer has filled
   bool ok = true;
   int pass = 0;
   for (int t0 = 0; t0 < rows; t0 += p.passTokens, ++pass) {
@@ -178,13 +169,12 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
         const int wRow = expert * p.N + tile * kRows;
         for (int kb = kBegin; kb < kEnd && ok; ++kb) {
           ok = tc::mbarWait(emptyBar(st), ph ^ 1, abortWord, p.timeoutNs);
-          if (!ok) { giveUp(1, kb); break; }
+          if (!ok) { recordTimeout(p.status, 1, tile, kb); break; }
           const uint32_t sW = base + st * stageBytes, sX = sW + kWBytes;
           tc::mbarExpectTx(fullBar(st), uint32_t(kWBytes + cols * kK * 2));
           tc::tmaLoad2d(sW, &maps.w, kb * kK, wRow, fullBar(st));
           for (int i = 0; i < loads; ++i)
             tc::tmaLoad2d(sX + uint32_t(i * p.tokenBox * kK * 2), &maps.x, kb * kK, firstRow + t0 + i * p.tokenBox, fullBar(st));
-          ++issued;
           if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; }
         }
       }
@@ -194,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
         const uint64_t descW = tc::smemDescSw128(base), descX = tc::smemDescSw128(base + kWBytes);
         for (int kb = kBegin; kb < kEnd && ok; ++kb) {
           ok = tc::mbarWait(fullBar(st), ph, abortWord, p.timeoutNs);
-          if (!ok) { giveUp(3, kb); break; }
+          if (!ok) { recordTimeout(p.status, 3, tile, kb); break; }
           tc::fenceAfterThreadSync();
           const uint64_t step = uint64_t(st * (stageBytes >> 4));
 #pragma unroll
@@ -210,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
       const int quarter = warp & 3;                           // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
       ok = tc::mbarWait(accFull, uint32_t(pass & 1), abortWord, p.timeoutNs);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok && lane == 0) giveUp(5, pass);
+      if (!ok && lane == 0) recordTimeout(p.status, 5, tile, pass);
       if (ok) {
         // every load of the pass has landed and every MMA has read its stage, so the stages' memory is free
         tc::fenceAfterThreadSync();
@@ -225,6 +215,12 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
         }
         tc::fenceBeforeThreadSync();
       }
+    }
+    // A wait that gave up is everybody's business: the partial tile of this CTA is not what its peers would add. They learn of it
+    // through their own abort words, written before the cluster barrier after which they are read.
+    if (!ok) {
+      const uint32_t word = tc::smemAddr(words + 1);
+      for (uint32_t q = 0; q < split; ++q) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(tc::mapToCta(word, q)), "r"(1) : "memory");
     }
     __syncwarp();
     tc::clusterSync();                                        // every partial tile of the cluster is in shared memory
@@ -271,10 +267,9 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
     tc::clusterSync();
   }
   if (*abortWord) {
-    // copies and MMAs under way end before shared memory and TMEM go away: the last copy into each stage, the last MMA issued
-    if (warp == 0 && lane == 0)
-      for (uint32_t j = issued > uint32_t(p.stages) ? issued - uint32_t(p.stages) : 0u; j < issued; ++j)
-        tc::mbarDrain(fullBar(j % uint32_t(p.stages)), (j / uint32_t(p.stages)) & 1u);
+    // copies and MMAs under way end before shared memory and TMEM go away: the last copy into each stage (of this lap of the ring
+    // or the one before; a stage never used counts as landed), the last MMA issued
+    if (warp == 0 && lane == 0) for (uint32_t s = 0; s < uint32_t(p.stages); ++s) tc::mbarDrain(fullBar(s), s < st ? ph : ph ^ 1);
     if (warp == 1 && lane == 0) { tc::mmaCommit(mmasDone); tc::mbarDrain(mmasDone, 0); }
     __syncwarp();
   }

@@ -842,14 +842,16 @@ struct GroupedArgs {
 bool fewWeightRows(int M, int N, int K, int epilogue) { return epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens && K >= 2048; }
 bool useSkinny(int M, int N, int K, int epilogue) {
   if (fewWeightRows(M, N, K, epilogue)) return true;
-  // always up to 64 rows: 64 x 57344 x 8192 153 / 165, 48 x 4096 x 4096 14 / 22
-  if (M <= 64) return true;
+  // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 57344 x 8192 153 / 165, 48 x 4096 x 4096 14 / 22,
+  // 64 x 264 x 528 5.8 / 6.7; but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4
+  if (M <= 64) return M <= 32 || K >= 512;
   // up to 128 while W has too few rows to give every SM a tile of its own and k is worth splitting: 128 x 8192 x 7168 31.5 /
-  // 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 14336 x 4096 28.2 / 27.4, 128 x 264 x 72 7.4 / 5.3
-  if (M <= 128) return N <= 8192 && K >= 1024;
+  // 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 8192 x 1024 11.2 / 9.8, 128 x 14336 x 4096 28.2 /
+  // 27.4, 128 x 264 x 72 7.4 / 5.3
+  if (M <= 128) return N <= 8192 && K >= (N < 4096 ? 1024 : 1536);
   // up to 256 where the tiles are few and k is long: 256 x 4096 x 4096 21.2 / 25.1, 256 x 8192 x 7168 40.4 / 42.4, 140 x 8192 x
-  // 4096 21.1 / 22.6; but 200 x 14336 x 8192 74.9 / 67.5, 200 x 264 x 72 9.2 / 5.3
-  return M <= skinny::kMaxTokens && N >= 4096 && N <= 8192 && K >= 4096;
+  // 4096 21.1 / 22.6; but 200 x 8192 x 4096 25.5 / 24.1, 200 x 14336 x 8192 74.9 / 67.5, 200 x 264 x 72 9.2 / 5.3
+  return M <= skinny::kMaxTokens && N >= 4096 && N <= 8192 && K >= (M <= 160 || N == 4096 ? 4096 : 6144);
 }
 
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
@@ -873,13 +875,17 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   const int budget = (perSm == 2 ? 113 : 227) * 1024 - 1024 - skinny::kBarrierBytes;
   p.stages = std::min(budget / stageBytes, skinny::kMaxStages);
   for (p.tmemCols = 32; p.tmemCols < p.passTokens; p.tmemCols *= 2) {}
-  // Split k until the CTAs fill three quarters of the places on the GPU and a part keeps at least four k-blocks. Measured,
+  // Split k while the CTAs have a place on the GPU at the same time and a part keeps at least four k-blocks; eight where many
+  // tiles are split four ways (64 x 7744 x 1160, 61 tiles: 12.0 us whole, 10.6 in two parts, 13.0 in four). Measured,
   // 1 x 8192 x 3584: one CTA per tile 20.1 us, two 14.4, four 14.2, eight 18.2; 64 x 8192 x 28672: 142.6 / 87.4 / 79.1 /
-  // 90.5 us. At most 15 clusters of eight fit on the GPU at once, so eight are used for no more tiles than that.
+  // 90.5 us. More CTAs than places cost a second wave: 64 x 11232 x 1952 SwiGLU (88 tiles, 296 places) 16.6 / 14.7 / 26.7,
+  // 192 x 5824 x 1280 (46 tiles, 148 places) 17.0 / 13.1 / 23.9. At most 15 clusters of eight fit on the GPU at once, so eight
+  // are used for no more tiles than that.
   const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
   const long slots = long(smCount()) * perSm;
+  const long allTiles = long(tiles) * g.experts;
   int split = 1;
-  while (split < (long(tiles) * g.experts <= 15 ? skinny::kMaxSplit : 4) && long(tiles) * g.experts * split * 4 < slots * 3 && kBlocks >= 8 * split) split *= 2;
+  while (split < (allTiles <= 15 ? skinny::kMaxSplit : 4) && allTiles * split * 2 <= slots && kBlocks >= (split > 1 && allTiles > 24 ? 16 : 8) * split) split *= 2;
   skinny::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
   const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;

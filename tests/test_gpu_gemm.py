@@ -252,3 +252,17 @@ def test_grouped_gemm_split_over_clusters_and_over_many_groups(likely, n, k, cou
         assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
     else:
         assert torch.equal(out.float(), ref)
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 264, 504), (33, 264, 512), (64, 96, 72), (64, 11168, 1072), (80, 12056, 1320), (192, 5824, 4104), (65, 4096, 1536)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_few_rows_around_the_limits_of_the_split(m, n, k, swiglu):
+    # where the few-rows kernel begins to be used and where one more split would not have room on the GPU
+    from purlin_b200.ops.gemm import gemm, gemm_swiglu
+    n = (n + 31) // 32 * 32
+    a, w = _small_integers(m, n, k, 19)
+    if swiglu:
+        ref = _swiglu_ref(a, w)
+        assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+    else:
+        assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())

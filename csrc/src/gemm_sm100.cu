@@ -982,10 +982,13 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
 
 // Rows that are no multiple of 512 go through the ragged kernel once its 512 x 256 tiles give five eighths of the CTA pairs
 // work (one B200, us, it / the tiles of this file: 1000 x 14336 x 8192 177 / 222, 1000 x 8192 x 7168 83 / 104, 5000 x 4096 x
-// 4096 126 / 158, 1500 x 4096 x 4096 41 / 62; with fewer tiles 700 x 4096 x 4096 51 / 31, 300 x 8192 x 7168 61 / 56).
-bool useRagged(int M, int N) {
+// 4096 126 / 158, 1500 x 4096 x 4096 41 / 62; with fewer tiles 700 x 4096 x 4096 51 / 31, 300 x 8192 x 7168 61 / 56) and k is
+// long enough to hide its epilogue, which stands between the tiles and stores short row pieces (3189 x 1672 x 840 17.4 / 24.4,
+// 1121 x 18144 x 968 42 / 53, 2277 x 11680 x 1016 SwiGLU 56 / 79; but 4144 x 3296 x 512 22.8 / 15.3, 3708 x 20672 x 336 SwiGLU
+// 88 / 58, 3357 x 20472 x 80 61 / 37).
+bool useRagged(int M, int N, int K) {
   const long tiles = long((M + ragged::kMaxCols - 1) / ragged::kMaxCols) * ((N + ragged::kTileRows - 1) / ragged::kTileRows);
-  return M % (4 * kBM) != 0 && tiles * 16 >= long(smCount()) * 5;
+  return M % (4 * kBM) != 0 && K >= 768 && tiles * 16 >= long(smCount()) * 5;
 }
 
 }  // namespace
@@ -1029,7 +1032,7 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
   if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
-  if (bn == 0 && !switches().singleCta && !switches().oneAcc && useRagged(M, N)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+  if (bn == 0 && !switches().singleCta && !switches().oneAcc && useRagged(M, N, K)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
       !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;

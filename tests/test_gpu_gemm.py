@@ -266,3 +266,17 @@ def test_few_rows_around_the_limits_of_the_split(m, n, k, swiglu):
         assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
     else:
         assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("m,n,k", [(257, 14336, 768), (513, 8192, 840), (777, 8200, 776), (1000, 14336, 832), (2049, 4104, 768), (2368, 8192, 1032), (1000, 14336, 760)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_ragged_rows_with_a_k_that_hides_the_epilogue(m, n, k, swiglu):
+    # the sizes of the ragged kernel's remainders and waves at the shortest k it is used for, and one below
+    from purlin_b200.ops.gemm import gemm, gemm_swiglu
+    n = (n + 31) // 32 * 32 if swiglu else n
+    a, w = _small_integers(m, n, k, 21)
+    if swiglu:
+        ref = _swiglu_ref(a, w)
+        assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+    else:
+        assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())

@@ -61,7 +61,10 @@ class ExpertParallelMoE:
         """The weights of this rank's experts as one contiguous [experts, N, K], as the grouped GEMM reads them, or None: a list
         with a tensor per expert, or a stack of which only the slices are contiguous."""
         n = self.ep.experts_per_rank
-        return w[:n] if isinstance(w, torch.Tensor) and w.dim() == 3 and w.shape[0] >= n and w[:n].is_contiguous() else None
+        if not isinstance(w, torch.Tensor) or w.dim() != 3 or len(w) < n:
+            return None
+        w = w if len(w) == n else w[:n]
+        return w if w.is_contiguous() else None
 
     def _expert_by_expert(self, recv, counts, outb):
         """The experts when their weights are not one block: two GEMMs each, for which the host has to read the row counts."""

@@ -843,8 +843,8 @@ bool fewWeightRows(int M, int N, int K, int epilogue) { return epilogue == kEpiS
 bool useSkinny(int M, int N, int K, int epilogue) {
   if (fewWeightRows(M, N, K, epilogue)) return true;
   // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 57344 x 8192 153 / 165, 48 x 4096 x 4096 14 / 22,
-  // 64 x 264 x 528 5.8 / 6.7; but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4
-  if (M <= 64) return M <= 32 || K >= 512;
+  // 64 x 264 x 528 5.8 / 6.7; but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4, 64 x 14336 x 512 SwiGLU 9.8 / 8.6
+  if (M <= 64) return M <= 32 || K >= (N <= 8192 ? 512 : 1024);
   // up to 128 while W has too few rows to give every SM a tile of its own and k is worth splitting: 128 x 8192 x 7168 31.5 /
   // 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 8192 x 1024 11.2 / 9.8, 128 x 14336 x 4096 28.2 /
   // 27.4, 128 x 264 x 72 7.4 / 5.3

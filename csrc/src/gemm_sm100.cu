@@ -753,6 +753,14 @@ cudaLaunchAttribute overlapAttribute() {
   return a;
 }
 
+// Whether a launch is better placed on an empty GPU. Between half as many CTAs as SMs and six sevenths of them, a kernel that is
+// set up early takes the SMs its predecessor leaves free and then some of those it gives back, so neighbouring SMs that share
+// their path to L2 are both busy, where a launch on its own would have spread out. Where the main loop is short, the microsecond
+// that the overlap saves is more than that costs; from 28 k-blocks on it is not. Apart / overlapped, us: 6148 x 448 x 7000 SwiGLU
+// (98 CTAs) 64.5 / 72.6, 108 x 12672 x 2584 (99) 21.4 / 24.9, 7822 x 384 x 5064 (124) 44.6 / 49.6. Of 1074 shapes on these tiles
+// the overlap slows 32 by more than 5 %; with this rule two, and two that gained more than 3 % lose it.
+bool betterApart(long ctas, int K) { return ctas * 2 > smCount() && ctas * 7 < smCount() * 6 && K >= 28 * kBK; }
+
 template <int EPI, int COMM, int CTAS, int ACCS>
 int launchImpl(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t stream) {
   auto kernel = gemmKernel<EPI, COMM, CTAS, ACCS>;
@@ -791,7 +799,7 @@ int launchImpl(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t 
   attr[1] = overlapAttribute();
   attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(pairs * CTAS); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smemFor(p, sh); cfg.stream = stream;
-  cfg.attrs = attr; cfg.numAttrs = COMM == kCommNone ? 2 : 1;
+  cfg.attrs = attr; cfg.numAttrs = COMM == kCommNone && !betterApart(long(pairs) * CTAS, p.K) ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, q);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
@@ -974,7 +982,9 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   ragged::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), ragged::kBM) ||
       !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.xBox))) return 1;
-  cfg.gridDim = dim3(unsigned(std::min(pairs, items) * 2)); cfg.stream = stream; cfg.numAttrs = 2;
+  cfg.gridDim = dim3(unsigned(std::min(pairs, items) * 2)); cfg.stream = stream;
+  // (fewer tiles than pairs: the pairs without one leave at once; 2066 x 3144 x 4264, 63 tiles: 49.7 us apart, 58.0 overlapped)
+  cfg.numAttrs = betterApart(items, K) ? 1 : 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;

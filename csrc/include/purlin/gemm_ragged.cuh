@@ -9,11 +9,17 @@
 //     pairs is issued as half tiles (256 rows of W);
 //   * one persistent CTA pair per two SMs walks the tiles; with `counts` (rows per expert, on the device) the walk goes
 //     expert by expert, so the host never waits for the counts;
-//   * the epilogue turns the accumulator around: TMEM lanes are rows of W, so neighbouring lanes pair up (one shuffle per
-//     two values) and write rows of X into a small shared-memory tile, from which 16-byte row pieces go to C.
+//   * with both accumulators of a tile in use (all of TMEM) the next tile's MMAs wait for the epilogue, so it gives an accumulator
+//     back as soon as its values are in registers, activated and packed to bf16, and stores them under the next main loop: an SM
+//     stores about 32 bytes a cycle, 4096 cycles for its 128 KiB of a tile. The fragment form of the TMEM load and a transposing
+//     stmatrix turn rows of W into columns of C (gate and up of one value come to the same thread), from a small shared-memory
+//     tile 16-byte row pieces go to C. The exchange with shuffles and the stores before the release took 8000 to 9600 cycles of
+//     every tile, and the release then waited about 2000 more for the stores; now 800 (plain) and 2500 (SwiGLU, bound by its
+//     exponentials and divisions) per accumulator. The main loop runs at the tensor pipe's rate, 1024 cycles per k-block;
+//   * what is left of the epilogue is hidden by moving the accumulators against each other (kLead).
+// One B200, before / now in turn, us (all of it under the power cap): 32 experts of 1024 rows, 4096 x 7168 SwiGLU 1623 / 1494,
+// 7168 x 2048 944 / 752; 8190 x 7168 x 2048 212 / 172, 1000 x 14336 x 8192 SwiGLU 209 / 203.
 #pragma once
-#include <type_traits>
-
 #include "gemm_skinny.cuh"
 
 namespace purlin {
@@ -23,15 +29,20 @@ constexpr int kBM = 128, kBK = 64, kMaxCols = 256;
 constexpr int kABytes = kBM * kBK * 2;
 constexpr int kTileRows = 512;                  // rows of W per tile: 2 accumulators x 2 CTAs x 128
 constexpr int kAccStride = 256, kTmemCols = 512;
-// Four epilogue warps per accumulator: with both accumulators of a tile in use the epilogue is exposed, and eight warps halve it
-// (four / eight warps, one B200: 3000 x 7168 x 2048 77.5 / 73.3 us, 1500 x 4096 x 4096 SwiGLU 51.1 / 46.9, 32 experts of 1024
-// rows 1748 + 1151 / 1631 + 1130).
+// Two epilogue warps per quarter of the TMEM lanes (a quarter is all that a warp may read): the drain is exposed, and with one
+// each it took twice as long.
 constexpr int kEpiWarps = 8, kThreads = 32 * (2 + kEpiWarps);
 constexpr int kStagingBytes = kEpiWarps * 2048;       // a 32 x 32 bf16 tile per epilogue warp
 constexpr int kBarrierBytes = 256;
 constexpr int kMaxExperts = 512;
 constexpr int kTableBytes = 2 * (kMaxExperts + 1) * 4;
 constexpr int kMaxStages = 6;
+// k-blocks at either end of a tile that the first accumulator gets before the second one: it is finished, and drained, while the
+// second one's last k-blocks run, and the next tile starts with it while the second one is drained. The MMAs of a k-block go into
+// one accumulator then, and each waits for the one before (174 cycles instead of 128, measured): longer leads cost more than they
+// hide (0 / 1 / 2 / 3 k-blocks, us, 32 experts of 1024 rows: 4096 x 7168 SwiGLU 1541 / 1513 / 1494 / 1507, 7168 x 2048 800 / 771 /
+// 752 / 758). A lead holds that many stages.
+constexpr int kLead = 2;
 constexpr int kBand = 8;                        // column tiles that are in flight together (their X rows stay in L2)
 
 struct alignas(64) Maps { CUtensorMap w, x; };
@@ -78,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
-    for (int a = 0; a < 2; ++a) { tc::mbarInit(tmemFullBar(a), 1); tc::mbarInit(tmemEmptyBar(a), kEpiWarps); }   // 4 warps in each CTA
+    for (int a = 0; a < 2; ++a) { tc::mbarInit(tmemFullBar(a), 1); tc::mbarInit(tmemEmptyBar(a), 2 * kEpiWarps); }   // the warps of both CTAs
     *abortWord = 0;
     tc::mbarFenceInit();
     tc::tmaPrefetchDescriptor(&maps.w);
@@ -181,36 +192,69 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
         const uint32_t idesc = tc::instrDescBf16(uint32_t(m.cols), uint32_t(2 * kBM));
         const bool two = m.accs == 2;
         ok = tc::mbarWait(tmemEmptyBar(0), (use0 & 1) ^ 1, abortWord, p.timeoutNs);
-        if (ok && two) ok = tc::mbarWait(tmemEmptyBar(1), (use1 & 1) ^ 1, abortWord, p.timeoutNs);
         if (!ok) { skinny::recordTimeout(p.status, 2, it, 0); break; }
-        // One thread feeds the tensor cores of two SMs (an MMA takes about 128 cycles), so the loop over the stages holds
-        // nothing but waits, MMAs and commits: which accumulators there are is decided outside of it.
-        auto issue = [&](auto both) {
-          uint32_t accumulate = 0;
-          for (int kb = 0; kb < kBlocks; ++kb) {
-            ok = tc::mbarWait(fullBar(st), ph, abortWord, p.timeoutNs);
-            if (!ok) { skinny::recordTimeout(p.status, 3, it, kb); break; }
-            tc::fenceAfterThreadSync();
-            const uint64_t step = uint64_t(st * (kStageBytes >> 4));
-#pragma unroll
-            for (int k = 0; k < kBK / 16; ++k) {
-              tc::mmaPair(tmemBase, descW0 + step + 2 * k, descX0 + step + 2 * k, idesc, accumulate);
-              if constexpr (decltype(both)::value) tc::mmaPair(tmemBase + kAccStride, descW0 + step + (kABytes >> 4) + 2 * k, descX0 + step + 2 * k, idesc, accumulate);
-              accumulate = 1;
-            }
-            tc::mmaCommitPair(leaderBars + 8u * (uint32_t(p.stages) + st));
-            tc::mmaCommitPair(peerBars + 8u * (uint32_t(p.stages) + st));
-            if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; }
-          }
+        uint32_t accumulate = 0;
+        // One thread feeds the tensor cores of two SMs (an MMA takes about 128 cycles), so the loops over the stages hold
+        // nothing but waits, MMAs and commits: which accumulators there are is decided outside of them.
+        auto landed = [&](int kb) {                            // the k-block in the current stage
+          ok = tc::mbarWait(fullBar(st), ph, abortWord, p.timeoutNs);
+          if (!ok) { skinny::recordTimeout(p.status, 3, it, kb); return false; }
+          tc::fenceAfterThreadSync();
+          return true;
         };
-        if (two) issue(std::true_type{}); else issue(std::false_type{});
-        if (ok) {
-          for (int a = 0; a < m.accs; ++a) {
-            tc::mmaCommitPair(leaderBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
-            tc::mmaCommitPair(peerBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
+        auto release = [&]() {                                 // of the current stage, once the MMAs issued so far have read it
+          tc::mmaCommitPair(leaderBars + 8u * (uint32_t(p.stages) + st));
+          tc::mmaCommitPair(peerBars + 8u * (uint32_t(p.stages) + st));
+        };
+        auto advance = [&]() { if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; } };
+        auto complete = [&](int a) {                           // the epilogue may read accumulator a
+          tc::mmaCommitPair(leaderBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
+          tc::mmaCommitPair(peerBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
+        };
+        auto mma = [&](uint32_t stage, int a, int k, uint32_t acc) {
+          const uint64_t step = uint64_t(stage * (kStageBytes >> 4));
+          tc::mmaPair(tmemBase + uint32_t(a) * kAccStride, descW0 + step + uint32_t(a) * (kABytes >> 4) + 2 * k, descX0 + step + 2 * k, idesc, acc);
+        };
+        if (two) {
+          const int ends = min(kLead, kBlocks / 2);
+          auto oneThenOther = [&](int kb0, bool last) {
+            const uint32_t st0 = st, ph0 = ph;
+            for (int i = 0; i < ends && ok; ++i) {
+              if (!landed(kb0 + i)) return;
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); accumulate = 1; }
+              advance();
+            }
+            if (last) complete(0);
+            else ok = tc::mbarWait(tmemEmptyBar(1), (use1 & 1) ^ 1, abortWord, p.timeoutNs);
+            if (!ok) { skinny::recordTimeout(p.status, 2, it, 1); return; }
+            st = st0; ph = ph0;
+            for (int i = 0; i < ends; ++i) {
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k) mma(st, 1, k, uint32_t(last || i || k));
+              release();
+              advance();
+            }
+          };
+          oneThenOther(0, false);
+          for (int kb = ends; kb < kBlocks - ends && ok; ++kb) {
+            if (!landed(kb)) break;
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); mma(st, 1, k, accumulate); accumulate = 1; }
+            release();
+            advance();
           }
-          ++use0;
-          if (two) ++use1;
+          if (ok) oneThenOther(kBlocks - ends, true);
+          if (ok) { complete(1); ++use0; ++use1; }
+        } else {
+          for (int kb = 0; kb < kBlocks; ++kb) {
+            if (!landed(kb)) break;
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); accumulate = 1; }
+            release();
+            advance();
+          }
+          if (ok) { complete(0); ++use0; }
         }
       }
     }
@@ -218,84 +262,88 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     // ------------------------------- epilogue -------------------------------
     constexpr int kOut = SWIGLU ? 16 : 32;                     // output columns of this warp's 32 rows of W
     constexpr int kPitch = kOut * 2;                           // bytes of a token's row in the staging tile
+    constexpr int kChunks = kMaxCols / 64, kHeld = kOut / 2;   // per accumulator of a warp: 32-column chunks, packed registers of each
+    constexpr int kPieces = kOut / 8, kRowsPer = 32 / kPieces; // 16-byte pieces of such a row; rows per access of the warp
     const int quarter = warp & 3;                              // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
     const int outCols = SWIGLU ? p.N / 2 : p.N;
-    const int a = (warp - 2) / 4;                              // this warp's accumulator
+    const int group = (warp - 2) / 4;                          // two warps per quarter share the columns, 32 by 32
     const uint32_t buf = stagingAll + uint32_t(warp - 2) * 2048u;
-    uint32_t use = 0;
+    // where 16-byte piece `piece` of token row `row` lies in the staging tile: rotated so that neither the eight rows of a
+    // transposed store nor the reads meet in a bank
+    auto stagedAt = [&](int row, int piece) { return buf + uint32_t(row * kPitch + ((piece ^ ((row * kPitch >> 7) & (kPieces - 1))) << 4)); };
+    const int piece = lane % kPieces, rr = lane / kPieces;
+    uint32_t use = 0;                                          // bit a: parity of the uses of accumulator a so far
     bool ok = true;
     for (int it = pairIdx; it < numItems && ok; it += numPairs) {
       const Item m = itemOf(it);
-      if (a < m.accs) {
-        ok = tc::mbarWait(tmemFullBar(a), use & 1, abortWord, p.timeoutNs);
+      // into registers, activated and packed; the accumulator goes back to the MMA warp
+      uint32_t held[2][kChunks][kHeld];
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (a >= m.accs || !ok) continue;
+        ok = tc::mbarWait(tmemFullBar(a), (use >> a) & 1, abortWord, p.timeoutNs);
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok) { if (lane == 0) skinny::recordTimeout(p.status, 5, it, a); break; }
-        ++use;
+        if (!ok) { if (lane == 0) skinny::recordTimeout(p.status, 5, it, a); continue; }
+        use ^= 1u << a;
         tc::fenceAfterThreadSync();
-        const uint32_t taddr = tmemBase + (uint32_t(quarter * 32) << 16) + uint32_t(a) * kAccStride;
-        const int wRow = m.w0 + a * 2 * kBM + int(ctaRank) * kBM + quarter * 32;     // of lane 0
-        const int n0 = SWIGLU ? wRow / 2 : wRow;
-        __nv_bfloat16* out = p.C + size_t(m.row0) * p.ldc + n0;
-
-        // 32 columns (tokens) of this warp's 32 rows of W -> rows of C
-        auto drain = [&](const uint32_t (&r)[32], int c) {
-          if constexpr (SWIGLU) {
-            // lanes 0-15 hold gate, 16-31 up, of the same 16 output columns: the lower half finishes tokens t and t + 1, the
-            // upper half t + 2 and t + 3; then neighbouring lanes pair up so that each writes two columns of one token
-            const bool low = lane < 16, even = (lane & 1) == 0;
+        const uint32_t taddr = tmemBase + (uint32_t(quarter * 32) << 16) + uint32_t(a) * kAccStride + uint32_t(group * 32);
+        // 32 columns (tokens) of this warp's 32 rows of W at a time, as fragments of rows 0-15 and of rows 16-31
 #pragma unroll
-            for (int t = 0; t < 32; t += 4) {
-              float v[2];
+        for (int j = 0; j < kChunks; ++j) {
+          if (group * 32 + j * 64 >= m.count) continue;
+          uint32_t lo[16], hi[16];
+          tc::tmemLoadFragments(taddr + uint32_t(j * 64), lo);
+          tc::tmemLoadFragments(taddr + (16u << 16) + uint32_t(j * 64), hi);
+          tc::tmemLoadWaitFor(lo);
+          tc::tmemLoadWaitFor(hi);
+          auto f = [](uint32_t v) { return __uint_as_float(v); };
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const float got = __uint_as_float(__shfl_xor_sync(0xffffffffu, low ? r[t + 2 + h] : r[t + h], 16));
-                const float own = __uint_as_float(low ? r[t + h] : r[t + 2 + h]);
-                v[h] = low ? skinny::siluOf(own) * got : skinny::siluOf(got) * own;
-              }
-              const float other = __shfl_xor_sync(0xffffffffu, even ? v[1] : v[0], 1);
-              const uint32_t w = even ? skinny::pack2(v[0], other) : skinny::pack2(other, v[1]);
-              const int token = t + (low ? 0 : 2) + (even ? 0 : 1);
-              asm volatile("st.shared.u32 [%0], %1;" ::"r"(buf + uint32_t(token * kPitch + ((lane & 15) >> 1) * 4)), "r"(w) : "memory");
+          for (int i = 0; i < 8; ++i) {
+            if constexpr (SWIGLU)                              // rows 0-15 are gate, 16-31 up, of the same 16 output columns
+              held[a][j][i] = skinny::pack2(skinny::siluOf(f(lo[2 * i])) * f(hi[2 * i]), skinny::siluOf(f(lo[2 * i + 1])) * f(hi[2 * i + 1]));
+            else {
+              held[a][j][i] = skinny::pack2(f(lo[2 * i]), f(lo[2 * i + 1]));
+              held[a][j][8 + i] = skinny::pack2(f(hi[2 * i]), f(hi[2 * i + 1]));
             }
-          } else {
-            const bool even = (lane & 1) == 0;
-#pragma unroll
-            for (int t = 0; t < 32; t += 2) {
-              const float v0 = __uint_as_float(r[t]), v1 = __uint_as_float(r[t + 1]);
-              const float other = __shfl_xor_sync(0xffffffffu, even ? v1 : v0, 1);
-              const uint32_t w = even ? skinny::pack2(v0, other) : skinny::pack2(other, v1);
-              asm volatile("st.shared.u32 [%0], %1;" ::"r"(buf + uint32_t((t + (even ? 0 : 1)) * kPitch + (lane >> 1) * 4)), "r"(w) : "memory");
-            }
-          }
-          __syncwarp();
-          constexpr int kPieces = kOut / 8, kRowsPer = 32 / kPieces;
-          const int piece = lane % kPieces, rr = lane / kPieces;
-          const bool colOk = n0 + piece * 8 + 8 <= outCols;
-#pragma unroll
-          for (int i = 0; i < kPieces; ++i) {
-            const int row = i * kRowsPer + rr;
-            Vec16 v;
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]) : "r"(buf + uint32_t(row * kPitch + piece * 16)) : "memory");
-            if (colOk && c + row < m.count) st16(out + size_t(c + row) * p.ldc + piece * 8, v);
-          }
-          __syncwarp();                                        // the tile has been read before the next chunk fills it
-        };
-        uint32_t ra[32], rb[32];
-        tc::tmemLoad32(taddr, ra);
-#pragma unroll 1
-        for (int c = 0; c < m.count; c += 64) {
-          tc::tmemLoadWaitFor(ra);
-          if (c + 32 < m.count) tc::tmemLoad32(taddr + uint32_t(c + 32), rb);
-          drain(ra, c);
-          if (c + 32 < m.count) {
-            tc::tmemLoadWaitFor(rb);
-            if (c + 64 < m.count) tc::tmemLoad32(taddr + uint32_t(c + 64), ra);
-            drain(rb, c + 32);
           }
         }
         tc::fenceBeforeThreadSync();
         __syncwarp();
         if (lane == 0) tc::mbarArriveCluster(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a)));
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (a >= m.accs) continue;
+        const int wRow = m.w0 + a * 2 * kBM + int(ctaRank) * kBM + quarter * 32;     // of lane 0
+        const int n0 = (SWIGLU ? wRow / 2 : wRow) + piece * 8;
+        const bool colOk = n0 + 8 <= outCols;
+        __nv_bfloat16* out = p.C + size_t(m.row0) * p.ldc + n0;
+#pragma unroll
+        for (int j = 0; j < kChunks; ++j) {
+          const int c = group * 32 + j * 64;
+          if (c >= m.count) continue;
+          const uint32_t (&h)[kHeld] = held[a][j];
+          // turned around on the way into the staging tile: rows of W become columns of C
+          if constexpr (SWIGLU) {
+#pragma unroll
+            for (int i = 0; i < 4; i += 2)
+              tc::stMatrixTransposed4(stagedAt(8 * (i + (lane >> 4)) + (lane & 7), (lane >> 3) & 1), h[2 * i], h[2 * i + 1], h[2 * i + 2], h[2 * i + 3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              tc::stMatrixTransposed4(stagedAt(8 * i + (lane & 7), lane >> 3), h[2 * i], h[2 * i + 1], h[8 + 2 * i], h[8 + 2 * i + 1]);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < kPieces; ++i) {
+            Vec16 v;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]) : "r"(stagedAt(i * kRowsPer + rr, piece)) : "memory");
+            const int row = c + i * kRowsPer + rr;
+            if (colOk && row < m.count) st16(out + size_t(row) * p.ldc, v);
+          }
+          __syncwarp();                                        // the tile has been read before the next chunk fills it
+        }
       }
     }
   }

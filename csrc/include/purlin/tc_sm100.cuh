@@ -110,7 +110,7 @@ PURLIN_D void clusterSync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 PURLIN_D void mbarArriveCluster(uint32_t clusterBarAddress) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterBarAddress) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterBarAddress) : "memory");
 }
 // tile load of one CTA of a pair; the transaction bytes are credited to a barrier that may live in the other CTA
 PURLIN_D void tmaLoad2dPair(uint32_t smemDst, const CUtensorMap* map, int x, int y, uint32_t clusterBarAddress) {
@@ -186,6 +186,23 @@ PURLIN_D void tmemLoad32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr) : "memory");
 }
+// 16 lanes x 32 columns of fp32 as fragments: thread t receives, for every group i of eight columns, in r[4 i + 0..1] columns
+// 8 i + 2 (t % 4) + {0, 1} of lane t / 4 and in r[4 i + 2..3] the same columns of lane t / 4 + 8. Packed to 16 bits this is the
+// operand of stMatrixTransposed4(). The address selects lanes 0-15 or 16-31
+// of the warp's 32.
+PURLIN_D void tmemLoadFragments(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values (fragments: thread t holds row t / 4, columns 2 (t % 4) + {0, 1}) are stored transposed:
+// thread t gives the 16-byte address of column t % 8 of matrix t / 8.
+PURLIN_D void stMatrixTransposed4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 PURLIN_D void tmemLoadWait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // The same wait, tied to the registers of an earlier tmemLoad32: when other work sits between a load and its wait
 // (software pipelining), the compiler must not move a use of those registers above the wait.
@@ -196,6 +213,13 @@ PURLIN_D void tmemLoadWaitFor(uint32_t (&r)[32]) {
         "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
         "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
         "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+      :: "memory");
+}
+PURLIN_D void tmemLoadWaitFor(uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.wait::ld.sync.aligned;"
+      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+        "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
       :: "memory");
 }
 

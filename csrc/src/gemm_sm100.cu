@@ -945,6 +945,7 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   constexpr int stageBytes = 2 * ragged::kABytes + ragged::kMaxCols / 2 * ragged::kBK * 2;
   constexpr int fixedBytes = 1024 + ragged::kStagingBytes + ragged::kBarrierBytes + ragged::kTableBytes;
   constexpr int stages = (kSmemLimit - fixedBytes) / stageBytes < ragged::kMaxStages ? (kSmemLimit - fixedBytes) / stageBytes : ragged::kMaxStages;
+  static_assert(stages >= ragged::kLead, "a lead holds its stages until the second accumulator has read them");
   cfg.dynamicSmemBytes = size_t(stages) * stageBytes + fixedBytes;
   {
     std::lock_guard<std::mutex> lock(mu);

@@ -2,11 +2,13 @@
 //
 // What bounds it is the tensor pipe, and the loss it removes is padding: the rows of X (a prompt chunk, the rows of an
 // expert) are no multiple of a 256- or 512-row tile. So W fills the rows of the MMA (its row count is a multiple of the
-// tile in practice) and the rows of X are the columns, whose number may be any multiple of 32: T rows are cut into
-// column tiles of `tileCols` and one narrower tile for the remainder.
+// tile in practice) and the rows of X are the columns, whose number may be any multiple of 32: T rows are shared out over as many
+// column tiles as leave the pairs least idle (rows of 1030 in five tiles of 192 to 224 and not four of 256 and one of 32: the loads
+// of W make a narrow tile dear).
 //   * a tile is 512 rows of W (two accumulators of a CTA pair, 256 rows each) x up to 256 rows of X; the two accumulators
-//     share the X operand, which the tensor pipe rewards (see gemm_sm100.cu). A last wave that fills at most half of the
-//     pairs is issued as half tiles (256 rows of W);
+//     share the X operand, and their MMAs alternate: an MMA waits for the one before into the same columns (174 cycles instead of
+//     128, measured). Where there are few tiles a tile is 256 rows of W. A last wave that fills at most half of the pairs is issued
+//     as half tiles;
 //   * one persistent CTA pair per two SMs walks the tiles; with `counts` (rows per expert, on the device) the walk goes
 //     expert by expert, so the host never waits for the counts;
 //   * with both accumulators of a tile in use (all of TMEM) the next tile's MMAs wait for the epilogue, so it gives an accumulator
@@ -27,7 +29,7 @@ namespace ragged {
 
 constexpr int kBM = 128, kBK = 64, kMaxCols = 256;
 constexpr int kABytes = kBM * kBK * 2;
-constexpr int kTileRows = 512;                  // rows of W per tile: 2 accumulators x 2 CTAs x 128
+constexpr int kAccRows = 256;                   // rows of W per accumulator of a pair; a tile has one or two of them
 constexpr int kAccStride = 256, kTmemCols = 512;
 // Two epilogue warps per quarter of the TMEM lanes (a quarter is all that a warp may read): the drain is exposed, and with one
 // each it took twice as long.
@@ -36,7 +38,8 @@ constexpr int kStagingBytes = kEpiWarps * 2048;       // a 32 x 32 bf16 tile per
 constexpr int kBarrierBytes = 256;
 constexpr int kMaxExperts = 512;
 constexpr int kTableBytes = 2 * (kMaxExperts + 1) * 4;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8, kRingBytes = 192 * 1024;
+constexpr int kXBox = 32;                       // rows of one X load
 // k-blocks at either end of a tile that the first accumulator gets before the second one: it is finished, and drained, while the
 // second one's last k-blocks run, and the next tile starts with it while the second one is drained. The MMAs of a k-block go into
 // one accumulator then, and each waits for the one before (174 cycles instead of 128, measured): longer leads cost more than they
@@ -49,9 +52,11 @@ struct alignas(64) Maps { CUtensorMap w, x; };
 
 struct Params {
   int N, K, tokens;        // N: rows of W per expert; tokens: rows of X (with counts: an upper bound of their sum)
-  int tileCols;            // columns of a tile: a multiple of 64, at most 256
-  int xBox;                // rows of one X load
-  int stages;
+  int tileAccs;            // accumulators of a tile: 2 (512 rows of W) or 1 (256)
+  int colTiles, maxCols;   // column tiles, and columns of the widest one; with counts an expert has a tile per maxCols rows
+  int parts;               // SPLIT: pairs of a cluster
+  int stages;              // of stageBytes each, in kRingBytes
+  uint32_t stageBytes;
   int experts;
   const int32_t* counts;   // rows per expert, or null: one group of `tokens` rows
   __nv_bfloat16* C;
@@ -60,21 +65,28 @@ struct Params {
   uint64_t timeoutNs;
 };
 
-template <bool SWIGLU>
+PURLIN_D void stCluster16(uint32_t clusterAddress, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(clusterAddress), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// SPLIT: a cluster holds several pairs, which share one tile: each takes a part of its k range, and the partial tiles meet in
+// distributed shared memory, in the place of the stages, where each pair finishes every so-many-th chunk of 32 columns, added in the
+// order of k. (Through global memory, the last pair to arrive adding them up, the same took 19000 to 45000 cycles instead of about
+// 5000.) One tile per cluster, nobody waits for another cluster.
+template <bool SWIGLU, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) {
   extern __shared__ unsigned char smemRaw[];
   const uint32_t rawAddr = tc::smemAddr(smemRaw);
   const uint32_t base = (rawAddr + 1023u) & ~1023u;
   unsigned char* smem = smemRaw + (base - rawAddr);
-  constexpr int kXBytes = kMaxCols / 2 * kBK * 2;              // this CTA's half of the columns
-  constexpr uint32_t kStageBytes = 2 * kABytes + kXBytes;      // [W block 0][W block 1][X]
-  const uint32_t stagingAll = base + uint32_t(p.stages) * kStageBytes;
+  const uint32_t xAt = uint32_t(p.tileAccs * kABytes);         // a stage: [W block 0][W block 1, with two accumulators][X: this CTA's half of the columns]
+  const uint32_t stagingAll = base + kRingBytes;
   const uint32_t barBase = stagingAll + kStagingBytes;
   auto fullBar = [&](uint32_t s) { return barBase + 8u * s; };
   auto emptyBar = [&](uint32_t s) { return barBase + 8u * (uint32_t(p.stages) + s); };
   auto tmemFullBar = [&](int a) { return barBase + 8u * (2u * uint32_t(p.stages) + uint32_t(a)); };
   auto tmemEmptyBar = [&](int a) { return barBase + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a)); };
-  unsigned char* tail = smem + size_t(p.stages) * kStageBytes + kStagingBytes;
+  unsigned char* tail = smem + kRingBytes + kStagingBytes;
   uint32_t* words = reinterpret_cast<uint32_t*>(tail + 8 * (2 * p.stages + 4));
   volatile uint32_t* tmemBaseWord = words;
   volatile int* abortWord = reinterpret_cast<volatile int*>(words + 1);
@@ -82,10 +94,11 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   int* rowStart = itemStart + (kMaxExperts + 1);                      // [experts + 1] first row of X of an expert
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t ctaRank = tc::clusterCtaRank();
-  const int pairIdx = int(blockIdx.x) / 2, numPairs = int(gridDim.x) / 2;
-  const int wTiles = (p.N + kTileRows - 1) / kTileRows;
-  auto tilesOf = [&](int rows) { return (rows + p.tileCols - 1) / p.tileCols; };
+  const uint32_t clusterRank = tc::clusterCtaRank(), ctaRank = clusterRank & 1u;
+  const int parts = SPLIT ? p.parts : 1, part = SPLIT ? int(clusterRank / 2) : 0;     // pairs that share a tile
+  const int pairIdx = int(blockIdx.x) / (2 * parts), numPairs = int(gridDim.x) / (2 * parts);
+  const int tileRows = kAccRows * p.tileAccs, wTiles = (p.N + tileRows - 1) / tileRows;
+  auto tilesOf = [&](int rows) { return p.counts ? (rows + p.maxCols - 1) / p.maxCols : p.colTiles; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
@@ -126,9 +139,10 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   tc::fenceAfterThreadSync();
   tc::gridLaunchDependents();
   const uint32_t tmemBase = *tmemBaseWord;
-  const uint32_t leaderBars = tc::mapToCta(barBase, 0), peerBars = tc::mapToCta(barBase, 1);
+  const uint32_t leaderBars = tc::mapToCta(barBase, clusterRank & ~1u), pairMask = 3u << (clusterRank & ~1u);
   const int numTiles = itemStart[p.experts], rest = numTiles % numPairs;
-  const int fullItems = 2 * rest <= numPairs ? numTiles - rest : numTiles;        // whole tiles; the others count as two items each
+  // whole tiles; the others count as two items each
+  const int fullItems = !SPLIT && p.tileAccs == 2 && 2 * rest <= numPairs ? numTiles - rest : numTiles;
   const int numItems = fullItems + 2 * (numTiles - fullItems);
   const int kBlocks = (p.K + kBK - 1) / kBK;
 
@@ -141,122 +155,173 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     Item m;
     m.expert = expert;
     const int rows = rowStart[expert + 1] - rowStart[expert], tiles = tilesOf(rows);
-    const int i = tile - itemStart[expert], perBand = kBand * wTiles, band = i / perBand, within = i - band * perBand;
-    const int inBand = min(tiles - band * kBand, kBand);
-    const int col = band * kBand + within % inBand;
-    m.w0 = within / inBand * kTileRows;
-    m.row0 = rowStart[expert] + col * p.tileCols;
-    m.count = min(p.tileCols, rows - col * p.tileCols);
-    m.cols = (m.count + 31) / 32 * 32;                         // steps of 32, as the MMA of a pair wants them
-    m.accs = m.w0 + kTileRows / 2 < p.N ? 2 : 1;
-    if (it >= fullItems) {                                     // half a tile: 256 rows of W (none, when the tile has no second half)
+    const int i = tile - itemStart[expert], units = (rows + 31) / 32;
+    int first = 0, width = units;                              // of the column tile, in units of 32 (steps of an MMA of a pair)
+    m.w0 = i * tileRows;
+    if (tiles > 1) {                                           // (a few divisions that a stream of small tiles would notice: decode 6 %)
+      const int perBand = kBand * wTiles, band = i / perBand, within = i - band * perBand;
+      const int inBand = min(tiles - band * kBand, kBand), wTile = within / inBand;
+      const int col = band * kBand + within - wTile * inBand;
+      m.w0 = wTile * tileRows;
+      // the rows of X are shared out evenly over the column tiles
+      const int each = units / tiles, more = units - each * tiles;
+      first = col * each + min(col, more);
+      width = each + (col < more ? 1 : 0);
+    }
+    m.cols = 32 * width;
+    m.row0 = rowStart[expert] + 32 * first;
+    m.count = min(m.cols, rows - 32 * first);
+    m.accs = p.tileAccs == 2 && m.w0 + kAccRows < p.N ? 2 : 1;
+    if (it >= fullItems) {                    // half a tile: 256 rows of W (none, when the tile has no second half)
       const int half = (it - fullItems) & 1;
       m.accs = half < m.accs ? 1 : 0;
-      m.w0 += half * (kTileRows / 2);
+      m.w0 += half * kAccRows;
     }
     return m;
+  };
+  const int kbBegin = int(int64_t(kBlocks) * part / parts), kbEnd = int(int64_t(kBlocks) * (part + 1) / parts);   // this pair's k-blocks
+  auto forItems = [&](auto&& body) {
+    for (int it = pairIdx; it < numItems; it += numPairs) {
+      const Item m = itemOf(it);
+      if (m.accs && !body(m)) return;
+    }
+  };
+  // One accumulator alone (a tile of 256 rows of W, half a tile): its columns are two chains of MMAs, the two halves in turn, because
+  // MMAs into the same columns wait for one another. The pair supplies the columns of each MMA in equal shares, so the rows of X are
+  // loaded in quarters then: CTA 0 the first and the third, CTA 1 the others.
+  auto inHalves = [&](const Item& m) { return m.accs == 1 && m.cols % 128 == 0; };
+
+  // The pairs' main loops are over, and a wait that gave up in one of them is known to all: they learn of it through their abort words.
+  auto agree = [&](bool ok) {
+    if (!ok) {
+      const uint32_t word = tc::smemAddr(words + 1);
+      for (int q = 0; q < 2 * parts; ++q) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(tc::mapToCta(word, uint32_t(q))), "r"(1) : "memory");
+    }
+    __syncwarp();
+    tc::clusterSync();
   };
 
   if (warp == 0) {
     if (lane == 0) {
       uint32_t st = 0, ph = 0;
       bool ok = true;
-      for (int it = pairIdx; it < numItems && ok; it += numPairs) {
-        const Item m = itemOf(it);
-        if (m.accs == 0) continue;
-        const int half = m.cols / 2, loads = (half + p.xBox - 1) / p.xBox;
-        const int wRow = m.expert * p.N + m.w0 + int(ctaRank) * kBM, xRow = m.row0 + int(ctaRank) * half;
-        const uint32_t bytes = uint32_t(2 * (m.accs * kABytes + loads * p.xBox * kBK * 2));
-        for (int kb = 0; kb < kBlocks; ++kb) {
+      forItems([&](const Item& m) {
+        const int half = m.cols / 2, loads = (half + kXBox - 1) / kXBox;
+        const bool quarters = inHalves(m);
+        const int wRow = m.expert * p.N + m.w0 + int(ctaRank) * kBM;
+        const int xRow = m.row0 + int(ctaRank) * (quarters ? half / 2 : half), jump = quarters ? half / 2 : 0;
+        const uint32_t bytes = uint32_t(2 * (m.accs * kABytes + loads * kXBox * kBK * 2));
+        for (int kb = kbBegin; kb < kbEnd; ++kb) {
           ok = tc::mbarWait(emptyBar(st), ph ^ 1, abortWord, p.timeoutNs);
-          if (!ok) { skinny::recordTimeout(p.status, 1, it, kb); break; }
-          const uint32_t sW = base + st * kStageBytes, sX = sW + 2 * kABytes;
+          if (!ok) { skinny::recordTimeout(p.status, 1, m.w0, kb); break; }
+          const uint32_t sW = base + st * p.stageBytes, sX = sW + xAt;
           const uint32_t leaderFull = leaderBars + 8u * st;
           if (ctaRank == 0) tc::mbarExpectTx(fullBar(st), bytes);        // both CTAs' bytes are credited to CTA 0's barrier
           tc::tmaLoad2dPair(sW, &maps.w, kb * kBK, wRow, leaderFull);
           if (m.accs == 2) tc::tmaLoad2dPair(sW + kABytes, &maps.w, kb * kBK, wRow + 2 * kBM, leaderFull);
           for (int i = 0; i < loads; ++i)
-            tc::tmaLoad2dPair(sX + uint32_t(i * p.xBox * kBK * 2), &maps.x, kb * kBK, xRow + i * p.xBox, leaderFull);
+            tc::tmaLoad2dPair(sX + uint32_t(i * kXBox * kBK * 2), &maps.x, kb * kBK, xRow + i * kXBox + (2 * i >= loads ? jump : 0), leaderFull);
           if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; }
         }
-      }
+        return ok;
+      });
     }
   } else if (warp == 1) {
     if (lane == 0 && ctaRank == 0) {
-      const uint64_t descW0 = tc::smemDescSw128(base), descX0 = tc::smemDescSw128(base + 2 * kABytes);
-      uint32_t st = 0, ph = 0, use0 = 0, use1 = 0;
+      // descriptors differ only in their 14-bit start address: one constant upper half, the lower halves of the current stage
+      const uint64_t descW0 = tc::smemDescSw128(base), descX0 = tc::smemDescSw128(base + xAt);
+      const uint32_t high = uint32_t(descW0 >> 32), stageStep = p.stageBytes >> 4;
+      auto desc = [&](uint32_t low) { return uint64_t(high) << 32 | low; };
+      uint32_t st = 0, ph = 0, at = 0, use = 0, single = 0;    // at: offset of stage st; bit a of `use`: parity of the uses of accumulator a so far
       bool ok = true;
-      for (int it = pairIdx; it < numItems && ok; it += numPairs) {
-        const Item m = itemOf(it);
-        if (m.accs == 0) continue;
-        const uint32_t idesc = tc::instrDescBf16(uint32_t(m.cols), uint32_t(2 * kBM));
-        const bool two = m.accs == 2;
-        ok = tc::mbarWait(tmemEmptyBar(0), (use0 & 1) ^ 1, abortWord, p.timeoutNs);
-        if (!ok) { skinny::recordTimeout(p.status, 2, it, 0); break; }
+      const int n = kbEnd - kbBegin;
+      forItems([&](const Item& m) {
+        const bool two = m.accs == 2, halves = inHalves(m);
+        const uint32_t idesc = tc::instrDescBf16(uint32_t(halves ? m.cols / 2 : m.cols), uint32_t(2 * kBM));
+        const int a0 = two ? 0 : int(single++ & 1);            // tiles of one accumulator alternate between the two
+        ok = tc::mbarWait(tmemEmptyBar(a0), ((use >> a0) & 1) ^ 1, abortWord, p.timeoutNs);
+        if (!ok) { skinny::recordTimeout(p.status, 2, m.w0, a0); return false; }
         uint32_t accumulate = 0;
         // One thread feeds the tensor cores of two SMs (an MMA takes about 128 cycles), so the loops over the stages hold
         // nothing but waits, MMAs and commits: which accumulators there are is decided outside of them.
         auto landed = [&](int kb) {                            // the k-block in the current stage
           ok = tc::mbarWait(fullBar(st), ph, abortWord, p.timeoutNs);
-          if (!ok) { skinny::recordTimeout(p.status, 3, it, kb); return false; }
+          if (!ok) { skinny::recordTimeout(p.status, 3, m.w0, kb); return false; }
           tc::fenceAfterThreadSync();
           return true;
         };
         auto release = [&]() {                                 // of the current stage, once the MMAs issued so far have read it
-          tc::mmaCommitPair(leaderBars + 8u * (uint32_t(p.stages) + st));
-          tc::mmaCommitPair(peerBars + 8u * (uint32_t(p.stages) + st));
+          tc::mmaCommitPairs(emptyBar(st), pairMask);
         };
-        auto advance = [&]() { if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; } };
+        auto advance = [&]() {
+          at += stageStep;
+          if (++st == uint32_t(p.stages)) { st = 0; at = 0; ph ^= 1; }
+        };
         auto complete = [&](int a) {                           // the epilogue may read accumulator a
-          tc::mmaCommitPair(leaderBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
-          tc::mmaCommitPair(peerBars + 8u * (2u * uint32_t(p.stages) + uint32_t(a)));
+          tc::mmaCommitPairs(tmemFullBar(a), pairMask);
         };
-        auto mma = [&](uint32_t stage, int a, int k, uint32_t acc) {
-          const uint64_t step = uint64_t(stage * (kStageBytes >> 4));
-          tc::mmaPair(tmemBase + uint32_t(a) * kAccStride, descW0 + step + uint32_t(a) * (kABytes >> 4) + 2 * k, descX0 + step + 2 * k, idesc, acc);
-        };
+        const uint32_t w0 = uint32_t(descW0), w1 = w0 + (kABytes >> 4), x0 = uint32_t(descX0);
+        const uint32_t d0 = tmemBase + uint32_t(a0) * kAccStride, d1 = tmemBase + kAccStride;
         if (two) {
-          const int ends = min(kLead, kBlocks / 2);
+          const int ends = min(kLead, n / 2);
           auto oneThenOther = [&](int kb0, bool last) {
-            const uint32_t st0 = st, ph0 = ph;
+            const uint32_t st0 = st, ph0 = ph, at0 = at;
             for (int i = 0; i < ends && ok; ++i) {
               if (!landed(kb0 + i)) return;
 #pragma unroll
-              for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); accumulate = 1; }
+              for (int k = 0; k < kBK / 16; ++k) { tc::mmaPair(d0, desc(w0 + at + 2 * k), desc(x0 + at + 2 * k), idesc, accumulate); accumulate = 1; }
               advance();
             }
             if (last) complete(0);
-            else ok = tc::mbarWait(tmemEmptyBar(1), (use1 & 1) ^ 1, abortWord, p.timeoutNs);
-            if (!ok) { skinny::recordTimeout(p.status, 2, it, 1); return; }
-            st = st0; ph = ph0;
+            else ok = tc::mbarWait(tmemEmptyBar(1), ((use >> 1) & 1) ^ 1, abortWord, p.timeoutNs);
+            if (!ok) { skinny::recordTimeout(p.status, 2, m.w0, 1); return; }
+            st = st0; ph = ph0; at = at0;
             for (int i = 0; i < ends; ++i) {
 #pragma unroll
-              for (int k = 0; k < kBK / 16; ++k) mma(st, 1, k, uint32_t(last || i || k));
+              for (int k = 0; k < kBK / 16; ++k) tc::mmaPair(d1, desc(w1 + at + 2 * k), desc(x0 + at + 2 * k), idesc, uint32_t(last || i || k));
               release();
               advance();
             }
           };
           oneThenOther(0, false);
-          for (int kb = ends; kb < kBlocks - ends && ok; ++kb) {
+          for (int kb = ends; kb < n - ends && ok; ++kb) {
             if (!landed(kb)) break;
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); mma(st, 1, k, accumulate); accumulate = 1; }
+            for (int k = 0; k < kBK / 16; ++k) {
+              tc::mmaPair(d0, desc(w0 + at + 2 * k), desc(x0 + at + 2 * k), idesc, accumulate);
+              tc::mmaPair(d1, desc(w1 + at + 2 * k), desc(x0 + at + 2 * k), idesc, accumulate);
+              accumulate = 1;
+            }
             release();
             advance();
           }
-          if (ok) oneThenOther(kBlocks - ends, true);
-          if (ok) { complete(1); ++use0; ++use1; }
+          if (ok) oneThenOther(n - ends, true);
+          if (ok) { complete(1); use ^= 3u; }
+        } else if (halves) {
+          const uint32_t dh = d0 + uint32_t(m.cols / 2), xh = x0 + uint32_t(m.cols / 4 * kBK * 2 >> 4);
+          for (int kb = 0; kb < n; ++kb) {
+            if (!landed(kb)) break;
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) {
+              tc::mmaPair(d0, desc(w0 + at + 2 * k), desc(x0 + at + 2 * k), idesc, accumulate);
+              tc::mmaPair(dh, desc(w0 + at + 2 * k), desc(xh + at + 2 * k), idesc, accumulate);
+              accumulate = 1;
+            }
+            release();
+            advance();
+          }
         } else {
-          for (int kb = 0; kb < kBlocks; ++kb) {
+          for (int kb = 0; kb < n; ++kb) {
             if (!landed(kb)) break;
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k) { mma(st, 0, k, accumulate); accumulate = 1; }
+            for (int k = 0; k < kBK / 16; ++k) { tc::mmaPair(d0, desc(w0 + at + 2 * k), desc(x0 + at + 2 * k), idesc, accumulate); accumulate = 1; }
             release();
             advance();
           }
-          if (ok) { complete(0); ++use0; }
         }
-      }
+        if (ok && !two) { complete(a0); use ^= 1u << a0; }
+        return ok;
+      });
     }
   } else {
     // ------------------------------- epilogue -------------------------------
@@ -272,81 +337,149 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     // transposed store nor the reads meet in a bank
     auto stagedAt = [&](int row, int piece) { return buf + uint32_t(row * kPitch + ((piece ^ ((row * kPitch >> 7) & (kPieces - 1))) << 4)); };
     const int piece = lane % kPieces, rr = lane / kPieces;
-    uint32_t use = 0;                                          // bit a: parity of the uses of accumulator a so far
+    auto f = [](uint32_t v) { return __uint_as_float(v); };
+    // 32 columns (tokens) of this warp's 32 rows of W, fragments of rows 0-15 and of rows 16-31 -> activated and packed
+    auto activate = [&](const uint32_t (&lo)[16], const uint32_t (&hi)[16], uint32_t (&h)[kHeld]) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if constexpr (SWIGLU)                                  // rows 0-15 are gate, 16-31 up, of the same 16 output columns
+          h[i] = skinny::pack2(skinny::siluOf(f(lo[2 * i])) * f(hi[2 * i]), skinny::siluOf(f(lo[2 * i + 1])) * f(hi[2 * i + 1]));
+        else {
+          h[i] = skinny::pack2(f(lo[2 * i]), f(lo[2 * i + 1]));
+          h[8 + i] = skinny::pack2(f(hi[2 * i]), f(hi[2 * i + 1]));
+        }
+      }
+    };
+    // ... -> C, turned around on the way through the staging tile: rows of W become columns of C. c: first column of the chunk.
+    auto store = [&](const Item& m, int block, int c, const uint32_t (&h)[kHeld]) {
+      const int wRow = m.w0 + block * kAccRows + int(ctaRank) * kBM + quarter * 32;  // of lane 0
+      const int n0 = (SWIGLU ? wRow / 2 : wRow) + piece * 8;
+      const bool colOk = n0 + 8 <= outCols;
+      __nv_bfloat16* out = p.C + size_t(m.row0) * p.ldc + n0;
+      if constexpr (SWIGLU) {
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+          tc::stMatrixTransposed4(stagedAt(8 * (i + (lane >> 4)) + (lane & 7), (lane >> 3) & 1), h[2 * i], h[2 * i + 1], h[2 * i + 2], h[2 * i + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          tc::stMatrixTransposed4(stagedAt(8 * i + (lane & 7), lane >> 3), h[2 * i], h[2 * i + 1], h[8 + 2 * i], h[8 + 2 * i + 1]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        Vec16 v;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]) : "r"(stagedAt(i * kRowsPer + rr, piece)) : "memory");
+        const int row = c + i * kRowsPer + rr;
+        if (colOk && row < m.count) st16(out + size_t(row) * p.ldc, v);
+      }
+      __syncwarp();                                            // the tile has been read before the next chunk fills it
+    };
+    auto load = [&](int a, int c, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
+      const uint32_t taddr = tmemBase + (uint32_t(quarter * 32) << 16) + uint32_t(a) * kAccStride + uint32_t(c);
+      tc::tmemLoadFragments(taddr, lo);
+      tc::tmemLoadFragments(taddr + (16u << 16), hi);
+      tc::tmemLoadWaitFor(lo);
+      tc::tmemLoadWaitFor(hi);
+    };
+    uint32_t use = 0, single = 0;                              // as in the MMA warp
     bool ok = true;
-    for (int it = pairIdx; it < numItems && ok; it += numPairs) {
-      const Item m = itemOf(it);
-      // into registers, activated and packed; the accumulator goes back to the MMA warp
-      uint32_t held[2][kChunks][kHeld];
+    auto finished = [&](const Item& m, int a) {
+      ok = tc::mbarWait(tmemFullBar(a), (use >> a) & 1, abortWord, p.timeoutNs);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) { if (lane == 0) skinny::recordTimeout(p.status, 5, m.w0, a); return false; }
+      use ^= 1u << a;
+      tc::fenceAfterThreadSync();
+      return true;
+    };
+    if constexpr (!SPLIT) {
+      forItems([&](const Item& m) {
+        const int a0 = m.accs == 2 ? 0 : int(single++ & 1);
+        // into registers, activated and packed; the accumulator goes back to the MMA warp
+        uint32_t held[2][kChunks][kHeld];
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        if (a >= m.accs || !ok) continue;
-        ok = tc::mbarWait(tmemFullBar(a), (use >> a) & 1, abortWord, p.timeoutNs);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) { if (lane == 0) skinny::recordTimeout(p.status, 5, it, a); continue; }
-        use ^= 1u << a;
-        tc::fenceAfterThreadSync();
-        const uint32_t taddr = tmemBase + (uint32_t(quarter * 32) << 16) + uint32_t(a) * kAccStride + uint32_t(group * 32);
-        // 32 columns (tokens) of this warp's 32 rows of W at a time, as fragments of rows 0-15 and of rows 16-31
+        for (int b = 0; b < 2; ++b) {
+          if (b >= m.accs || !ok || !finished(m, a0 + b)) continue;
 #pragma unroll
-        for (int j = 0; j < kChunks; ++j) {
-          if (group * 32 + j * 64 >= m.count) continue;
-          uint32_t lo[16], hi[16];
-          tc::tmemLoadFragments(taddr + uint32_t(j * 64), lo);
-          tc::tmemLoadFragments(taddr + (16u << 16) + uint32_t(j * 64), hi);
-          tc::tmemLoadWaitFor(lo);
-          tc::tmemLoadWaitFor(hi);
-          auto f = [](uint32_t v) { return __uint_as_float(v); };
+          for (int j = 0; j < kChunks; ++j) {
+            if (group * 32 + j * 64 >= m.count) continue;
+            uint32_t lo[16], hi[16];
+            load(a0 + b, group * 32 + j * 64, lo, hi);
+            activate(lo, hi, held[b][j]);
+          }
+          tc::fenceBeforeThreadSync();
+          __syncwarp();
+          if (lane == 0) tc::mbarArriveCluster(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a0 + b)));
+        }
+        if (!ok) return false;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            if constexpr (SWIGLU)                              // rows 0-15 are gate, 16-31 up, of the same 16 output columns
-              held[a][j][i] = skinny::pack2(skinny::siluOf(f(lo[2 * i])) * f(hi[2 * i]), skinny::siluOf(f(lo[2 * i + 1])) * f(hi[2 * i + 1]));
-            else {
-              held[a][j][i] = skinny::pack2(f(lo[2 * i]), f(lo[2 * i + 1]));
-              held[a][j][8 + i] = skinny::pack2(f(hi[2 * i]), f(hi[2 * i + 1]));
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int j = 0; j < kChunks; ++j)
+            if (b < m.accs && group * 32 + j * 64 < m.count) store(m, b, group * 32 + j * 64, held[b][j]);
+        return true;
+      });
+    } else {
+      // (one item, so accumulator b is b) a chunk c of accumulator b is finished by pair c % parts, there it has a slot for every other
+      // pair; a warp's 32 x 32 values lie in it as the fragments lie in registers, 512 bytes per access of the warp
+      const int slots = (kMaxCols / 32 + parts - 1) / parts;
+      auto slotOf = [&](int from, int at, int b, int c) {
+        const int q = from < at ? from : from - 1;
+        return base + uint32_t((((q * 2 + b) * slots + c / parts) * 4 + quarter) * 4096 + lane * 16);
+      };
+      forItems([&](const Item& m) { for (int b = 0; b < m.accs && finished(m, b); ++b) {} return ok; });
+      agree(ok);
+      forItems([&](const Item& m) {
+        for (int b = 0; b < m.accs; ++b)
+          for (int c = group; c * 32 < m.count; c += 2) {
+            if (c % parts == part || *abortWord) continue;
+            uint32_t lo[16], hi[16];
+            load(b, c * 32, lo, hi);
+            const uint32_t to = tc::mapToCta(slotOf(part, c % parts, b, c), uint32_t(c % parts) * 2 + ctaRank);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              stCluster16(to + i * 512, lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]);
+              stCluster16(to + (i + 4) * 512, hi[4 * i], hi[4 * i + 1], hi[4 * i + 2], hi[4 * i + 3]);
             }
           }
-        }
-        tc::fenceBeforeThreadSync();
-        __syncwarp();
-        if (lane == 0) tc::mbarArriveCluster(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a)));
-      }
-      if (!ok) break;
+        return true;
+      });
+      __syncwarp();
+      tc::clusterSync();
+      forItems([&](const Item& m) {
+        for (int b = 0; b < m.accs; ++b)
+          for (int c = group; c * 32 < m.count; c += 2) {
+            if (c % parts != part || *abortWord) continue;
+            uint32_t lo[16], hi[16], own[2][16], h[kHeld];
+            load(b, c * 32, own[0], own[1]);
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        if (a >= m.accs) continue;
-        const int wRow = m.w0 + a * 2 * kBM + int(ctaRank) * kBM + quarter * 32;     // of lane 0
-        const int n0 = (SWIGLU ? wRow / 2 : wRow) + piece * 8;
-        const bool colOk = n0 + 8 <= outCols;
-        __nv_bfloat16* out = p.C + size_t(m.row0) * p.ldc + n0;
+            for (int i = 0; i < 16; ++i) lo[i] = hi[i] = 0u;
+            auto add = [&](uint32_t& to, uint32_t x) { to = __float_as_uint(f(to) + f(x)); };
+#pragma unroll 1
+            for (int q = 0; q < parts; ++q) {
+              if (q == part) {
 #pragma unroll
-        for (int j = 0; j < kChunks; ++j) {
-          const int c = group * 32 + j * 64;
-          if (c >= m.count) continue;
-          const uint32_t (&h)[kHeld] = held[a][j];
-          // turned around on the way into the staging tile: rows of W become columns of C
-          if constexpr (SWIGLU) {
+                for (int i = 0; i < 16; ++i) { add(lo[i], own[0][i]); add(hi[i], own[1][i]); }
+              } else {
+                const uint32_t from = slotOf(q, part, b, c);
 #pragma unroll
-            for (int i = 0; i < 4; i += 2)
-              tc::stMatrixTransposed4(stagedAt(8 * (i + (lane >> 4)) + (lane & 7), (lane >> 3) & 1), h[2 * i], h[2 * i + 1], h[2 * i + 2], h[2 * i + 3]);
-          } else {
+                for (int i = 0; i < 4; ++i) {
+                  uint32_t v[4], u[4];
+                  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(from + i * 512) : "memory");
+                  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(from + (i + 4) * 512) : "memory");
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              tc::stMatrixTransposed4(stagedAt(8 * i + (lane & 7), lane >> 3), h[2 * i], h[2 * i + 1], h[8 + 2 * i], h[8 + 2 * i + 1]);
+                  for (int e = 0; e < 4; ++e) { add(lo[4 * i + e], v[e]); add(hi[4 * i + e], u[e]); }
+                }
+              }
+            }
+            activate(lo, hi, h);
+            store(m, b, c * 32, h);
           }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < kPieces; ++i) {
-            Vec16 v;
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]) : "r"(stagedAt(i * kRowsPer + rr, piece)) : "memory");
-            const int row = c + i * kRowsPer + rr;
-            if (colOk && row < m.count) st16(out + size_t(row) * p.ldc, v);
-          }
-          __syncwarp();                                        // the tile has been read before the next chunk fills it
-        }
-      }
+        return true;
+      });
     }
   }
+  if (SPLIT && warp < 2) { agree(*abortWord == 0); __syncwarp(); tc::clusterSync(); }      // the two barriers of the exchange
 
   if (*abortWord) __nanosleep(20000);   // let copies already in flight land before shared memory and TMEM go away
   __syncwarp();

@@ -135,6 +135,10 @@ PURLIN_D void mmaPair(uint32_t tmemD, uint64_t aDesc, uint64_t bDesc, uint32_t i
 PURLIN_D void mmaCommitPair(uint32_t clusterBarAddress) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(clusterBarAddress) : "memory");
 }
+// the same on the barrier at this CTA's address `bar` in every CTA of the mask
+PURLIN_D void mmaCommitPairs(uint32_t bar, uint32_t ctaMask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(uint16_t(ctaMask)) : "memory");
+}
 
 // ---- TMEM ----
 PURLIN_D void tmemAlloc(uint32_t smemResult, uint32_t columns) {   // whole warp

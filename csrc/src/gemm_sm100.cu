@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -850,16 +851,20 @@ struct GroupedArgs {
 bool fewWeightRows(int M, int N, int K, int epilogue) { return epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens && K >= 2048; }
 bool useSkinny(int M, int N, int K, int epilogue) {
   if (fewWeightRows(M, N, K, epilogue)) return true;
-  // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 57344 x 8192 153 / 165, 48 x 4096 x 4096 14 / 22,
-  // 64 x 264 x 528 5.8 / 6.7; but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4, 64 x 14336 x 512 SwiGLU 9.8 / 8.6
-  if (M <= 64) return M <= 32 || K >= (N <= 8192 ? 512 : 1024);
-  // up to 128 while W has too few rows to give every SM a tile of its own and k is worth splitting: 128 x 8192 x 7168 31.5 /
-  // 37.6, 128 x 1024 x 4096 12 / 22.7, 96 x 8192 x 4096 21.6 / 23.5; but 128 x 8192 x 1024 11.2 / 9.8, 128 x 14336 x 4096 28.2 /
-  // 27.4, 128 x 264 x 72 7.4 / 5.3
-  if (M <= 128) return N <= 8192 && K >= (N < 4096 ? 1024 : 1536);
-  // up to 256 where the tiles are few and k is long: 256 x 4096 x 4096 21.2 / 25.1, 256 x 8192 x 7168 40.4 / 42.4, 140 x 8192 x
-  // 4096 21.1 / 22.6; but 200 x 8192 x 4096 25.5 / 24.1, 200 x 14336 x 8192 74.9 / 67.5, 200 x 264 x 72 9.2 / 5.3
-  return M <= skinny::kMaxTokens && N >= 4096 && N <= 8192 && K >= (M <= 160 || N == 4096 ? 4096 : 6144);
+  // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 4096 x 1024 7.9 / 8.3, 54 x 7648 x 1336 SwiGLU 14.3 / 17.2;
+  // but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4. Above, what the others would take decides (gemmRoute).
+  return M <= 64 && (M <= 32 || K >= (N <= 8192 ? 512 : 1024));
+}
+// Parts that the few-rows kernel cuts k into: while the CTAs have a place on the GPU at the same time and a part keeps at least four
+// k-blocks; eight where many tiles are split four ways (64 x 7744 x 1160, 61 tiles: 12.0 us whole, 10.6 in two parts, 13.0 in four).
+// Measured, 1 x 8192 x 3584: one CTA per tile 20.1 us, two 14.4, four 14.2, eight 18.2; 64 x 8192 x 28672: 142.6 / 87.4 / 79.1 /
+// 90.5 us. More CTAs than places cost a second wave: 64 x 11232 x 1952 SwiGLU (88 tiles, 296 places) 16.6 / 14.7 / 26.7,
+// 192 x 5824 x 1280 (46 tiles, 148 places) 17.0 / 13.1 / 23.9. At most 15 clusters of eight fit on the GPU at once, so eight
+// are used for no more tiles than that.
+int skinnySplit(long tiles, int kBlocks, long slots) {
+  int split = 1;
+  while (split < (tiles <= 15 ? skinny::kMaxSplit : 4) && tiles * split * 2 <= slots && kBlocks >= (split > 1 && tiles > 24 ? 16 : 8) * split) split *= 2;
+  return split;
 }
 
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
@@ -883,17 +888,9 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   const int budget = (perSm == 2 ? 113 : 227) * 1024 - 1024 - skinny::kBarrierBytes;
   p.stages = std::min(budget / stageBytes, skinny::kMaxStages);
   for (p.tmemCols = 32; p.tmemCols < p.passTokens; p.tmemCols *= 2) {}
-  // Split k while the CTAs have a place on the GPU at the same time and a part keeps at least four k-blocks; eight where many
-  // tiles are split four ways (64 x 7744 x 1160, 61 tiles: 12.0 us whole, 10.6 in two parts, 13.0 in four). Measured,
-  // 1 x 8192 x 3584: one CTA per tile 20.1 us, two 14.4, four 14.2, eight 18.2; 64 x 8192 x 28672: 142.6 / 87.4 / 79.1 /
-  // 90.5 us. More CTAs than places cost a second wave: 64 x 11232 x 1952 SwiGLU (88 tiles, 296 places) 16.6 / 14.7 / 26.7,
-  // 192 x 5824 x 1280 (46 tiles, 148 places) 17.0 / 13.1 / 23.9. At most 15 clusters of eight fit on the GPU at once, so eight
-  // are used for no more tiles than that.
   const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
   const long slots = long(smCount()) * perSm;
-  const long allTiles = long(tiles) * g.experts;
-  int split = 1;
-  while (split < (allTiles <= 15 ? skinny::kMaxSplit : 4) && allTiles * split * 2 <= slots && kBlocks >= (split > 1 && allTiles > 24 ? 16 : 8) * split) split *= 2;
+  const int split = skinnySplit(long(tiles) * g.experts, kBlocks, slots);
   skinny::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
   const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;
@@ -927,79 +924,173 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
 constexpr int kFewGroupRows = 12;
 
 // ---- any number of rows of activations: gemm_ragged.cuh ----
-int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
+constexpr int kMaxParts = 4;            // pairs of a cluster (eight CTAs, the largest portable cluster)
+auto raggedKernel(int epilogue, bool split) {
+  return epilogue == kEpiSwiglu ? (split ? ragged::raggedGemmKernel<true, true> : ragged::raggedGemmKernel<true, false>)
+                                : (split ? ragged::raggedGemmKernel<false, true> : ragged::raggedGemmKernel<false, false>);
+}
+constexpr size_t kRaggedSmem = 1024 + ragged::kRingBytes + ragged::kStagingBytes + ragged::kBarrierBytes + ragged::kTableBytes;
+static_assert(kRaggedSmem <= size_t(kSmemLimit), "the ring, the staging tiles and the tables fit one CTA per SM");
+static_assert(ragged::kRingBytes >= (kMaxParts - 1) * 2 * (ragged::kMaxCols / 32 / kMaxParts) * 4 * 4096 &&
+              ragged::kRingBytes >= 2 * (ragged::kMaxCols / 32 / 2) * 4 * 4096, "the partial tiles of the other pairs take the place of the stages");
+// stages of a ring for `accs` accumulators and `cols` columns per tile
+int raggedStages(int accs, int cols, uint32_t& stageBytes) {
+  stageBytes = uint32_t(accs * ragged::kABytes + (cols / 2 + ragged::kXBox - 1) / ragged::kXBox * ragged::kXBox * kBK * 2);
+  return std::min(int(ragged::kRingBytes / stageBytes), ragged::kMaxStages);
+}
+static_assert(ragged::kRingBytes / (2 * ragged::kABytes + ragged::kMaxCols / 2 * kBK * 2) >= ragged::kLead, "a lead holds its stages until the second accumulator has read them");
+
+// Clusters of `parts` pairs (1, 2 or 4) that the device can hold at once; 0: none, or with the error set for one pair
+int raggedClusters(int epilogue, int parts) {
+  static std::mutex mu;
+  static int known[64][2][3] = {};      // (0: not asked yet, -1: none)
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) { setError("GEMM launch: no current device"); return 0; }
+  std::lock_guard<std::mutex> lock(mu);
+  int& clusters = known[device][epilogue == kEpiSwiglu ? 1 : 0][parts / 2];
+  if (!clusters) {
+    auto kernel = raggedKernel(epilogue, parts > 1);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess) { setError("cannot opt in to 227 KiB of shared memory"); return 0; }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(2 * parts); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(unsigned(smCount() / (2 * parts) * (2 * parts))); cfg.blockDim = dim3(ragged::kThreads); cfg.dynamicSmemBytes = kRaggedSmem; cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    clusters = parts == 1 ? smCount() / 2 : -1;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) clusters = std::min(smCount() / (2 * parts), n);
+  }
+  return std::max(clusters, 0);
+}
+
+// How the ragged kernel cuts a GEMM: one or two accumulators per tile, the number of column tiles, and how many pairs share a tile's k
+// range, whichever has the least expected time. The cycles are a model, its constants fitted to about 700 shapes on one B200:
+//   a k-block of a tile of two accumulators takes the tensor pipe 4 cycles a column, and its operands come at 44 bytes a cycle and SM;
+//   of one accumulator 500 and 2.1 a column (the round trips of its loads); rows of K that begin off a cache line 12 % more;
+//   drain: what a tile's epilogue exposes; behind the last one its stores remain;
+//   a cluster of several pairs is placed later than a pair (3500 cycles a pair) and exchanges partial tiles at 12 bytes a cycle;
+//   the weights come through HBM once.
+// What it buys, us, one B200, before / now: 2048 x 14336 x 8192 SwiGLU 371 / 325 (ten column tiles, where eight left a fourth wave of two
+// tiles), 1000 x 14336 x 8192 SwiGLU 205 / 168, 1000 x 8192 x 7168 97 / 85, 384 x 14336 x 8192 SwiGLU 121 / 78, 700 x 8192 x 28672 428 / 250;
+// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58. Over 900 random
+// shapes the geometric mean is 1.08; 18 are slower by more than 3 %, the worst by 14 % (4871 x 368 x 1456 15.6 / 18.6).
+struct RaggedPlan { int tileAccs = 2, colTiles = 1, tiles = 1, parts = 1; double cycles = 0; };
+RaggedPlan raggedPlan(int M, int N, int K, int epilogue, const int (&clusters)[3]) {
+  const int kBlocks = (K + kBK - 1) / kBK, units = (M + 31) / 32, fewest = (units + 7) / 8;
+  const double unaligned = K % kBK ? 1.12 : 1.;                 // rows of K that do not begin on a cache line
+  RaggedPlan best;
+  for (int accs = 1; accs <= 2; ++accs) {
+    // the fewest column tiles, one and two more, and the numbers that just fill one to three waves more than the fewest need
+    const int64_t wTiles = (N + accs * ragged::kAccRows - 1) / (accs * ragged::kAccRows), waves = fewest * wTiles / clusters[0];
+    for (int c = 0; c < 6; ++c) {
+      const int64_t want = c < 3 ? fewest + c : (waves + c - 2) * clusters[0] / wTiles;
+      if (want < fewest || want > units || want > 2 * fewest + 2) continue;
+      const int n = int(want);
+      const int64_t tiles = n * wTiles;
+      const double cols = 32. * units / n;                       // of a tile, on average
+      auto perBlock = [&](int a) {
+        if (a == 1) return (500 + 2.1 * cols) * unaligned;
+        return std::max(4 * cols, (2 * ragged::kABytes + cols * 64) / 44 * unaligned);
+      };
+      auto drain = [&](int a) { return 1200. + a * cols * (epilogue == kEpiSwiglu ? 8. : 3.); };
+      for (int parts = 1; parts <= kMaxParts; parts *= 2) {
+        const int places = clusters[parts / 2];
+        if (!places || kBlocks < 8 * parts) break;
+        if (parts > 1 && tiles > places) break;
+        const int64_t full = tiles / places, rest = tiles % places;
+        const double whole = (kBlocks + parts - 1) / parts * perBlock(accs) + drain(accs) + (parts > 1 ? 3500. * parts + accs * cols * 512. * (parts - 1) / parts / 12 : 0.);
+        const double tail = rest == 0 ? 0. : parts == 1 && accs == 2 && 2 * rest <= places ? kBlocks * perBlock(1) + drain(1) : whole;
+        // the weights once through HBM, at least
+        const double cycles = std::max(double(full) * whole + tail, (2. * N * K + 2. * M * K) / 3300. * unaligned) + 4500. + accs * cols * 8.;
+        if (best.cycles == 0 || cycles < best.cycles) best = RaggedPlan{accs, n, int(std::min<int64_t>(tiles, INT32_MAX / 4)), parts, cycles};
+      }
+    }
+  }
+  return best;
+}
+
+int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, const RaggedPlan& plan, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
   if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
   if (g.experts > ragged::kMaxExperts) { setError("grouped GEMM: at most 512 experts"); return 1; }
-  auto kernel = epilogue == kEpiSwiglu ? ragged::raggedGemmKernel<true> : ragged::raggedGemmKernel<false>;
-  static std::mutex mu;
-  static int pairsOf[64][2] = {};      // CTA pairs the device can hold at once (0: not asked yet)
-  int device = 0, pairs = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) { setError("GEMM launch: no current device"); return 1; }
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1] = overlapAttribute();
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  cfg.blockDim = dim3(ragged::kThreads);
-  constexpr int stageBytes = 2 * ragged::kABytes + ragged::kMaxCols / 2 * ragged::kBK * 2;
-  constexpr int fixedBytes = 1024 + ragged::kStagingBytes + ragged::kBarrierBytes + ragged::kTableBytes;
-  constexpr int stages = (kSmemLimit - fixedBytes) / stageBytes < ragged::kMaxStages ? (kSmemLimit - fixedBytes) / stageBytes : ragged::kMaxStages;
-  static_assert(stages >= ragged::kLead, "a lead holds its stages until the second accumulator has read them");
-  cfg.dynamicSmemBytes = size_t(stages) * stageBytes + fixedBytes;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    int& known = pairsOf[device][epilogue == kEpiSwiglu ? 1 : 0];
-    if (!known) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess) { setError("cannot opt in to 227 KiB of shared memory"); return 1; }
-      int n = 0;
-      cfg.gridDim = dim3(unsigned(smCount() / 2 * 2));
-      known = smCount() / 2;
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) known = std::min(known, n);
-    }
-    pairs = known;
-  }
+  const int pairs = raggedClusters(epilogue, 1);
+  if (!pairs) return 1;
   ragged::Params p{};
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.experts = g.experts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
-  p.stages = stages; p.status = status; p.timeoutNs = g.timeoutNs;
-  const int wTiles = (N + ragged::kTileRows - 1) / ragged::kTileRows;
+  p.status = status; p.timeoutNs = g.timeoutNs;
+  p.tileAccs = 2; p.colTiles = 1; p.parts = 1;
+  // (groups of a few dozen rows: narrow tiles leave room for a fifth stage)
+  p.maxCols = g.counts && g.likelyRows <= 40 ? 64 : ragged::kMaxCols;
   int items = INT32_MAX;
-  p.tileCols = ragged::kMaxCols; p.xBox = 32;
   if (!g.counts) {
-    // The cut that leaves the pairs least idle. A tile takes about as long as its columns, in steps of 64, and 57 more do
-    // (measured per wave at K = 8192: 256 columns 90 us, 224 89 us, 192 72.5 us, 160 71.5 us); half tiles in the last wave
-    // take about 0.85 of a whole one.
-    auto cost = [](int cols) { return double((cols + 63) / 64 * 64 + 57); };
-    double best = -1;
-    for (int cols : {256, 192, 128}) {
-      const long full = M / cols, rem = M % cols ? 1 : 0, tiles = (full + rem) * wTiles, rest = tiles % pairs;
-      const double tail = rest == 0 ? 0. : 2 * rest <= pairs ? 0.85 : 1.;
-      const double average = (double(full) * cost(cols) + double(rem) * cost(M % cols)) / double(full + rem);
-      const double time = tiles > pairs ? (double(tiles / pairs) + tail) * average : (tiles == pairs ? 1. : tail) * cost(full ? cols : M % cols);
-      if (best < 0 || time < best * 0.99) { best = time; p.tileCols = cols; items = int(std::min<long>(2 * tiles, INT32_MAX)); }
-    }
-    p.xBox = p.tileCols / 2;
+    p.tileAccs = plan.tileAccs; p.colTiles = plan.colTiles; p.parts = plan.parts;
+    p.maxCols = ((M + 31) / 32 + plan.colTiles - 1) / plan.colTiles * 32;
+    items = plan.parts > 1 ? plan.tiles : plan.tileAccs * plan.tiles;      // (the tiles of a small last wave are issued as halves)
   }
+  p.stages = raggedStages(p.tileAccs, p.maxCols, p.stageBytes);
   ragged::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), ragged::kBM) ||
-      !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.xBox))) return 1;
-  cfg.gridDim = dim3(unsigned(std::min(pairs, items) * 2)); cfg.stream = stream;
+      !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(ragged::kXBox))) return 1;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(2 * p.parts); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1] = overlapAttribute();
+  const int grid = (p.parts > 1 ? items : std::min(pairs, items)) * 2 * p.parts;
+  cfg.attrs = attr; cfg.blockDim = dim3(ragged::kThreads); cfg.dynamicSmemBytes = kRaggedSmem; cfg.gridDim = dim3(unsigned(grid)); cfg.stream = stream;
   // (fewer tiles than pairs: the pairs without one leave at once; 2066 x 3144 x 4264, 63 tiles: 49.7 us apart, 58.0 overlapped)
-  cfg.numAttrs = betterApart(items, K) ? 1 : 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
+  cfg.numAttrs = betterApart(p.parts > 1 ? grid : items, K) ? 1 : 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, raggedKernel(epilogue, p.parts > 1), maps, p);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
 }
 
-// Rows that are no multiple of 512 go through the ragged kernel once its 512 x 256 tiles give five eighths of the CTA pairs
-// work (one B200, us, it / the tiles of this file: 1000 x 14336 x 8192 177 / 222, 1000 x 8192 x 7168 83 / 104, 5000 x 4096 x
-// 4096 126 / 158, 1500 x 4096 x 4096 41 / 62; with fewer tiles 700 x 4096 x 4096 51 / 31, 300 x 8192 x 7168 61 / 56) and k is
-// long enough to hide its epilogue, which stands between the tiles and stores short row pieces (3189 x 1672 x 840 17.4 / 24.4,
-// 1121 x 18144 x 968 42 / 53, 2277 x 11680 x 1016 SwiGLU 56 / 79; but 4144 x 3296 x 512 22.8 / 15.3, 3708 x 20672 x 336 SwiGLU
-// 88 / 58, 3357 x 20472 x 80 61 / 37).
-bool useRagged(int M, int N, int K) {
-  const long tiles = long((M + ragged::kMaxCols - 1) / ragged::kMaxCols) * ((N + ragged::kTileRows - 1) / ragged::kTileRows);
-  return M % (4 * kBM) != 0 && K >= 768 && tiles * 16 >= long(smCount()) * 5;
+// The plain tiles of this file on the same scale.
+double plainCycles(const Params& p, const Shape& sh, int epilogue) {
+  const double tiles = double(p.tilesM) * p.tilesN, places = sh.ctas == 2 ? smCount() / 2 : smCount();
+  const double block = sh.accs == 2 ? std::max(4. * p.bn, 900.) : std::max({2. * p.bn + 184., (kABytes + p.bn / sh.ctas * 128) / 58., 700.});
+  const double drain = sh.accs == 2 ? (epilogue == kEpiSwiglu ? 9000. : 6000.) * p.bn / 256 : 0.;
+  const double waves = std::ceil(tiles / places), ragged = p.K % kBK ? 1.25 : 1.;      // rows of K that do not begin on a cache line
+  return std::max(waves * ((p.K + kBK - 1) / kBK * block * ragged + drain) + 3000., (2. * p.N * p.K + 2. * p.M * p.K) / 3300. * ragged);
+}
+
+// ... and the few-rows kernel: its CTAs' round trips (per k-block 450 cycles and 3.5 per row, measured with L2-sized weights) or the
+// weights, and a fixed part that grows with the rows (the partial tiles through distributed shared memory).
+double skinnyCycles(int M, int N, int K, int epilogue) {
+  if (M > skinny::kMaxTokens || N > 16384) return 1e30;
+  const long tiles = (N + skinny::kRows - 1) / skinny::kRows, slots = long(smCount()) * (M <= 128 ? 2 : 1);
+  const int kBlocks = (K + skinny::kK - 1) / skinny::kK, split = skinnySplit(tiles, kBlocks, slots);
+  const double waves = std::ceil(double(tiles * split) / slots), block = (450. + 3.5 * M) * (tiles * split > smCount() ? 1.3 : 1.);
+  return std::max(waves * kBlocks / split * block, 1.15 * (2. * N * K + 2. * M * K) / 3300.) + 7000. + (epilogue == kEpiSwiglu ? 105. : 45.) * M;
+}
+
+// Which kernel a GEMM takes, and its cut if it is the ragged one: the least expected time. The ragged kernel was 3 % ahead of the plain
+// tiles at 4096 x 8192 x 7168 (326 / 351 us) and 8192 x 2048 x 1024 (28.8 / 30.7), behind at 2048 x 4096 x 512 (13.8 / 12.1) and 1000 x 4096
+// x 4096 (36 / 33, one wave of narrower tiles); the few-rows kernel ahead at 128 x 8192 x 8192 (33.6, ragged 37.5, plain 42.2), behind at
+// 128 x 8192 x 2048 (18.2, plain 13.9) and 160 x 8192 x 8192 (38.6, ragged 36.6).
+enum { kRoutePlain = 0, kRouteSkinny = 1, kRouteRagged = 2 };
+struct Route { int M = 0, N = 0, K = 0, epilogue = 0, device = -1, kernel = kRoutePlain; RaggedPlan cut; };
+Route findRoute(const Params& p, const Shape& sh, int epilogue) {
+  Route r;
+  if (useSkinny(p.M, p.N, p.K, epilogue)) { r.kernel = kRouteSkinny; return r; }
+  const double plain = plainCycles(p, sh, epilogue), skinny = p.M > 64 ? skinnyCycles(p.M, p.N, p.K, epilogue) : 1e30;
+  double ragged = 1e30;
+  if (p.K >= 512 && !switches().singleCta && !switches().oneAcc) {
+    const int clusters[3] = {raggedClusters(epilogue, 1), raggedClusters(epilogue, 2), raggedClusters(epilogue, 4)};
+    if (clusters[0]) { r.cut = raggedPlan(p.M, p.N, p.K, epilogue, clusters); ragged = r.cut.cycles; }
+  }
+  r.kernel = skinny < std::min(plain, ragged) ? kRouteSkinny : ragged < plain ? kRouteRagged : kRoutePlain;
+  return r;
+}
+// A function of the sizes (and of the device's cluster counts): each thread keeps those of its recent sizes, a microsecond of host time.
+const Route& gemmRoute(const Params& p, const Shape& sh, int epilogue) {
+  static thread_local Route recent[64];
+  int device = 0;
+  cudaGetDevice(&device);
+  Route& r = recent[(uint32_t(p.M) * 2654435761u ^ uint32_t(p.N) * 2246822519u ^ uint32_t(p.K) * 3266489917u ^ uint32_t(epilogue)) >> 26];
+  if (r.M != p.M || r.N != p.N || r.K != p.K || r.epilogue != epilogue || r.device != device) {
+    r = findRoute(p, sh, epilogue);
+    r.M = p.M; r.N = p.N; r.K = p.K; r.epilogue = epilogue; r.device = device;
+  }
+  return r;
 }
 
 }  // namespace
@@ -1042,8 +1133,11 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   Shape sh{};
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
-  if (bn == 0 && useSkinny(M, N, K, epilogue)) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
-  if (bn == 0 && !switches().singleCta && !switches().oneAcc && useRagged(M, N, K)) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+  if (bn == 0) {
+    const Route& route = gemmRoute(p, sh, epilogue);
+    if (route.kernel == kRouteSkinny) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+    if (route.kernel == kRouteRagged) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, route.cut, status, static_cast<cudaStream_t>(stream));
+  }
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
       !cache.get(maps.c, C, uint64_t(M), uint64_t(epilogue == kEpiSwiglu ? N / 2 : N), 32)) return 1;
@@ -1073,7 +1167,8 @@ int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, in
   GroupedArgs g;
   g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);
   if (timeoutNs) g.timeoutNs = timeoutNs;
-  return (g.likelyRows <= kFewGroupRows ? launchSkinny : launchRagged)(cache, A, B, C, rows, N, K, epilogue, g, status, static_cast<cudaStream_t>(stream));
+  if (g.likelyRows <= kFewGroupRows) return launchSkinny(cache, A, B, C, rows, N, K, epilogue, g, status, static_cast<cudaStream_t>(stream));
+  return launchRagged(cache, A, B, C, rows, N, K, epilogue, g, RaggedPlan{}, status, static_cast<cudaStream_t>(stream));
 }
 
 size_t purlin_tp_workspace_bytes(int world, int M, int kAg, int nRs) { return tpLayout(world, M, kAg, nRs).total; }

@@ -280,3 +280,34 @@ def test_ragged_rows_with_a_k_that_hides_the_epilogue(m, n, k, swiglu):
         assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
     else:
         assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 8192, 4104), (333, 8192, 1096), (384, 7944, 4160), (250, 4096, 4096), (97, 4128, 3080), (512, 4352, 2056), (130, 2304, 5000),
+                                    (300, 1312, 1032), (1030, 14336, 520), (2048, 4096, 512), (2240, 5792, 584), (511, 18944, 648)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_tiles_of_one_accumulator_and_k_shared_by_the_pairs_of_a_cluster(m, n, k, swiglu):
+    # few tiles: 256 rows of W each, with columns in two halves (a multiple of 128) or not, k over one, two or four pairs, an odd last
+    # k-block; many: column tiles of unequal width, a last tile of W without its second half
+    from purlin_b200.ops.gemm import gemm, gemm_swiglu
+    n = (n + 31) // 32 * 32 if swiglu else n
+    a, w = _small_integers(m, n, k, 23)
+    if swiglu:
+        ref = _swiglu_ref(a, w)
+        assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+    else:
+        assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("k", [8, 64, 72, 128, 136, 192, 256, 328])
+@pytest.mark.parametrize("counts", [[257, 0, 300, 31], [513, 1030, 64, 65]])
+def test_grouped_gemm_with_a_k_shorter_than_the_lead_of_an_accumulator(k, counts):
+    from purlin_b200.ops.gemm import grouped_gemm
+    n, rows = 776, sum(counts)
+    a, _ = _small_integers(rows, 8, k, 29)
+    w = torch.stack([_small_integers(8, n, k, 31 + e)[1] for e in range(len(counts))])
+    out = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm(a, w, torch.tensor(counts, dtype=torch.int32, device="cuda"), 400, out)
+    at = 0
+    for e, c in enumerate(counts):
+        assert torch.equal(out[at:at + c].float(), (a[at:at + c].float() @ w[e].float().t()).to(torch.bfloat16).float())
+        at += c

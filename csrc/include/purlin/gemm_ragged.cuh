@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     tc::tmaPrefetchDescriptor(&maps.w);
     tc::tmaPrefetchDescriptor(&maps.x);
   }
+  const int kBlocks = (p.K + kBK - 1) / kBK;
+  const int kbBegin = int(int64_t(kBlocks) * part / parts), kbEnd = int(int64_t(kBlocks) * (part + 1) / parts);   // this pair's k-blocks
   if (warp == 1) { tc::tmemAllocPair(tc::smemAddr(words), kTmemCols); tc::tmemRelinquishPair(); }
   tc::gridDependencyWait();                                    // from here on memory that earlier kernels write may be read
   if (warp == 2) {
@@ -144,7 +146,6 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   // whole tiles; the others count as two items each
   const int fullItems = !SPLIT && p.tileAccs == 2 && 2 * rest <= numPairs ? numTiles - rest : numTiles;
   const int numItems = fullItems + 2 * (numTiles - fullItems);
-  const int kBlocks = (p.K + kBK - 1) / kBK;
 
   // work item -> expert, first row of X, valid columns, columns of the MMA, first row of W inside the expert, accumulators
   struct Item { int expert, row0, cols, count, w0, accs; };
@@ -179,7 +180,6 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     }
     return m;
   };
-  const int kbBegin = int(int64_t(kBlocks) * part / parts), kbEnd = int(int64_t(kBlocks) * (part + 1) / parts);   // this pair's k-blocks
   auto forItems = [&](auto&& body) {
     for (int it = pairIdx; it < numItems; it += numPairs) {
       const Item m = itemOf(it);

@@ -24,7 +24,7 @@ __device__ __forceinline__ float sanitizeLogit(float x) {
 // One warp routes one token. Lane k (k < topk) returns the k-th choice in `expert` / `weight`; other lanes get -1 / 0.
 // VPL = experts / 32 values per lane. Logit: float, or a 16-bit type that converts to it.
 template <int VPL, class Logit>
-__device__ __forceinline__ void routeToken(const Logit* __restrict__ row, int experts, int topk, int normalize, int lane,
+__device__ __forceinline__ void routeToken(const Logit* row, int experts, int topk, int normalize, int lane,
                                            int& expert, float& weight) {
   float v[VPL];
   float mx = -FLT_MAX;

@@ -31,12 +31,14 @@
 #include <cstdio>
 #include <cstdlib>
 #include <string>
+#include <utility>
 
 #include "purlin/atom.cuh"
 #include "purlin/constants.hpp"
 #include "purlin/moe.h"
 #include "purlin/moe_route.cuh"
 #include "purlin/signal.cuh"
+#include "purlin/tc_sm100.cuh"
 #include "purlin/telemetry.hpp"
 
 namespace purlin { void setError(const std::string& e); }
@@ -47,7 +49,7 @@ struct PurlinMoeContext {
   unsigned char* peers[kMaxRanks] = {};
   size_t stageOff = 0, metaOff = 0, recvOff = 0, outOff = 0, cbufOff = 0, countsOff = 0, flagsOff = 0, total = 0;
   void* local = nullptr;
-  size_t sendListOff = 0, posOff = 0, countsLocalOff = 0;
+  size_t sendListOff = 0, posOff = 0, countsLocalOff = 0, sumsOff = 0;
   const int32_t* topkIdx = nullptr;      // routing of the current layer (device pointers the caller owns)
   const float* topkWeight = nullptr;
   const int32_t* slot = nullptr;
@@ -69,7 +71,7 @@ constexpr int kRecvRows = 16;           // rows per receiver item of the dispatc
 constexpr int kMetaWords = 16;          // per staged row: 8 destination rows, 8 gate weights
 
 struct MoeParams {
-  int rank, world, tokens, maxTokens, hiddenBytes, experts, topk, expertsPerRank, capacityRows, maxChunks, senders;
+  int rank, world, tokens, routed, maxTokens, hiddenBytes, experts, topk, expertsPerRank, capacityRows, maxChunks, senders;
   const unsigned char* x;          // [tokens, hidden] bf16
   const int32_t* topkIdx;          // [tokens, topk]
   const float* topkWeight;         // [tokens, topk]
@@ -139,7 +141,8 @@ struct PlanParams {
   int32_t* slot;
   int32_t* pos;
   int32_t* sendList;
-  uint32_t* counts;      // [experts + world], zero before the kernel
+  uint32_t* counts;      // [experts + world]: the result
+  uint32_t* sums;        // [experts + world], the running counters of a launch, and a count of its blocks: zero between launches
   uint32_t* status;
 };
 
@@ -147,9 +150,11 @@ struct PlanParams {
 // k-th expert of the warp's token, -1 for a dropped pair. The pairs are counted in shared memory first and a block takes its
 // share of each global counter with ONE atomic: every token of a rank's own experts used to add to the same word, and 4096
 // additions to one address were most of the plan (4096 tokens, top-8 of 256: route + plan 8.7 + 12.6 us in two launches,
-// 11.9 us now).
+// 11.9 us now). The last block to finish hands the counters on and leaves them cleared for the next launch, where a memset before every
+// launch cost a launch of its own (300 tokens: route 8.2 -> 6.2 us in a graph, 9.0 -> 8.0 us of host time a call).
 PURLIN_D void planBlock(const PlanParams& p, int token, int e) {
   __shared__ uint32_t mine[kMaxExperts + kMaxRanks], first[kMaxExperts + kMaxRanks];
+  __shared__ int lastBlock;
   const int lane = threadIdx.x & 31, words = p.experts + p.world;
   for (int i = threadIdx.x; i < words; i += blockDim.x) mine[i] = 0;
   __syncthreads();
@@ -160,8 +165,16 @@ PURLIN_D void planBlock(const PlanParams& p, int token, int e) {
   if (e >= 0) at = atomicAdd(mine + e, 1u);
   if (e >= 0 && lane == leader) to = atomicAdd(mine + p.experts + dst, 1u);
   __syncthreads();
-  for (int i = threadIdx.x; i < words; i += blockDim.x) if (mine[i]) first[i] = atomicAdd(p.counts + i, mine[i]);
+  const bool alone = gridDim.x == 1;                                    // one block: its counters are the result
+  for (int i = threadIdx.x; i < words; i += blockDim.x) {
+    if (alone) { first[i] = 0; p.counts[i] = mine[i]; }
+    else if (mine[i]) first[i] = atomicAdd(p.sums + i, mine[i]);
+  }
   __syncthreads();
+  if (!alone && threadIdx.x == 0) {
+    __threadfence();
+    lastBlock = atomicAdd(p.sums + words, 1u) == gridDim.x - 1 ? 1 : 0;
+  }
   if (e >= 0) {
     at += first[e];
     if (lane == leader) {
@@ -174,10 +187,19 @@ PURLIN_D void planBlock(const PlanParams& p, int token, int e) {
     p.slot[size_t(token) * p.topk + lane] = e >= 0 ? int32_t(at) : -1;
     p.pos[size_t(token) * p.topk + lane] = e >= 0 ? int32_t(to) : -1;
   }
+  __syncthreads();
+  if (!alone && lastBlock) {
+    __threadfence();
+    for (int i = threadIdx.x; i <= words; i += blockDim.x) {
+      if (i < words) p.counts[i] = __ldcg(p.sums + i);
+      p.sums[i] = 0;
+    }
+  }
 }
 
 template <int VPL, class Logit>   // values per lane = experts / 32
 __global__ void __launch_bounds__(kThreads) routeKernel(const Logit* logits, int normalize, int32_t* topkIdx, float* topkWeight, const PlanParams p) {
+  tc::gridDependencyWait();
   const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   int myE = -1; float myW = 0.f;     // lane k keeps the k-th choice; always a valid expert id (see moe_route.cuh)
   if (token < p.tokens) {
@@ -192,6 +214,7 @@ __global__ void __launch_bounds__(kThreads) routeKernel(const Logit* logits, int
 
 // The plan alone, for routing that the caller brings. An expert id outside [0, experts) is reported and the pair dropped.
 __global__ void __launch_bounds__(kThreads) planKernel(const int32_t* topkIdx, const PlanParams p) {
+  tc::gridDependencyWait();
   const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   int e = -1;
   if (token < p.tokens && lane < p.topk) {
@@ -224,14 +247,17 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
   __shared__ int32_t upTo[kMaxExperts], blockSum[kMaxExperts / 32];
   __shared__ int32_t sendCount[kMaxRanks], recvFrom[kMaxRanks];
   __shared__ int bad, nextItem;
-  const uint64_t epoch = sig::ldRelaxedSys(p.epoch) + 1;
-  stampStart(p, 0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int W = p.world, stride = p.experts + W;
+  if (W == 1) tc::gridDependencyWait();      // (only a world of one is launched early)
+  // what the first steps need is asked for at once: each of them is a round trip of a small call
+  const uint64_t epoch = sig::ldRelaxedSys(p.epoch) + 1, combined = sig::ldRelaxedSys(p.epoch + 1);
+  const uint32_t ownCount = W == 1 && tid < stride ? p.localCounts[tid] : 0u;
+  stampStart(p, 0);
   if (tid == 0) bad = 0;
   __syncthreads();
   // dispatch n may only follow combine n - 1; a call out of order does nothing and is not counted
-  const bool outOfOrder = sig::ldRelaxedSys(p.epoch + 1) + 1 != epoch;
+  const bool outOfOrder = combined + 1 != epoch;
   if (outOfOrder && tid == 0) { bad = 1; reportBad(p, 9, 0); }
 
   // 1. publish this rank's counts on every rank (flagged stores; the flag is released after the data)
@@ -252,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
   for (int e0 = warp * 32; ok && e0 < p.experts; e0 += kWarps * 32) {
     const int e = e0 + lane;
     int tot = 0, before = 0;
-    for (int s = 0; s < W; ++s) { const int c = int(all[size_t(s) * stride + e]); tot += c; if (s < p.rank) before += c; }
+    for (int s = 0; s < W; ++s) { const int c = int(W == 1 && e == tid ? ownCount : all[size_t(s) * stride + e]); tot += c; if (s < p.rank) before += c; }
     int sum = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
@@ -367,13 +393,15 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
       {
         const int receivers = int(gridDim.x) - senders, me = int(blockIdx.x) - senders;
         const int perRow = (vecs + 31) / 32;
-        const int64_t pieces = int64_t(sendCount[p.rank]) * perRow, nw = int64_t(receivers) * kWarps, w = int64_t(warp) * receivers + me;
+        // In a world of one the list is the tokens themselves and a token's record lies at its own place, which saves a round trip
+        // here and two in the combine.
+        const int64_t pieces = int64_t(W == 1 ? p.routed : sendCount[p.rank]) * perRow, nw = int64_t(receivers) * kWarps, w = int64_t(warp) * receivers + me;
         int64_t u = pieces * w / nw;
         const int64_t stop = pieces * (w + 1) / nw;
         while (u < stop) {
           const int pp = int(u / perRow), first = int(u % perRow);
           const int n = int(min(int64_t(perRow - first), stop - u));
-          const int t = p.sendList[size_t(p.rank) * p.maxTokens + pp];
+          const int t = W == 1 ? pp : p.sendList[size_t(p.rank) * p.maxTokens + pp];
           int row;
           const int rec = recordOf(t, p.rank, row);
           // the combine reads the record like a peer's
@@ -475,18 +503,20 @@ template <int ALONE>
 __global__ void __launch_bounds__(kThreads, ALONE ? kCombineCtasPerSmAlone : kCombineCtasPerSm) combineKernel(const __grid_constant__ MoeParams p) {
   __shared__ int32_t recvFrom[kMaxRanks];
   __shared__ int bad, nextItem;
-  const uint64_t epoch = sig::ldRelaxedSys(p.epoch + 1) + 1;
-  stampStart(p, 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int W = p.world, stride = p.experts + W;
+  if (ALONE) tc::gridDependencyWait();       // (only a world of one is launched early)
+  const uint64_t epoch = sig::ldRelaxedSys(p.epoch + 1) + 1, dispatched = sig::ldRelaxedSys(p.epoch);
+  const uint32_t status = sig::ldRelaxedGpu32(p.status);
+  stampStart(p, 4);
   if (tid == 0) bad = 0;
   __syncthreads();
   // combine n follows dispatch n; a call out of order does nothing and is not counted
-  const bool outOfOrder = sig::ldRelaxedSys(p.epoch) != epoch;
+  const bool outOfOrder = dispatched != epoch;
   if (outOfOrder && tid == 0) { bad = 1; reportBad(p, 10, 0); }
   if (!ALONE && tid < W) recvFrom[tid] = int(p.countsAll[p.rank][size_t(tid) * stride + p.experts + p.rank]);
   __syncthreads();
-  const bool ok = __syncthreads_and(!bad && sig::ldRelaxedGpu32(p.status) == 0u) != 0;   // one answer for the whole CTA: the roles below hold barriers
+  const bool ok = __syncthreads_and(!bad && status == 0u) != 0;   // one answer for the whole CTA: the roles below hold barriers
   const int vecs32 = p.hiddenBytes / 32;
   const size_t rowBytes = size_t(p.hiddenBytes);
   const int senders = ALONE ? 0 : (p.senders < int(gridDim.x) ? p.senders : int(gridDim.x) - 1);
@@ -540,7 +570,11 @@ __global__ void __launch_bounds__(kThreads, ALONE ? kCombineCtasPerSmAlone : kCo
     auto finish = [&](int t, int begin, int end) {     // 32-byte pieces [begin, end) of token t
       int d = -1 - lane, pos = -1, ownRow = -1;
       float weight = 1.f;
-      if (lane < p.topk) {
+      if (ALONE) {                                     // the record lies at the token's own place
+        const int rec = lane < kMetaWords ? p.meta[0][size_t(t) * kMetaWords + lane] : -1;
+        weight = __int_as_float(__shfl_sync(0xffffffffu, rec, 8 + (lane & 7)));
+        if (lane < p.topk) ownRow = rec;
+      } else if (lane < p.topk) {
         const int e = p.topkIdx[size_t(t) * p.topk + lane];
         pos = p.pos[size_t(t) * p.topk + lane];
         if (e >= 0 && e < p.experts && pos >= 0) d = e / p.expertsPerRank;
@@ -649,7 +683,7 @@ void fillCommon(MoeParams& p, PurlinMoeContext* c, int tokens) {
   p.timeoutNs = c->timeoutNs;
 }
 
-// Clears the counters and adopts the routing arrays: every route or plan begins with it.
+// Adopts the routing arrays: every route or plan begins with it.
 bool beginPlan(PurlinMoeContext* c, const int32_t* topkIdx, const float* topkWeight, int tokens, int32_t* slot, cudaStream_t s, PlanParams& p) {
   unsigned char* lb = static_cast<unsigned char*>(c->local);
   p.tokens = tokens; p.maxTokens = c->maxTokens; p.experts = c->experts; p.topk = c->topk; p.expertsPerRank = c->experts / c->world; p.world = c->world;
@@ -657,10 +691,26 @@ bool beginPlan(PurlinMoeContext* c, const int32_t* topkIdx, const float* topkWei
   p.pos = reinterpret_cast<int32_t*>(lb + c->posOff);
   p.sendList = reinterpret_cast<int32_t*>(lb + c->sendListOff);
   p.counts = reinterpret_cast<uint32_t*>(lb + c->countsLocalOff);
+  p.sums = reinterpret_cast<uint32_t*>(lb + c->sumsOff);
   p.status = reinterpret_cast<uint32_t*>(lb + 256);
-  if (cudaMemsetAsync(p.counts, 0, size_t(c->experts + c->world) * 4, s) != cudaSuccess) { setError("route: clearing the counters failed"); return false; }
+  // (an empty layer has no kernel that would write the counts)
+  if (tokens == 0 && cudaMemsetAsync(p.counts, 0, size_t(c->experts + c->world) * 4, s) != cudaSuccess) { setError("route: clearing the counters failed"); return false; }
   c->topkIdx = topkIdx; c->topkWeight = topkWeight; c->slot = slot; c->routed = tokens;
   return true;
+}
+
+// A launch that may be set up while the kernel before it on the stream drains: the kernel waits for it by itself. None of these kernels lets
+// its successor start before it ends: CTAs that wait early took places from the ones at work (route, dispatch and combine of 300 x 1024,
+// top-8 of 64, in a graph: 24.7 us without overlap, 21.0 like this, 27.1 with an early start).
+template <class... Params, class... Args>
+int launchEarly(const char* what, void (*kernel)(Params...), int blocks, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(unsigned(blocks)); cfg.blockDim = dim3(kThreads); cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (e != cudaSuccess) { setError(std::string(what) + " launch: " + cudaGetErrorString(e)); return 1; }
+  return 0;
 }
 
 template <class Logit>
@@ -672,15 +722,8 @@ int routeOn(PurlinMoeContext* c, const Logit* logits, int tokens, int normalize,
   if (!beginPlan(c, topkIdx, topkWeight, tokens, slot, s, p)) return 1;
   if (tokens == 0) return 0;             // an empty layer all the same: the counters of the layer before are gone
   const int blocks = (tokens * 32 + kThreads - 1) / kThreads;
-  switch (vpl) {
-    case 1: routeKernel<1><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
-    case 2: routeKernel<2><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
-    case 4: routeKernel<4><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
-    case 8: routeKernel<8><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
-    default: routeKernel<16><<<blocks, kThreads, 0, s>>>(logits, normalize, topkIdx, topkWeight, p); break;
-  }
-  if (cudaGetLastError() != cudaSuccess) { setError("route launch failed"); return 1; }
-  return 0;
+  auto kernel = vpl == 1 ? routeKernel<1, Logit> : vpl == 2 ? routeKernel<2, Logit> : vpl == 4 ? routeKernel<4, Logit> : vpl == 8 ? routeKernel<8, Logit> : routeKernel<16, Logit>;
+  return launchEarly("route", kernel, blocks, s, logits, normalize, topkIdx, topkWeight, p);
 }
 
 }  // namespace
@@ -709,7 +752,8 @@ PurlinMoeContext* purlin_moe_create(int rank, int world, const uint64_t* peerPtr
   c->timeoutNs = timeoutNs ? timeoutNs : 10ull * 1000 * 1000 * 1000;
   // local block: [0] epochs, [64] exit counters, [256] status, then counters, send lists, positions
   c->countsLocalOff = 1024;
-  c->sendListOff = roundUp(c->countsLocalOff + size_t(kMaxExperts + kMaxRanks) * 4, 1024);
+  c->sumsOff = roundUp(c->countsLocalOff + size_t(kMaxExperts + kMaxRanks) * 4, 1024);
+  c->sendListOff = roundUp(c->sumsOff + size_t(kMaxExperts + kMaxRanks + 1) * 4, 1024);
   c->posOff = c->sendListOff + roundUp(size_t(world) * maxTokens * 4, 1024);
   const size_t localBytes = c->posOff + roundUp(size_t(maxTokens) * topk * 4, 1024);
   if (cudaMalloc(&c->local, localBytes) != cudaSuccess) { delete c; setError("cudaMalloc failed"); return nullptr; }
@@ -783,8 +827,7 @@ int purlin_moe_plan(PurlinMoeContext* c, const int32_t* topkIdx, const float* to
   PlanParams p;
   if (!beginPlan(c, topkIdx, topkWeight, tokens, slot, s, p)) return 1;
   const int blocks = (tokens * 32 + kThreads - 1) / kThreads;
-  if (blocks > 0) planKernel<<<blocks, kThreads, 0, s>>>(topkIdx, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+  return blocks > 0 ? launchEarly("plan", planKernel, blocks, s, topkIdx, p) : 0;
 }
 
 int purlin_moe_dispatch(PurlinMoeContext* c, const void* x, int tokens, const int32_t* topkIdx, const int32_t* slot,
@@ -796,11 +839,12 @@ int purlin_moe_dispatch(PurlinMoeContext* c, const void* x, int tokens, const in
   c->dispatched = c->routed;
   MoeParams p{};
   fillCommon(p, c, tokens);
-  p.x = static_cast<const unsigned char*>(x); p.sentRow = sentRow; p.recvCounts = recvCounts;
+  p.x = static_cast<const unsigned char*>(x); p.sentRow = sentRow; p.recvCounts = recvCounts; p.routed = c->routed;
   const int grid = smCount() * kDispatchCtasPerSm;
   // remote stores fill the links with far fewer CTAs (about 32 GB/s each) than the local fan-out needs for HBM; the
   // receivers end last (4 GPUs, 296 CTAs: 32 senders 352 us, 48 senders 357 - 372 us, 64 senders 363 us)
   p.senders = blocks > 0 ? std::min(blocks, grid - 1) : std::max(std::min(grid / 3, 32), 1);
+  if (c->world == 1) return launchEarly("dispatch", dispatchKernel, grid, static_cast<cudaStream_t>(stream), p);
   dispatchKernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { setError(std::string("dispatch launch: ") + cudaGetErrorString(e)); return 1; }
@@ -822,8 +866,9 @@ int purlin_moe_combine(PurlinMoeContext* c, void* y, int tokens, const int32_t* 
   // 343 us; 98 pushers 366 us, 110 pushers 392 us): the finishers end last. The pushers now have (W - 1) / W of that work and
   // the finishers the rest, so their number shrinks with it (bytes per CTA as measured; not timed again on several GPUs).
   p.senders = blocks > 0 ? std::min(blocks, grid - 1) : std::max(grid * 54 * (c->world - 1) / (100 * c->world), 1);
-  auto kernel = c->world > 1 ? combineKernel<0> : c->topk <= 2 ? combineKernel<2> : c->topk <= 4 ? combineKernel<4> : combineKernel<8>;
-  kernel<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  if (c->world == 1)
+    return launchEarly("combine", c->topk <= 2 ? combineKernel<2> : c->topk <= 4 ? combineKernel<4> : combineKernel<8>, grid, static_cast<cudaStream_t>(stream), p);
+  combineKernel<0><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { setError(std::string("combine launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;

@@ -34,8 +34,10 @@ struct alignas(64) Maps { CUtensorMap w, x; };
 struct Params {
   int N, K, tokens;        // N: rows of W per expert; tokens: rows of X (with counts: an upper bound of their sum); exchanged with kTokenRows
   int passTokens;          // columns of one pass: multiple of tokenBox
+  int columnGroups;        // without counts: this many CTAs share a tile's columns, a pass each (blockIdx.y)
   int tokenBox;            // rows of one X load: 16 or 32
   int stages, tmemCols;
+  int ahead;               // k-blocks of W that are asked into L2 while the kernel before this one drains (0 where it has ended)
   const int32_t* counts;   // rows per expert, or null: one group of `tokens` rows
   __nv_bfloat16* C;
   int ldc;
@@ -122,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
   uint32_t split;
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(split));
   const uint32_t part = tc::clusterCtaRank();
-  const int tile = int(blockIdx.x / split), expert = int(blockIdx.y);
+  const int tile = int(blockIdx.x / split), expert = p.counts ? int(blockIdx.y) : 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
@@ -139,12 +141,16 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
   // W may be what that kernel writes). 1 x 8192 x 3584 MLP block 36.0 -> 34.1 us, 32 x 8192 x 8192 74.0 -> 71.8; half a lap gains less,
   // two or the whole range take bandwidth from the kernel that still runs (35.7, 39.1 us).
   if (warp == 0 && lane == 0)
-    for (int kb = kBegin; kb < min(kEnd, kBegin + p.stages); ++kb) tc::tmaPrefetchL2(&maps.w, kb * kK, expert * p.N + tile * kRows);
+    for (int kb = kBegin; kb < min(kEnd, kBegin + p.ahead); ++kb) tc::tmaPrefetchL2(&maps.w, kb * kK, expert * p.N + tile * kRows);
   if (warp == 1) { tc::tmemAlloc(tc::smemAddr(words), uint32_t(p.tmemCols)); tc::tmemRelinquish(); }
   tc::gridDependencyWait();                                   // from here on memory that earlier kernels write may be read
   if (warp == 2) {
     const uint32_t limit = uint32_t(p.tokens);
     uint32_t first = 0, rows = limit;
+    if (p.columnGroups > 1) {
+      first = min(blockIdx.y * uint32_t(p.passTokens), limit);
+      rows = min(uint32_t(p.passTokens), limit - first);
+    }
     if (p.counts) {
       for (int e = lane; e < expert; e += 32) first = addRows(first, groupRowsOf(p.counts[e], limit), limit);
 #pragma unroll
@@ -240,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinnyGemmKernel(const __grid_con
         if (row >= p.N) continue;
         float v[8];
         sumPartialColumns(peer, int(split), uint32_t(piece * 8 * kRows + r) * 4u, v);
-        st16(p.C + size_t(row) * p.ldc + t0 + piece * 8, Vec16{{pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7])}});
+        st16(p.C + size_t(row) * p.ldc + firstRow + t0 + piece * 8, Vec16{{pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7])}});
       }
     } else if (*abortWord == 0) {
       constexpr bool SWIGLU = MODE == kWeightRowsSwiglu;

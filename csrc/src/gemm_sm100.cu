@@ -867,6 +867,16 @@ int skinnySplit(long tiles, int kBlocks, long slots) {
   return split;
 }
 
+// CTAs that share the columns of a tile, where its k parts leave SMs without one: a k-block takes 450 cycles and 3.5 per column, and the
+// few rows of W that they all read come from L2 (fifteen clusters of eight fit on the GPU). In a graph, us, one CTA for all columns /
+// shared: 128 x 32 x 7168 9.8 / 7.5, 128 x 256 x 4096 10.9 / 7.1, 200 x 512 x 7168 17.4 / 12.0, 300 x 256 x 7168 16.5 / 9.6, 128 x 2048 x 4096
+// 13.8 / 11.4, 50 x 600 x 1000 6.7 / 5.4. More than half the SMs only for parts of six k-blocks: 40 x 2048 x 1024 5.7 / 6.3.
+int skinnyGroups(int columns, long tiles, int split, int kBlocks) {
+  const long ctas = std::max(tiles * split, 1l), places = kBlocks >= 6 * split ? smCount() : smCount() / 2;
+  const long room = split == skinny::kMaxSplit ? 15 / std::max(tiles, 1l) : places / ctas;
+  return int(std::max(std::min(long(columns + 31) / 32, room), 1l));
+}
+
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
 int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
@@ -882,15 +892,19 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   const int room = std::min(g.counts ? 2 * g.likelyRows + 16 : M, M);
   p.tokenBox = room <= 16 ? 16 : 32;
   p.passTokens = std::min(int(roundUp(size_t(room), size_t(p.tokenBox))), skinny::kMaxTokens);
+  const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
+  const int split = skinnySplit(long(tiles) * g.experts, kBlocks, long(smCount()) * (p.passTokens <= 128 ? 2 : 1));
+  p.columnGroups = 1;
+  if (!g.counts && M <= p.passTokens) {
+    p.columnGroups = skinnyGroups(M, tiles, split, kBlocks);
+    p.passTokens = int(roundUp(size_t(M + p.columnGroups - 1) / p.columnGroups, size_t(p.tokenBox)));
+  }
   // up to 128 columns two CTAs share an SM (128 columns: 3 stages of 32 KiB each)
   const int stageBytes = skinny::kWBytes + p.passTokens * skinny::kK * 2;
   const int perSm = p.passTokens <= 128 ? 2 : 1;
   const int budget = (perSm == 2 ? 113 : 227) * 1024 - 1024 - skinny::kBarrierBytes;
   p.stages = std::min(budget / stageBytes, skinny::kMaxStages);
   for (p.tmemCols = 32; p.tmemCols < p.passTokens; p.tmemCols *= 2) {}
-  const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
-  const long slots = long(smCount()) * perSm;
-  const int split = skinnySplit(long(tiles) * g.experts, kBlocks, slots);
   skinny::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
   const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;
@@ -910,12 +924,15 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   cudaLaunchAttribute attr[2];
   attr[1] = overlapAttribute();
   attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(split); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(unsigned(tiles * split), unsigned(g.experts)); cfg.blockDim = dim3(skinny::kThreads);
+  cfg.gridDim = dim3(unsigned(tiles * split), unsigned(g.experts * p.columnGroups)); cfg.blockDim = dim3(skinny::kThreads);
   cfg.dynamicSmemBytes = size_t(p.stages) * stageBytes + skinny::kBarrierBytes + 1024; cfg.stream = stream;
   // Between half as many CTAs as SMs and as many, they are better placed on an empty GPU, one to an SM: set up early they pile
   // up two to an SM where the kernel before left room (97-token MLP block 5824 x 1888, 120 CTAs: 40.7 us apart, 42.5 overlapped).
-  const long ctas = long(tiles) * split * g.experts;
-  cfg.attrs = attr; cfg.numAttrs = ctas * 2 > smCount() && ctas < smCount() ? 1 : 2;
+  const long ctas = long(tiles) * split * g.experts * p.columnGroups;
+  // With shared columns the tiles are small and the launch is the larger part: 200 x 2048 x 4096 15.1 us apart, 13.7 overlapped.
+  const bool apart = ctas * 2 > smCount() && ctas < smCount() && p.columnGroups == 1;
+  p.ahead = apart ? 0 : p.stages;
+  cfg.attrs = attr; cfg.numAttrs = apart ? 1 : 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
@@ -1058,7 +1075,7 @@ double skinnyCycles(int M, int N, int K, int epilogue) {
   if (M > skinny::kMaxTokens || N > 16384) return 1e30;
   const long tiles = (N + skinny::kRows - 1) / skinny::kRows, slots = long(smCount()) * (M <= 128 ? 2 : 1);
   const int kBlocks = (K + skinny::kK - 1) / skinny::kK, split = skinnySplit(tiles, kBlocks, slots);
-  const double waves = std::ceil(double(tiles * split) / slots), block = (450. + 3.5 * M) * (tiles * split > smCount() ? 1.3 : 1.);
+  const double waves = std::ceil(double(tiles * split) / slots), block = (450. + 3.5 * M / skinnyGroups(M, tiles, split, kBlocks)) * (tiles * split > smCount() ? 1.3 : 1.);
   return std::max(waves * kBlocks / split * block, 1.15 * (2. * N * K + 2. * M * K) / 3300.) + 7000. + (epilogue == kEpiSwiglu ? 105. : 45.) * M;
 }
 

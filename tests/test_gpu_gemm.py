@@ -298,6 +298,21 @@ def test_tiles_of_one_accumulator_and_k_shared_by_the_pairs_of_a_cluster(m, n, k
         assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 8, 520), (128, 32, 7168), (97, 136, 4104), (200, 504, 7176), (129, 2080, 4096), (300, 256, 7168), (257, 200, 2056), (50, 600, 1000),
+                                    (255, 1024, 3080)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_few_rows_with_the_columns_of_a_tile_shared(m, n, k, swiglu):
+    # few tiles: several CTAs take 32 to 64 columns each of the same weight rows (or, with few weight rows, of the same tokens); odd last groups
+    from purlin_b200.ops.gemm import gemm, gemm_swiglu
+    n = (n + 31) // 32 * 32 if swiglu else n
+    a, w = _small_integers(m, n, k, 37)
+    if swiglu:
+        ref = _swiglu_ref(a, w)
+        assert ((gemm_swiglu(a, w).float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+    else:
+        assert torch.equal(gemm(a, w).float(), (a.float() @ w.float().t()).to(torch.bfloat16).float())
+
+
 @pytest.mark.parametrize("k", [8, 64, 72, 128, 136, 192, 256, 328])
 @pytest.mark.parametrize("counts", [[257, 0, 300, 31], [513, 1030, 64, 65]])
 def test_grouped_gemm_with_a_k_shorter_than_the_lead_of_an_accumulator(k, counts):

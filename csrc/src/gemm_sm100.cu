@@ -988,37 +988,46 @@ int raggedClusters(int epilogue, int parts) {
 //   the weights come through HBM once.
 // What it buys, us, one B200, before / now: 2048 x 14336 x 8192 SwiGLU 371 / 325 (ten column tiles, where eight left a fourth wave of two
 // tiles), 1000 x 14336 x 8192 SwiGLU 205 / 168, 1000 x 8192 x 7168 97 / 85, 384 x 14336 x 8192 SwiGLU 121 / 78, 700 x 8192 x 28672 428 / 250;
-// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58. Over 900 random
-// shapes the geometric mean is 1.08; 18 are slower by more than 3 %, the worst by 14 % (4871 x 368 x 1456 15.6 / 18.6).
+// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58. Over 750 random
+// shapes the geometric mean is 1.09; 22 are slower by more than 3 %, the worst by 18 % (2006 x 64 x 1320 11.6 / 14.2).
 struct RaggedPlan { int tileAccs = 2, colTiles = 1, tiles = 1, parts = 1; double cycles = 0; };
 RaggedPlan raggedPlan(int M, int N, int K, int epilogue, const int (&clusters)[3]) {
   const int kBlocks = (K + kBK - 1) / kBK, units = (M + 31) / 32, fewest = (units + 7) / 8;
   const double unaligned = K % kBK ? 1.12 : 1.;                 // rows of K that do not begin on a cache line
+  auto cyclesOf = [&](int accs, double cols, int64_t tiles, int parts) {
+    auto perBlock = [&](int a) {
+      if (a == 1) return (500 + 2.1 * cols) * unaligned;
+      return std::max(4 * cols, (2 * ragged::kABytes + cols * 64) / 44 * unaligned);
+    };
+    auto drain = [&](int a) { return 1200. + a * cols * (epilogue == kEpiSwiglu ? 8. : 3.); };
+    const int places = clusters[parts / 2];
+    const int64_t full = tiles / places, rest = tiles % places;
+    const double whole = (kBlocks + parts - 1) / parts * perBlock(accs) + drain(accs) + (parts > 1 ? 3500. * parts + accs * cols * 512. * (parts - 1) / parts / 12 : 0.);
+    const double tail = rest == 0 ? 0. : parts == 1 && accs == 2 && 2 * rest <= places ? kBlocks * perBlock(1) + drain(1) : whole;
+    // the weights once through HBM, at least
+    return std::max(double(full) * whole + tail, (2. * N * K + 2. * M * K) / 3300. * unaligned) + 4500. + accs * cols * 8.;
+  };
   RaggedPlan best;
+  double bestKey = 0;
   for (int accs = 1; accs <= 2; ++accs) {
-    // the fewest column tiles, one and two more, and the numbers that just fill one to three waves more than the fewest need
+    // the fewest column tiles, one and two more, tiles of at most 7 to 4 units (of 32 rows), and the numbers that just fill one to three
+    // waves more than the fewest need
     const int64_t wTiles = (N + accs * ragged::kAccRows - 1) / (accs * ragged::kAccRows), waves = fewest * wTiles / clusters[0];
-    for (int c = 0; c < 6; ++c) {
-      const int64_t want = c < 3 ? fewest + c : (waves + c - 2) * clusters[0] / wTiles;
+    for (int c = 0; c < 10; ++c) {
+      const int64_t want = c < 3 ? fewest + c : c < 7 ? (units + 9 - c) / (10 - c) : (waves + c - 6) * clusters[0] / wTiles;
       if (want < fewest || want > units || want > 2 * fewest + 2) continue;
       const int n = int(want);
       const int64_t tiles = n * wTiles;
-      const double cols = 32. * units / n;                       // of a tile, on average
-      auto perBlock = [&](int a) {
-        if (a == 1) return (500 + 2.1 * cols) * unaligned;
-        return std::max(4 * cols, (2 * ragged::kABytes + cols * 64) / 44 * unaligned);
-      };
-      auto drain = [&](int a) { return 1200. + a * cols * (epilogue == kEpiSwiglu ? 8. : 3.); };
+      const double average = 32. * units / n, widest = (units + n - 1) / n * 32;
       for (int parts = 1; parts <= kMaxParts; parts *= 2) {
-        const int places = clusters[parts / 2];
-        if (!places || kBlocks < 8 * parts) break;
-        if (parts > 1 && tiles > places) break;
-        const int64_t full = tiles / places, rest = tiles % places;
-        const double whole = (kBlocks + parts - 1) / parts * perBlock(accs) + drain(accs) + (parts > 1 ? 3500. * parts + accs * cols * 512. * (parts - 1) / parts / 12 : 0.);
-        const double tail = rest == 0 ? 0. : parts == 1 && accs == 2 && 2 * rest <= places ? kBlocks * perBlock(1) + drain(1) : whole;
-        // the weights once through HBM, at least
-        const double cycles = std::max(double(full) * whole + tail, (2. * N * K + 2. * M * K) / 3300. * unaligned) + 4500. + accs * cols * 8.;
-        if (best.cycles == 0 || cycles < best.cycles) best = RaggedPlan{accs, n, int(std::min<int64_t>(tiles, INT32_MAX / 4)), parts, cycles};
+        if (!clusters[parts / 2] || kBlocks < 8 * parts || (parts > 1 && tiles > clusters[parts / 2])) break;
+        // Among cuts: a pair with few tiles has the widest among them, and narrow tiles move more bytes per operation, which costs power
+        // (2072 x 4800 x 5016 SwiGLU: 11 tiles of 192 88.7 us, 14 of 128 and 160 97.2).
+        const double key = cyclesOf(accs, average + (widest - average) * clusters[0] / std::max<int64_t>(tiles, clusters[0]), tiles, parts) * (0.95 + 12.8 / average);
+        if (bestKey == 0 || key < bestKey) {
+          bestKey = key;
+          best = RaggedPlan{accs, n, int(std::min<int64_t>(tiles, INT32_MAX / 4)), parts, cyclesOf(accs, average, tiles, parts)};
+        }
       }
     }
   }

@@ -18,6 +18,8 @@
 // at most in any case. Arithmetic is packed f32x2; the number of accesses in flight per
 // thread is a knob chosen by the tuning policy.
 #pragma once
+#include <type_traits>
+
 #include "math.cuh"
 #include "signal.cuh"
 
@@ -166,29 +168,34 @@ struct AtomSm100 {
     const int tid = threadIdx.x, nt = blockDim.x;
     const size_t n = a.bytes / 16;
     if (a.world <= WB) {
-      for (size_t i0 = tid; i0 < n; i0 += size_t(U) * nt) {
+      // the loads of a whole step carry no conditions where the world is WB, so they leave together
+      auto sum = [&](size_t i0, auto whole) {
         Vec16 v[U][WB];
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
           for (int b = 0; b < WB; ++b)
-            if (b < a.world && i0 + size_t(u) * nt < n) v[u][b] = ld16(a.srcs[b] + (i0 + size_t(u) * nt) * 16);
+            if (whole || (b < a.world && i0 + size_t(u) * nt < n)) v[u][b] = ld16(a.srcs[b] + (i0 + size_t(u) * nt) * 16);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          if (i0 + size_t(u) * nt >= n) break;
+          if (!whole && i0 + size_t(u) * nt >= n) break;
           Acc<T> lo, hi;
 #pragma unroll
           for (int e = 0; e < ElemTraits<T>::perWord; ++e) lo.v[e] = hi.v[e] = identity<Op>();
 #pragma unroll
           for (int b = 0; b < WB; ++b)
-            if (b < a.world) {
+            if (whole || b < a.world) {
               accumulate<T, Op>(lo, unpack<T>(uint64_t(v[u][b].x[0]) | (uint64_t(v[u][b].x[1]) << 32)));
               accumulate<T, Op>(hi, unpack<T>(uint64_t(v[u][b].x[2]) | (uint64_t(v[u][b].x[3]) << 32)));
             }
           const uint64_t w0 = pack<T>(lo), w1 = pack<T>(hi);
           emit(a, (i0 + size_t(u) * nt) * 16, Vec16{{uint32_t(w0), uint32_t(w0 >> 32), uint32_t(w1), uint32_t(w1 >> 32)}});
         }
-      }
+      };
+      size_t i0 = tid;
+      if (a.world == WB)
+        for (; i0 + size_t(U - 1) * nt < n; i0 += size_t(U) * nt) sum(i0, std::true_type{});
+      for (; i0 < n; i0 += size_t(U) * nt) sum(i0, std::false_type{});
       return;
     }
     for (size_t i = tid; i < n; i += nt) {

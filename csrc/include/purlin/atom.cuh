@@ -169,7 +169,8 @@ struct AtomSm100 {
     const size_t n = a.bytes / 16;
     if (a.world <= WB) {
       // the loads of a whole step carry no conditions where the world is WB, so they leave together
-      auto sum = [&](size_t i0, auto whole) {
+      auto sum = [&](size_t i0, auto allRanks) {
+        constexpr bool whole = decltype(allRanks)::value;
         Vec16 v[U][WB];
 #pragma unroll
         for (int u = 0; u < U; ++u)

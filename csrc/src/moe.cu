@@ -71,14 +71,14 @@ constexpr int kRecvRows = 16;           // rows per receiver item of the dispatc
 constexpr int kMetaWords = 16;          // per staged row: 8 destination rows, 8 gate weights
 
 struct MoeParams {
-  int rank, world, tokens, routed, maxTokens, hiddenBytes, experts, topk, expertsPerRank, capacityRows, maxChunks, senders;
+  int rank, world, tokens, maxTokens, hiddenBytes, experts, topk, expertsPerRank, capacityRows, maxChunks, senders;
   const unsigned char* x;          // [tokens, hidden] bf16
   const int32_t* topkIdx;          // [tokens, topk]
   const float* topkWeight;         // [tokens, topk]
   const int32_t* slot;             // [tokens, topk] position of the row among this rank's rows of that expert
   const int32_t* pos;              // [tokens, topk] position of the token in the send list of that expert's GPU
   const int32_t* sendList;         // [world][maxTokens] token ids in position order
-  const uint32_t* localCounts;     // [experts + world] rows per expert, then distinct tokens per destination rank
+  const uint32_t* localCounts;     // [experts + world + 1] rows per expert, then distinct tokens per destination rank, then the tokens routed
   int32_t* sentRow;                // optional output [tokens, topk]: row inside the destination's expert-major buffer
   int32_t* recvCounts;             // [expertsPerRank + 1] rows received per local expert, then their total
   unsigned char* stage[kMaxRanks];     // every rank's staging area [world sources][maxTokens][hidden]
@@ -141,7 +141,7 @@ struct PlanParams {
   int32_t* slot;
   int32_t* pos;
   int32_t* sendList;
-  uint32_t* counts;      // [experts + world]: the result
+  uint32_t* counts;      // [experts + world + 1]: the result, and the number of tokens that it was made from
   uint32_t* sums;        // [experts + world], the running counters of a launch, and a count of its blocks: zero between launches
   uint32_t* status;
 };
@@ -170,6 +170,7 @@ PURLIN_D void planBlock(const PlanParams& p, int token, int e) {
     if (alone) { first[i] = 0; p.counts[i] = mine[i]; }
     else if (mine[i]) first[i] = atomicAdd(p.sums + i, mine[i]);
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.counts[words] = uint32_t(p.tokens);
   __syncthreads();
   if (!alone && threadIdx.x == 0) {
     __threadfence();
@@ -287,7 +288,9 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
     upTo[e] = sum;                                  // inclusive, inside the block of 32
     if (lane == 31) blockSum[e0 / 32] = sum;
   }
-  if (ok && tid < W) { sendCount[tid] = int(p.localCounts[p.experts + tid]); recvFrom[tid] = int(all[size_t(tid) * stride + p.experts + p.rank]); }
+  // A world of one walks its tokens (below). How many were routed is the plan's word, not the host's at the time of the launch: a captured
+  // dispatch may be replayed after another plan. (x has p.tokens rows.)
+  if (ok && tid < W) { sendCount[tid] = int(W == 1 ? min(p.localCounts[stride], uint32_t(p.tokens)) : p.localCounts[p.experts + tid]); recvFrom[tid] = int(all[size_t(tid) * stride + p.experts + p.rank]); }
   __syncthreads();
   auto rowsBefore = [&](int e) {                    // rows of all experts below e
     int v = upTo[e] - colTotal[e];
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtasPerSm) dispatchKernel(c
         const int perRow = (vecs + 31) / 32;
         // In a world of one the list is the tokens themselves and a token's record lies at its own place, which saves a round trip
         // here and two in the combine.
-        const int64_t pieces = int64_t(W == 1 ? p.routed : sendCount[p.rank]) * perRow, nw = int64_t(receivers) * kWarps, w = int64_t(warp) * receivers + me;
+        const int64_t pieces = int64_t(sendCount[p.rank]) * perRow, nw = int64_t(receivers) * kWarps, w = int64_t(warp) * receivers + me;
         int64_t u = pieces * w / nw;
         const int64_t stop = pieces * (w + 1) / nw;
         while (u < stop) {
@@ -694,7 +697,7 @@ bool beginPlan(PurlinMoeContext* c, const int32_t* topkIdx, const float* topkWei
   p.sums = reinterpret_cast<uint32_t*>(lb + c->sumsOff);
   p.status = reinterpret_cast<uint32_t*>(lb + 256);
   // (an empty layer has no kernel that would write the counts)
-  if (tokens == 0 && cudaMemsetAsync(p.counts, 0, size_t(c->experts + c->world) * 4, s) != cudaSuccess) { setError("route: clearing the counters failed"); return false; }
+  if (tokens == 0 && cudaMemsetAsync(p.counts, 0, size_t(c->experts + c->world + 1) * 4, s) != cudaSuccess) { setError("route: clearing the counters failed"); return false; }
   c->topkIdx = topkIdx; c->topkWeight = topkWeight; c->slot = slot; c->routed = tokens;
   return true;
 }
@@ -752,7 +755,7 @@ PurlinMoeContext* purlin_moe_create(int rank, int world, const uint64_t* peerPtr
   c->timeoutNs = timeoutNs ? timeoutNs : 10ull * 1000 * 1000 * 1000;
   // local block: [0] epochs, [64] exit counters, [256] status, then counters, send lists, positions
   c->countsLocalOff = 1024;
-  c->sumsOff = roundUp(c->countsLocalOff + size_t(kMaxExperts + kMaxRanks) * 4, 1024);
+  c->sumsOff = roundUp(c->countsLocalOff + size_t(kMaxExperts + kMaxRanks + 1) * 4, 1024);
   c->sendListOff = roundUp(c->sumsOff + size_t(kMaxExperts + kMaxRanks + 1) * 4, 1024);
   c->posOff = c->sendListOff + roundUp(size_t(world) * maxTokens * 4, 1024);
   const size_t localBytes = c->posOff + roundUp(size_t(maxTokens) * topk * 4, 1024);
@@ -839,7 +842,7 @@ int purlin_moe_dispatch(PurlinMoeContext* c, const void* x, int tokens, const in
   c->dispatched = c->routed;
   MoeParams p{};
   fillCommon(p, c, tokens);
-  p.x = static_cast<const unsigned char*>(x); p.sentRow = sentRow; p.recvCounts = recvCounts; p.routed = c->routed;
+  p.x = static_cast<const unsigned char*>(x); p.sentRow = sentRow; p.recvCounts = recvCounts;
   const int grid = smCount() * kDispatchCtasPerSm;
   // remote stores fill the links with far fewer CTAs (about 32 GB/s each) than the local fan-out needs for HBM; the
   // receivers end last (4 GPUs, 296 CTAs: 32 senders 352 us, 48 senders 357 - 372 us, 64 senders 363 us)

@@ -63,6 +63,47 @@ def test_layers_without_tokens_and_token_counts_that_do_not_match():
     ep.close()
 
 
+@pytest.mark.parametrize("experts,topk", [(32, 2), (64, 8)])
+def test_a_captured_exchange_follows_the_plan_of_its_replay(experts, topk):
+    # a decode server captures dispatch -> experts -> combine for its largest batch and replays it after plans of fewer tokens
+    from purlin_b200.parallel.expert_parallel import ExpertParallelContext
+    dev = torch.device("cuda", 0)
+    most, hidden = 64, 1040
+    ep = ExpertParallelContext(None, dev, max_tokens=most, hidden=hidden, experts=experts, topk=topk)
+    g = torch.Generator(device=dev).manual_seed(6)
+    x = torch.randn(most, hidden, generator=g, device=dev).to(torch.bfloat16)
+    y = torch.empty_like(x)
+
+    def layer():
+        rows, _ = ep.dispatch(x)
+        ep.out_rows().copy_(rows)
+        ep.combine(most, y)
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ep.route(torch.randn(most, experts, generator=g, device=dev))
+        layer()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            layer()
+        for n, routed in ((most, True), (8, False), (most, False), (33, True), (1, True), (0, False), (17, False)):
+            logits = torch.randn(n, experts, generator=g, device=dev)
+            if routed and n:
+                ep.route(logits)
+            else:
+                ep.plan(logits.topk(topk, dim=1).indices.to(torch.int32), torch.full((n, topk), 1.0 / topk, device=dev))
+            ep.recv_rows().fill_(3.0)
+            graph.replay()
+            torch.cuda.synchronize()
+            ep.check()
+            assert int(ep.recv_counts[-1]) == n * topk
+            assert (ep.recv_rows()[n * topk:] == 3).all()                                           # rows past the routed ones are not sent
+            assert torch.allclose(y[:n].float(), x[:n].float(), rtol=2 ** -7, atol=1e-6)             # the gate weights sum to one
+    del graph
+    ep.close()
+
+
 def test_check_sees_a_wait_that_ran_out_in_the_experts_gemm():
     # a grouped GEMM over a k so long that the wait for its accumulator outlasts a limit of 1 ns, reporting where the block's report
     from purlin_b200.models.moe_block import ExpertParallelMoE

@@ -27,9 +27,6 @@
 namespace purlin {
 namespace ragged {
 
-constexpr int kBM = 128, kBK = 64, kMaxCols = 256;
-constexpr int kABytes = kBM * kBK * 2;
-constexpr int kAccRows = 256;                   // rows of W per accumulator of a pair; a tile has one or two of them
 constexpr int kAccStride = 256, kTmemCols = 512;
 // Two epilogue warps per quarter of the TMEM lanes (a quarter is all that a warp may read): the drain is exposed, and with one
 // each it took twice as long.
@@ -38,8 +35,6 @@ constexpr int kStagingBytes = kEpiWarps * 2048;       // a 32 x 32 bf16 tile per
 constexpr int kBarrierBytes = 256;
 constexpr int kMaxExperts = 512;
 constexpr int kTableBytes = 2 * (kMaxExperts + 1) * 4;
-constexpr int kMaxStages = 8, kRingBytes = 192 * 1024;
-constexpr int kXBox = 32;                       // rows of one X load
 // k-blocks at either end of a tile that the first accumulator gets before the second one: it is finished, and drained, while the
 // second one's last k-blocks run, and the next tile starts with it while the second one is drained. The MMAs of a k-block go into
 // one accumulator then, and each waits for the one before (174 cycles instead of 128, measured): longer leads cost more than they

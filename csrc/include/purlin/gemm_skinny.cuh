@@ -16,18 +16,13 @@
 #include <cuda_bf16.h>
 
 #include "atom.cuh"
+#include "gemm_route.hpp"
 #include "tc_sm100.cuh"
 
 namespace purlin {
 namespace skinny {
 
-constexpr int kRows = 128, kK = 64;            // rows of W per tile, k per stage (128-byte swizzled rows)
-constexpr int kWBytes = kRows * kK * 2;
 constexpr int kThreads = 192;                  // warp 0: TMA, warp 1: MMA, warps 2-5: TMEM -> shared memory; all: the sum
-constexpr int kMaxStages = 8;
-constexpr int kMaxTokens = 256;                // columns of one pass
-constexpr int kBarrierBytes = 256;
-constexpr int kMaxSplit = 8;
 
 struct alignas(64) Maps { CUtensorMap w, x; };
 

@@ -31,7 +31,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -42,6 +41,7 @@
 #include "purlin/constants.hpp"
 #include "purlin/gemm.h"
 #include "purlin/gemm_ragged.cuh"
+#include "purlin/gemm_route.hpp"
 #include "purlin/gemm_skinny.cuh"
 #include "purlin/layout.hpp"
 #include "purlin/tc_sm100.cuh"
@@ -754,14 +754,6 @@ cudaLaunchAttribute overlapAttribute() {
   return a;
 }
 
-// Whether a launch is better placed on an empty GPU. Between half as many CTAs as SMs and six sevenths of them, a kernel that is
-// set up early takes the SMs its predecessor leaves free and then some of those it gives back, so neighbouring SMs that share
-// their path to L2 are both busy, where a launch on its own would have spread out. Where the main loop is short, the microsecond
-// that the overlap saves is more than that costs; from 28 k-blocks on it is not. Apart / overlapped, us: 6148 x 448 x 7000 SwiGLU
-// (98 CTAs) 64.5 / 72.6, 108 x 12672 x 2584 (99) 21.4 / 24.9, 7822 x 384 x 5064 (124) 44.6 / 49.6. Of 1074 shapes on these tiles
-// the overlap slows 32 by more than 5 %; with this rule two, and two that gained more than 3 % lose it.
-bool betterApart(long ctas, int K) { return ctas * 2 > smCount() && ctas * 7 < smCount() * 6 && K >= 28 * kBK; }
-
 template <int EPI, int COMM, int CTAS, int ACCS>
 int launchImpl(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t stream) {
   auto kernel = gemmKernel<EPI, COMM, CTAS, ACCS>;
@@ -800,7 +792,7 @@ int launchImpl(const Maps& maps, const Params& p, const Shape& sh, cudaStream_t 
   attr[1] = overlapAttribute();
   attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(pairs * CTAS); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smemFor(p, sh); cfg.stream = stream;
-  cfg.attrs = attr; cfg.numAttrs = COMM == kCommNone && !betterApart(long(pairs) * CTAS, p.K) ? 2 : 1;
+  cfg.attrs = attr; cfg.numAttrs = COMM == kCommNone && !route::betterApart(long(pairs) * CTAS, p.K, smCount()) ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, q);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
@@ -845,66 +837,19 @@ struct GroupedArgs {
   uint64_t timeoutNs = 2ull * 1000 * 1000 * 1000;   // of every wait inside the kernel
 };
 
-// Which GEMMs the few-rows kernel takes, each line with one B200's times in us, it / the other tiles. Few rows of W (a router)
-// with a long k: 4096 x 32 x 7168 11 / 75; with a short k the sum over the partial tiles costs more than it saves (1656 x 208
-// x 112 14.4 / 12.2 a call).
-bool fewWeightRows(int M, int N, int K, int epilogue) { return epilogue == kEpiStore && M > skinny::kMaxTokens / 2 && N <= skinny::kMaxTokens && K >= 2048; }
-bool useSkinny(int M, int N, int K, int epilogue) {
-  if (fewWeightRows(M, N, K, epilogue)) return true;
-  // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 4096 x 1024 7.9 / 8.3, 54 x 7648 x 1336 SwiGLU 14.3 / 17.2;
-  // but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4. Above, what the others would take decides (gemmRoute).
-  return M <= 64 && (M <= 32 || K >= (N <= 8192 ? 512 : 1024));
-}
-// Parts that the few-rows kernel cuts k into: while the CTAs have a place on the GPU at the same time and a part keeps at least four
-// k-blocks; eight where many tiles are split four ways (64 x 7744 x 1160, 61 tiles: 12.0 us whole, 10.6 in two parts, 13.0 in four).
-// Measured, 1 x 8192 x 3584: one CTA per tile 20.1 us, two 14.4, four 14.2, eight 18.2; 64 x 8192 x 28672: 142.6 / 87.4 / 79.1 /
-// 90.5 us. More CTAs than places cost a second wave: 64 x 11232 x 1952 SwiGLU (88 tiles, 296 places) 16.6 / 14.7 / 26.7,
-// 192 x 5824 x 1280 (46 tiles, 148 places) 17.0 / 13.1 / 23.9. At most 15 clusters of eight fit on the GPU at once, so eight
-// are used for no more tiles than that.
-int skinnySplit(long tiles, int kBlocks, long slots) {
-  int split = 1;
-  while (split < (tiles <= 15 ? skinny::kMaxSplit : 4) && tiles * split * 2 <= slots && kBlocks >= (split > 1 && tiles > 24 ? 16 : 8) * split) split *= 2;
-  return split;
-}
-
-// CTAs that share the columns of a tile, where its k parts leave SMs without one: a k-block takes 450 cycles and 3.5 per column, and the
-// few rows of W that they all read come from L2 (fifteen clusters of eight fit on the GPU). In a graph, us, one CTA for all columns /
-// shared: 128 x 32 x 7168 9.8 / 7.5, 128 x 256 x 4096 10.9 / 7.1, 200 x 512 x 7168 17.4 / 12.0, 300 x 256 x 7168 16.5 / 9.6, 128 x 2048 x 4096
-// 13.8 / 11.4, 50 x 600 x 1000 6.7 / 5.4. More than half the SMs only for parts of six k-blocks: 40 x 2048 x 1024 5.7 / 6.3.
-int skinnyGroups(int columns, long tiles, int split, int kBlocks) {
-  const long ctas = std::max(tiles * split, 1l), places = kBlocks >= 6 * split ? smCount() : smCount() / 2;
-  const long room = split == skinny::kMaxSplit ? 15 / std::max(tiles, 1l) : places / ctas;
-  return int(std::max(std::min(long(columns + 31) / 32, room), 1l));
-}
-
 // ---- few rows of activations (or of weights): gemm_skinny.cuh ----
 int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
   if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
   skinny::Params p{};
   // Few rows of W against many rows of X (a router): the operands change places and the output row is the MMA's row.
-  const bool tokenRows = !g.counts && fewWeightRows(M, N, K, epilogue);
+  const bool tokenRows = !g.counts && route::fewWeightRows(M, N, K, epilogue == kEpiSwiglu);
   if (tokenRows) { std::swap(A, B); std::swap(M, N); }
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status;
   p.timeoutNs = g.timeoutNs;
-  // one pass has to hold a group's rows (a second pass reads W again): a group of average size has twice the room
-  const int room = std::min(g.counts ? 2 * g.likelyRows + 16 : M, M);
-  p.tokenBox = room <= 16 ? 16 : 32;
-  p.passTokens = std::min(int(roundUp(size_t(room), size_t(p.tokenBox))), skinny::kMaxTokens);
-  const int tiles = (N + skinny::kRows - 1) / skinny::kRows, kBlocks = (K + skinny::kK - 1) / skinny::kK;
-  const int split = skinnySplit(long(tiles) * g.experts, kBlocks, long(smCount()) * (p.passTokens <= 128 ? 2 : 1));
-  p.columnGroups = 1;
-  if (!g.counts && M <= p.passTokens) {
-    p.columnGroups = skinnyGroups(M, tiles, split, kBlocks);
-    p.passTokens = int(roundUp(size_t(M + p.columnGroups - 1) / p.columnGroups, size_t(p.tokenBox)));
-  }
-  // up to 128 columns two CTAs share an SM (128 columns: 3 stages of 32 KiB each)
-  const int stageBytes = skinny::kWBytes + p.passTokens * skinny::kK * 2;
-  const int perSm = p.passTokens <= 128 ? 2 : 1;
-  const int budget = (perSm == 2 ? 113 : 227) * 1024 - 1024 - skinny::kBarrierBytes;
-  p.stages = std::min(budget / stageBytes, skinny::kMaxStages);
-  for (p.tmemCols = 32; p.tmemCols < p.passTokens; p.tmemCols *= 2) {}
+  const route::SkinnyCut cut = route::skinnyCut(M, N, K, g.experts, g.counts ? g.likelyRows : 0, smCount());
+  p.tokenBox = cut.tokenBox; p.passTokens = cut.passTokens; p.columnGroups = cut.columnGroups; p.stages = cut.stages; p.tmemCols = cut.tmemCols; p.ahead = cut.ahead;
   skinny::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), skinny::kRows) || !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(p.tokenBox))) return 1;
   const int mode = tokenRows ? skinny::kTokenRows : epilogue == kEpiSwiglu ? skinny::kWeightRowsSwiglu : skinny::kWeightRows;
@@ -923,38 +868,25 @@ int launchSkinny(MapCache& cache, const void* A, const void* B, void* C, int M, 
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   attr[1] = overlapAttribute();
-  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(split); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(unsigned(tiles * split), unsigned(g.experts * p.columnGroups)); cfg.blockDim = dim3(skinny::kThreads);
-  cfg.dynamicSmemBytes = size_t(p.stages) * stageBytes + skinny::kBarrierBytes + 1024; cfg.stream = stream;
-  // Between half as many CTAs as SMs and as many, they are better placed on an empty GPU, one to an SM: set up early they pile
-  // up two to an SM where the kernel before left room (97-token MLP block 5824 x 1888, 120 CTAs: 40.7 us apart, 42.5 overlapped).
-  const long ctas = long(tiles) * split * g.experts * p.columnGroups;
-  // With shared columns the tiles are small and the launch is the larger part: 200 x 2048 x 4096 15.1 us apart, 13.7 overlapped.
-  const bool apart = ctas * 2 > smCount() && ctas < smCount() && p.columnGroups == 1;
-  p.ahead = apart ? 0 : p.stages;
-  cfg.attrs = attr; cfg.numAttrs = apart ? 1 : 2;
+  attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(cut.split); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  const int tiles = (N + skinny::kRows - 1) / skinny::kRows;
+  cfg.gridDim = dim3(unsigned(tiles * cut.split), unsigned(g.experts * p.columnGroups)); cfg.blockDim = dim3(skinny::kThreads);
+  cfg.dynamicSmemBytes = size_t(p.stages) * cut.stageBytes + skinny::kBarrierBytes + 1024; cfg.stream = stream;
+  cfg.attrs = attr; cfg.numAttrs = cut.apart ? 1 : 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
 }
 
-constexpr int kFewGroupRows = 12;
-
 // ---- any number of rows of activations: gemm_ragged.cuh ----
-constexpr int kMaxParts = 4;            // pairs of a cluster (eight CTAs, the largest portable cluster)
 auto raggedKernel(int epilogue, bool split) {
   return epilogue == kEpiSwiglu ? (split ? ragged::raggedGemmKernel<true, true> : ragged::raggedGemmKernel<true, false>)
                                 : (split ? ragged::raggedGemmKernel<false, true> : ragged::raggedGemmKernel<false, false>);
 }
 constexpr size_t kRaggedSmem = 1024 + ragged::kRingBytes + ragged::kStagingBytes + ragged::kBarrierBytes + ragged::kTableBytes;
 static_assert(kRaggedSmem <= size_t(kSmemLimit), "the ring, the staging tiles and the tables fit one CTA per SM");
-static_assert(ragged::kRingBytes >= (kMaxParts - 1) * 2 * (ragged::kMaxCols / 32 / kMaxParts) * 4 * 4096 &&
+static_assert(ragged::kRingBytes >= (route::kMaxParts - 1) * 2 * (ragged::kMaxCols / 32 / route::kMaxParts) * 4 * 4096 &&
               ragged::kRingBytes >= 2 * (ragged::kMaxCols / 32 / 2) * 4 * 4096, "the partial tiles of the other pairs take the place of the stages");
-// stages of a ring for `accs` accumulators and `cols` columns per tile
-int raggedStages(int accs, int cols, uint32_t& stageBytes) {
-  stageBytes = uint32_t(accs * ragged::kABytes + (cols / 2 + ragged::kXBox - 1) / ragged::kXBox * ragged::kXBox * kBK * 2);
-  return std::min(int(ragged::kRingBytes / stageBytes), ragged::kMaxStages);
-}
 static_assert(ragged::kRingBytes / (2 * ragged::kABytes + ragged::kMaxCols / 2 * kBK * 2) >= ragged::kLead, "a lead holds its stages until the second accumulator has read them");
 
 // Clusters of `parts` pairs (1, 2 or 4) that the device can hold at once; 0: none, or with the error set for one pair
@@ -979,62 +911,7 @@ int raggedClusters(int epilogue, int parts) {
   return std::max(clusters, 0);
 }
 
-// How the ragged kernel cuts a GEMM: one or two accumulators per tile, the number of column tiles, and how many pairs share a tile's k
-// range, whichever has the least expected time. The cycles are a model, its constants fitted to about 700 shapes on one B200:
-//   a k-block of a tile of two accumulators takes the tensor pipe 4 cycles a column, and its operands come at 44 bytes a cycle and SM;
-//   of one accumulator 500 and 2.1 a column (the round trips of its loads); rows of K that begin off a cache line 12 % more;
-//   drain: what a tile's epilogue exposes; behind the last one its stores remain;
-//   a cluster of several pairs is placed later than a pair (3500 cycles a pair) and exchanges partial tiles at 12 bytes a cycle;
-//   the weights come through HBM once.
-// What it buys, us, one B200, before / now: 2048 x 14336 x 8192 SwiGLU 371 / 325 (ten column tiles, where eight left a fourth wave of two
-// tiles), 1000 x 14336 x 8192 SwiGLU 205 / 168, 1000 x 8192 x 7168 97 / 85, 384 x 14336 x 8192 SwiGLU 121 / 78, 700 x 8192 x 28672 428 / 250;
-// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58. Over 750 random
-// shapes the geometric mean is 1.09; 22 are slower by more than 3 %, the worst by 18 % (2006 x 64 x 1320 11.6 / 14.2).
-struct RaggedPlan { int tileAccs = 2, colTiles = 1, tiles = 1, parts = 1; double cycles = 0; };
-RaggedPlan raggedPlan(int M, int N, int K, int epilogue, const int (&clusters)[3]) {
-  const int kBlocks = (K + kBK - 1) / kBK, units = (M + 31) / 32, fewest = (units + 7) / 8;
-  const double unaligned = K % kBK ? 1.12 : 1.;                 // rows of K that do not begin on a cache line
-  auto cyclesOf = [&](int accs, double cols, int64_t tiles, int parts) {
-    auto perBlock = [&](int a) {
-      if (a == 1) return (500 + 2.1 * cols) * unaligned;
-      return std::max(4 * cols, (2 * ragged::kABytes + cols * 64) / 44 * unaligned);
-    };
-    auto drain = [&](int a) { return 1200. + a * cols * (epilogue == kEpiSwiglu ? 8. : 3.); };
-    const int places = clusters[parts / 2];
-    const int64_t full = tiles / places, rest = tiles % places;
-    const double whole = (kBlocks + parts - 1) / parts * perBlock(accs) + drain(accs) + (parts > 1 ? 3500. * parts + accs * cols * 512. * (parts - 1) / parts / 12 : 0.);
-    const double tail = rest == 0 ? 0. : parts == 1 && accs == 2 && 2 * rest <= places ? kBlocks * perBlock(1) + drain(1) : whole;
-    // the weights once through HBM, at least
-    return std::max(double(full) * whole + tail, (2. * N * K + 2. * M * K) / 3300. * unaligned) + 4500. + accs * cols * 8.;
-  };
-  RaggedPlan best;
-  double bestKey = 0;
-  for (int accs = 1; accs <= 2; ++accs) {
-    // the fewest column tiles, one and two more, tiles of at most 7 to 4 units (of 32 rows), and the numbers that just fill one to three
-    // waves more than the fewest need
-    const int64_t wTiles = (N + accs * ragged::kAccRows - 1) / (accs * ragged::kAccRows), waves = fewest * wTiles / clusters[0];
-    for (int c = 0; c < 10; ++c) {
-      const int64_t want = c < 3 ? fewest + c : c < 7 ? (units + 9 - c) / (10 - c) : (waves + c - 6) * clusters[0] / wTiles;
-      if (want < fewest || want > units || want > 2 * fewest + 2) continue;
-      const int n = int(want);
-      const int64_t tiles = n * wTiles;
-      const double average = 32. * units / n, widest = (units + n - 1) / n * 32;
-      for (int parts = 1; parts <= kMaxParts; parts *= 2) {
-        if (!clusters[parts / 2] || kBlocks < 8 * parts || (parts > 1 && tiles > clusters[parts / 2])) break;
-        // Among cuts: a pair with few tiles has the widest among them, and narrow tiles move more bytes per operation, which costs power
-        // (2072 x 4800 x 5016 SwiGLU: 11 tiles of 192 88.7 us, 14 of 128 and 160 97.2).
-        const double key = cyclesOf(accs, average + (widest - average) * clusters[0] / std::max<int64_t>(tiles, clusters[0]), tiles, parts) * (0.95 + 12.8 / average);
-        if (bestKey == 0 || key < bestKey) {
-          bestKey = key;
-          best = RaggedPlan{accs, n, int(std::min<int64_t>(tiles, INT32_MAX / 4)), parts, cyclesOf(accs, average, tiles, parts)};
-        }
-      }
-    }
-  }
-  return best;
-}
-
-int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, const RaggedPlan& plan, uint32_t* status, cudaStream_t stream) {
+int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const GroupedArgs& g, const route::RaggedPlan* plan, uint32_t* status, cudaStream_t stream) {
   const int outCols = epilogue == kEpiSwiglu ? N / 2 : N;
   if (reinterpret_cast<uintptr_t>(C) % 16 || (outCols * 2) % 16) { setError("TMA operands need 16-byte aligned base and row pitch"); return 1; }
   if (g.experts > ragged::kMaxExperts) { setError("grouped GEMM: at most 512 experts"); return 1; }
@@ -1043,16 +920,8 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   ragged::Params p{};
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.experts = g.experts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status; p.timeoutNs = g.timeoutNs;
-  p.tileAccs = 2; p.colTiles = 1; p.parts = 1;
-  // (groups of a few dozen rows: narrow tiles leave room for a fifth stage)
-  p.maxCols = g.counts && g.likelyRows <= 40 ? 64 : ragged::kMaxCols;
-  int items = INT32_MAX;
-  if (!g.counts) {
-    p.tileAccs = plan.tileAccs; p.colTiles = plan.colTiles; p.parts = plan.parts;
-    p.maxCols = ((M + 31) / 32 + plan.colTiles - 1) / plan.colTiles * 32;
-    items = plan.parts > 1 ? plan.tiles : plan.tileAccs * plan.tiles;      // (the tiles of a small last wave are issued as halves)
-  }
-  p.stages = raggedStages(p.tileAccs, p.maxCols, p.stageBytes);
+  const route::RaggedCut cut = route::raggedCut(M, K, plan, g.likelyRows, pairs, smCount());
+  p.tileAccs = cut.tileAccs; p.colTiles = cut.colTiles; p.maxCols = cut.maxCols; p.parts = cut.parts; p.stages = cut.stages; p.stageBytes = cut.stageBytes;
   ragged::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), ragged::kBM) ||
       !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(ragged::kXBox))) return 1;
@@ -1060,32 +929,11 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = unsigned(2 * p.parts); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1] = overlapAttribute();
-  const int grid = (p.parts > 1 ? items : std::min(pairs, items)) * 2 * p.parts;
-  cfg.attrs = attr; cfg.blockDim = dim3(ragged::kThreads); cfg.dynamicSmemBytes = kRaggedSmem; cfg.gridDim = dim3(unsigned(grid)); cfg.stream = stream;
-  // (fewer tiles than pairs: the pairs without one leave at once; 2066 x 3144 x 4264, 63 tiles: 49.7 us apart, 58.0 overlapped)
-  cfg.numAttrs = betterApart(p.parts > 1 ? grid : items, K) ? 1 : 2;
+  cfg.attrs = attr; cfg.blockDim = dim3(ragged::kThreads); cfg.dynamicSmemBytes = kRaggedSmem; cfg.gridDim = dim3(unsigned(cut.grid)); cfg.stream = stream;
+  cfg.numAttrs = cut.apart ? 1 : 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, raggedKernel(epilogue, p.parts > 1), maps, p);
   if (e != cudaSuccess) { setError(std::string("GEMM launch: ") + cudaGetErrorString(e)); return 1; }
   return 0;
-}
-
-// The plain tiles of this file on the same scale.
-double plainCycles(const Params& p, const Shape& sh, int epilogue) {
-  const double tiles = double(p.tilesM) * p.tilesN, places = sh.ctas == 2 ? smCount() / 2 : smCount();
-  const double block = sh.accs == 2 ? std::max(4. * p.bn, 900.) : std::max({2. * p.bn + 184., (kABytes + p.bn / sh.ctas * 128) / 58., 700.});
-  const double drain = sh.accs == 2 ? (epilogue == kEpiSwiglu ? 9000. : 6000.) * p.bn / 256 : 0.;
-  const double waves = std::ceil(tiles / places), ragged = p.K % kBK ? 1.25 : 1.;      // rows of K that do not begin on a cache line
-  return std::max(waves * ((p.K + kBK - 1) / kBK * block * ragged + drain) + 3000., (2. * p.N * p.K + 2. * p.M * p.K) / 3300. * ragged);
-}
-
-// ... and the few-rows kernel: its CTAs' round trips (per k-block 450 cycles and 3.5 per row, measured with L2-sized weights) or the
-// weights, and a fixed part that grows with the rows (the partial tiles through distributed shared memory).
-double skinnyCycles(int M, int N, int K, int epilogue) {
-  if (M > skinny::kMaxTokens || N > 16384) return 1e30;
-  const long tiles = (N + skinny::kRows - 1) / skinny::kRows, slots = long(smCount()) * (M <= 128 ? 2 : 1);
-  const int kBlocks = (K + skinny::kK - 1) / skinny::kK, split = skinnySplit(tiles, kBlocks, slots);
-  const double waves = std::ceil(double(tiles * split) / slots), block = (450. + 3.5 * M / skinnyGroups(M, tiles, split, kBlocks)) * (tiles * split > smCount() ? 1.3 : 1.);
-  return std::max(waves * kBlocks / split * block, 1.15 * (2. * N * K + 2. * M * K) / 3300.) + 7000. + (epilogue == kEpiSwiglu ? 105. : 45.) * M;
 }
 
 // Which kernel a GEMM takes, and its cut if it is the ragged one: the least expected time. The ragged kernel was 3 % ahead of the plain
@@ -1093,15 +941,17 @@ double skinnyCycles(int M, int N, int K, int epilogue) {
 // x 4096 (36 / 33, one wave of narrower tiles); the few-rows kernel ahead at 128 x 8192 x 8192 (33.6, ragged 37.5, plain 42.2), behind at
 // 128 x 8192 x 2048 (18.2, plain 13.9) and 160 x 8192 x 8192 (38.6, ragged 36.6).
 enum { kRoutePlain = 0, kRouteSkinny = 1, kRouteRagged = 2 };
-struct Route { int M = 0, N = 0, K = 0, epilogue = 0, device = -1, kernel = kRoutePlain; RaggedPlan cut; };
+struct Route { int M = 0, N = 0, K = 0, epilogue = 0, device = -1, kernel = kRoutePlain; route::RaggedPlan cut; };
 Route findRoute(const Params& p, const Shape& sh, int epilogue) {
   Route r;
-  if (useSkinny(p.M, p.N, p.K, epilogue)) { r.kernel = kRouteSkinny; return r; }
-  const double plain = plainCycles(p, sh, epilogue), skinny = p.M > 64 ? skinnyCycles(p.M, p.N, p.K, epilogue) : 1e30;
+  const bool swiglu = epilogue == kEpiSwiglu;
+  if (route::useSkinny(p.M, p.N, p.K, swiglu)) { r.kernel = kRouteSkinny; return r; }
+  const double plain = route::plainCycles(route::PlainTiles{p.tilesM, p.tilesN, p.bn, sh.ctas, sh.accs}, p.M, p.N, p.K, swiglu, smCount());
+  const double skinny = p.M > 64 ? route::skinnyCycles(p.M, p.N, p.K, swiglu, smCount()) : 1e30;
   double ragged = 1e30;
   if (p.K >= 512 && !switches().singleCta && !switches().oneAcc) {
     const int clusters[3] = {raggedClusters(epilogue, 1), raggedClusters(epilogue, 2), raggedClusters(epilogue, 4)};
-    if (clusters[0]) { r.cut = raggedPlan(p.M, p.N, p.K, epilogue, clusters); ragged = r.cut.cycles; }
+    if (clusters[0]) { r.cut = route::raggedPlan(p.M, p.N, p.K, swiglu, clusters); ragged = r.cut.cycles; }
   }
   r.kernel = skinny < std::min(plain, ragged) ? kRouteSkinny : ragged < plain ? kRouteRagged : kRoutePlain;
   return r;
@@ -1162,7 +1012,7 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   if (bn == 0) {
     const Route& route = gemmRoute(p, sh, epilogue);
     if (route.kernel == kRouteSkinny) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
-    if (route.kernel == kRouteRagged) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, route.cut, status, static_cast<cudaStream_t>(stream));
+    if (route.kernel == kRouteRagged) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, &route.cut, status, static_cast<cudaStream_t>(stream));
   }
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||
@@ -1193,8 +1043,8 @@ int purlin_gemm_grouped_bf16(const void* A, const void* B, void* C, int rows, in
   GroupedArgs g;
   g.experts = experts; g.counts = counts; g.likelyRows = std::max(likelyRows, 1);
   if (timeoutNs) g.timeoutNs = timeoutNs;
-  if (g.likelyRows <= kFewGroupRows) return launchSkinny(cache, A, B, C, rows, N, K, epilogue, g, status, static_cast<cudaStream_t>(stream));
-  return launchRagged(cache, A, B, C, rows, N, K, epilogue, g, RaggedPlan{}, status, static_cast<cudaStream_t>(stream));
+  if (g.likelyRows <= route::kFewGroupRows) return launchSkinny(cache, A, B, C, rows, N, K, epilogue, g, status, static_cast<cudaStream_t>(stream));
+  return launchRagged(cache, A, B, C, rows, N, K, epilogue, g, nullptr, status, static_cast<cudaStream_t>(stream));
 }
 
 size_t purlin_tp_workspace_bytes(int world, int M, int kAg, int nRs) { return tpLayout(world, M, kAg, nRs).total; }

@@ -99,7 +99,10 @@ inline SkinnyCut skinnyCut(int M, int N, int K, int experts, int likelyRows, int
   const long ctas = long(tiles) * c.split * experts * c.columnGroups;
   // With shared columns the tiles are small and the launch is the larger part: 200 x 2048 x 4096 15.1 us apart, 13.7 overlapped.
   c.apart = ctas * 2 > sms && ctas < sms && c.columnGroups == 1;
-  c.ahead = c.apart ? 0 : c.stages;
+  // Grouped, nobody knows yet which experts have rows: a lap of every idle expert's ring was up to four times the bytes that the call
+  // needs (MoE block 7168 / 2048 with / without it, us, one token: top-1 of 32 100.4 / 84.0, top-1 of 64 114.7 / 92.2,
+  // top-8 of 64 215 / 184; two tokens, top-8 of 64 306 / 279).
+  c.ahead = c.apart || likelyRows ? 0 : c.stages;
   return c;
 }
 

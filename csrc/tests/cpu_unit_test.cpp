@@ -1,4 +1,4 @@
-// Host-only unit tests of the compile-time loop and the prefetch-ring driver (no GPU, no CUDA headers).
+// Host-only unit tests of the compile-time loop, the prefetch-ring driver and the rules that cut a GEMM (no GPU, no CUDA headers).
 //
 // Counterpart of csrc/tests/static_for.cu:6-77 and csrc/tests/pipeline.cu:8-156 in the reference: the loop's
 // order, index type, empty-loop and non-copyable-functor behaviour; the pipeline's hook order and data for depths
@@ -11,6 +11,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "purlin/gemm_route.hpp"
 #include "purlin/pipeline.hpp"
 #include "purlin/plan.hpp"
 #include "purlin/static_for.hpp"
@@ -164,6 +165,17 @@ static void testPartition() {
   CHECK(ok, "partitionAligned: contiguous, aligned, complete, balanced within one access");
 }
 
+// ---- how the GEMM kernels are cut (sizes alone; 148 SMs) ----
+static void testSkinnyCut() {
+  bool idleReadNothing = true;
+  for (int rows : {1, 8, 40, 1000})
+    for (int experts : {1, 8, 32, 64, 512})
+      for (int likely : {1, 4, 12})
+        for (int n : {256, 4096, 7168}) idleReadNothing = idleReadNothing && route::skinnyCut(rows, n, 7168, experts, likely, 148).ahead == 0;
+  CHECK(idleReadNothing, "grouped few-rows GEMM: nothing of W is asked for before the counts are known");
+  CHECK(route::skinnyCut(1, 8192, 3584, 1, 0, 148).ahead > 0, "few-rows GEMM: a lap of W is asked for while the kernel before drains");
+}
+
 int main() {
   testStaticFor();
   testPipelineDepth<1>();
@@ -172,6 +184,7 @@ int main() {
   testPipelineDepth<8>();
   testPipelineOrder();
   testPartition();
+  testSkinnyCut();
   std::printf("%s: %d failure(s)\n", g_failures ? "FAILED" : "PASSED", g_failures);
   return g_failures ? 1 : 0;
 }

@@ -87,6 +87,7 @@ inline SkinnyCut skinnyCut(int M, int N, int K, int experts, int likelyRows, int
   if (!likelyRows && M <= c.passTokens) {
     c.columnGroups = skinnyGroups(M, tiles, c.split, kBlocks, sms);
     c.passTokens = up((M + c.columnGroups - 1) / c.columnGroups, c.tokenBox);
+    c.columnGroups = (M + c.passTokens - 1) / c.passTokens;      // (160 columns for four: 64 each, and nothing for the fourth)
   }
   // up to 128 columns two CTAs share an SM (128 columns: 3 stages of 32 KiB each)
   c.stageBytes = skinny::kWBytes + c.passTokens * skinny::kK * 2;

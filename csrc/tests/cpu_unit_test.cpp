@@ -173,6 +173,14 @@ static void testSkinnyCut() {
       for (int likely : {1, 4, 12})
         for (int n : {256, 4096, 7168}) idleReadNothing = idleReadNothing && route::skinnyCut(rows, n, 7168, experts, likely, 148).ahead == 0;
   CHECK(idleReadNothing, "grouped few-rows GEMM: nothing of W is asked for before the counts are known");
+  bool everyGroupHasColumns = true;
+  for (int m = 1; m <= skinny::kMaxTokens; ++m)
+    for (int n : {8, 128, 264, 1024, 2048, 4096, 8192})
+      for (int k : {64, 520, 1000, 4096, 7168}) {
+        const route::SkinnyCut c = route::skinnyCut(m, n, k, 1, 0, 148);
+        everyGroupHasColumns = everyGroupHasColumns && (c.columnGroups - 1) * c.passTokens < m && c.columnGroups * c.passTokens >= m;
+      }
+  CHECK(everyGroupHasColumns, "few-rows GEMM: the CTAs that share a tile's columns all have some");
   CHECK(route::skinnyCut(1, 8192, 3584, 1, 0, 148).ahead > 0, "few-rows GEMM: a lap of W is asked for while the kernel before drains");
 }
 

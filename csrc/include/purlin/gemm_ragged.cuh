@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
           }
           tc::fenceBeforeThreadSync();
           __syncwarp();
-          if (lane == 0) tc::mbarArriveCluster(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a0 + b)));
+          if (lane == 0) tc::mbarArriveClusterTmem(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a0 + b)));
         }
         if (!ok) return false;
 #pragma unroll

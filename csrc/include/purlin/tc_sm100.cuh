@@ -110,7 +110,14 @@ PURLIN_D void clusterSync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 PURLIN_D void mbarArriveCluster(uint32_t clusterBarAddress) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterBarAddress) : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterBarAddress) : "memory");
+}
+// The same to hand back tensor memory and nothing else: the loads from it have been waited for and fenceBeforeThreadSync() orders them
+// before the arrival, as fenceAfterThreadSync() orders the waiter's MMAs after it. The release at cluster scope would wait for every
+// global store before it, which the ragged GEMM's epilogue has in flight (one B200, us, released / relaxed: MoE block of 128 tokens
+// 508 / 499, MLP block 8192 x 7168 of 1000 tokens 301 / 296.5).
+PURLIN_D void mbarArriveClusterTmem(uint32_t clusterBarAddress) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterBarAddress) : "memory");
 }
 // tile load of one CTA of a pair; the transaction bytes are credited to a barrier that may live in the other CTA
 PURLIN_D void tmaLoad2dPair(uint32_t smemDst, const CUtensorMap* map, int x, int y, uint32_t clusterBarAddress) {

@@ -50,8 +50,8 @@ struct Params {
   int tileAccs;            // accumulators of a tile: 2 (512 rows of W) or 1 (256)
   int colTiles, maxCols;   // column tiles, and columns of the widest one; with counts an expert has a tile per maxCols rows
   int parts;               // SPLIT: pairs of a cluster
-  int stages;              // of stageBytes each, in kRingBytes
-  uint32_t stageBytes;
+  int stages, narrowStages;            // of so many bytes each, in kRingBytes; narrow: with counts, tiles of kNarrowCols columns
+  uint32_t stageBytes, narrowStageBytes;
   int experts;
   const int32_t* counts;   // rows per expert, or null: one group of `tokens` rows
   __nv_bfloat16* C;
@@ -78,13 +78,14 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   const uint32_t stagingAll = base + kRingBytes;
   const uint32_t barBase = stagingAll + kStagingBytes;
   auto fullBar = [&](uint32_t s) { return barBase + 8u * s; };
-  auto emptyBar = [&](uint32_t s) { return barBase + 8u * (uint32_t(p.stages) + s); };
-  auto tmemFullBar = [&](int a) { return barBase + 8u * (2u * uint32_t(p.stages) + uint32_t(a)); };
-  auto tmemEmptyBar = [&](int a) { return barBase + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a)); };
+  auto emptyBar = [&](uint32_t s) { return barBase + 8u * (uint32_t(kMaxStages) + s); };
+  auto tmemFullBar = [&](int a) { return barBase + 8u * (2u * uint32_t(kMaxStages) + uint32_t(a)); };
+  auto tmemEmptyBar = [&](int a) { return barBase + 8u * (2u * uint32_t(kMaxStages) + 2u + uint32_t(a)); };
   unsigned char* tail = smem + kRingBytes + kStagingBytes;
-  uint32_t* words = reinterpret_cast<uint32_t*>(tail + 8 * (2 * p.stages + 4));
+  uint32_t* words = reinterpret_cast<uint32_t*>(tail + 8 * (2 * kMaxStages + 4));
   volatile uint32_t* tmemBaseWord = words;
   volatile int* abortWord = reinterpret_cast<volatile int*>(words + 1);
+  volatile uint32_t* narrowWord = words + 2;                          // whether the experts' tiles are narrow
   int* itemStart = reinterpret_cast<int*>(tail + kBarrierBytes);      // [experts + 1] first tile of an expert
   int* rowStart = itemStart + (kMaxExperts + 1);                      // [experts + 1] first row of X of an expert
 
@@ -93,10 +94,13 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   const int parts = SPLIT ? p.parts : 1, part = SPLIT ? int(clusterRank / 2) : 0;     // pairs that share a tile
   const int pairIdx = int(blockIdx.x) / (2 * parts), numPairs = int(gridDim.x) / (2 * parts);
   const int tileRows = kAccRows * p.tileAccs, wTiles = (p.N + tileRows - 1) / tileRows;
-  auto tilesOf = [&](int rows) { return p.counts ? (rows + p.maxCols - 1) / p.maxCols : p.colTiles; };
+  auto tilesOf = [&](int rows, bool narrow) {
+    const int cols = narrow ? kNarrowCols : p.maxCols;
+    return p.counts ? (rows + cols - 1) / cols : p.colTiles;
+  };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
+    for (int s = 0; s < kMaxStages; ++s) { tc::mbarInit(fullBar(s), 1); tc::mbarInit(emptyBar(s), 1); }
     for (int a = 0; a < 2; ++a) { tc::mbarInit(tmemFullBar(a), 1); tc::mbarInit(tmemEmptyBar(a), 2 * kEpiWarps); }   // the warps of both CTAs
     *abortWord = 0;
     tc::mbarFenceInit();
@@ -112,6 +116,22 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     const uint32_t limit = uint32_t(p.tokens);
     uint32_t rows0 = 0;
     int items0 = 0;
+    // Narrow tiles have room for a fifth stage, but an expert of many rows then reads its weights once for every 64 of them: they are taken
+    // where they are at most an eighth more tiles (MoE block 7168 / 2048 of 32 experts, one of which gets the most rows, us, wide / narrow:
+    // average 32, most 128 497 / 489; 19, 300 493 / 484; 40, 640 498 / 548; 40, 654 501 / 556).
+    bool narrow = false;
+    if (p.counts) {
+      uint32_t few = 0, many = 0;
+      for (int e = lane; e < p.experts; e += 32) {
+        const int r = int(skinny::groupRowsOf(p.counts[e], limit));
+        few += uint32_t(tilesOf(r, false));
+        many += uint32_t(tilesOf(r, true));
+      }
+      few = __reduce_add_sync(0xffffffffu, few);
+      many = __reduce_add_sync(0xffffffffu, many);
+      narrow = uint64_t(many) * 8 <= uint64_t(few) * 9;
+    }
+    if (lane == 0) *narrowWord = narrow ? 1u : 0u;
     for (int e0 = 0; e0 < p.experts; e0 += 32) {
       const int e = e0 + lane;
       uint32_t sum = e < p.experts ? (p.counts ? skinny::groupRowsOf(p.counts[e], limit) : limit) : 0u;
@@ -120,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
       const uint32_t before = __shfl_up_sync(0xffffffffu, sum, 1);
       const int first = int(lane ? skinny::addRows(rows0, before, limit) : rows0), end = int(skinny::addRows(rows0, sum, limit));
       const int r = end - first;
-      const int n = r > 0 ? tilesOf(r) * wTiles : 0;
+      const int n = r > 0 ? tilesOf(r, narrow) * wTiles : 0;
       int items = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, items, o); if (lane >= o) items += v; }
@@ -136,6 +156,8 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   tc::fenceAfterThreadSync();
   tc::gridLaunchDependents();
   const uint32_t tmemBase = *tmemBaseWord;
+  const bool narrow = *narrowWord != 0;
+  const uint32_t stages = uint32_t(narrow ? p.narrowStages : p.stages), stageBytes = narrow ? p.narrowStageBytes : p.stageBytes;
   const uint32_t leaderBars = tc::mapToCta(barBase, clusterRank & ~1u), pairMask = 3u << (clusterRank & ~1u);
   const int numTiles = itemStart[p.experts], rest = numTiles % numPairs;
   // whole tiles; the others count as two items each
@@ -150,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     while (tile >= itemStart[expert + 1]) ++expert;
     Item m;
     m.expert = expert;
-    const int rows = rowStart[expert + 1] - rowStart[expert], tiles = tilesOf(rows);
+    const int rows = rowStart[expert + 1] - rowStart[expert], tiles = tilesOf(rows, narrow);
     const int i = tile - itemStart[expert], units = (rows + 31) / 32;
     int first = 0, width = units;                              // of the column tile, in units of 32 (steps of an MMA of a pair)
     m.w0 = i * tileRows;
@@ -209,14 +231,14 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
         for (int kb = kbBegin; kb < kbEnd; ++kb) {
           ok = tc::mbarWait(emptyBar(st), ph ^ 1, abortWord, p.timeoutNs);
           if (!ok) { skinny::recordTimeout(p.status, 1, m.w0, kb); break; }
-          const uint32_t sW = base + st * p.stageBytes, sX = sW + xAt;
+          const uint32_t sW = base + st * stageBytes, sX = sW + xAt;
           const uint32_t leaderFull = leaderBars + 8u * st;
           if (ctaRank == 0) tc::mbarExpectTx(fullBar(st), bytes);        // both CTAs' bytes are credited to CTA 0's barrier
           tc::tmaLoad2dPair(sW, &maps.w, kb * kBK, wRow, leaderFull);
           if (m.accs == 2) tc::tmaLoad2dPair(sW + kABytes, &maps.w, kb * kBK, wRow + 2 * kBM, leaderFull);
           for (int i = 0; i < loads; ++i)
             tc::tmaLoad2dPair(sX + uint32_t(i * kXBox * kBK * 2), &maps.x, kb * kBK, xRow + i * kXBox + (2 * i >= loads ? jump : 0), leaderFull);
-          if (++st == uint32_t(p.stages)) { st = 0; ph ^= 1; }
+          if (++st == stages) { st = 0; ph ^= 1; }
         }
         return ok;
       });
@@ -225,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
     if (lane == 0 && ctaRank == 0) {
       // descriptors differ only in their 14-bit start address: one constant upper half, the lower halves of the current stage
       const uint64_t descW0 = tc::smemDescSw128(base), descX0 = tc::smemDescSw128(base + xAt);
-      const uint32_t high = uint32_t(descW0 >> 32), stageStep = p.stageBytes >> 4;
+      const uint32_t high = uint32_t(descW0 >> 32), stageStep = stageBytes >> 4;
       auto desc = [&](uint32_t low) { return uint64_t(high) << 32 | low; };
       uint32_t st = 0, ph = 0, at = 0, use = 0, single = 0;    // at: offset of stage st; bit a of `use`: parity of the uses of accumulator a so far
       bool ok = true;
@@ -250,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
         };
         auto advance = [&]() {
           at += stageStep;
-          if (++st == uint32_t(p.stages)) { st = 0; at = 0; ph ^= 1; }
+          if (++st == stages) { st = 0; at = 0; ph ^= 1; }
         };
         auto complete = [&](int a) {                           // the epilogue may read accumulator a
           tc::mmaCommitPairs(tmemFullBar(a), pairMask);
@@ -404,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
           }
           tc::fenceBeforeThreadSync();
           __syncwarp();
-          if (lane == 0) tc::mbarArriveClusterTmem(leaderBars + 8u * (2u * uint32_t(p.stages) + 2u + uint32_t(a0 + b)));
+          if (lane == 0) tc::mbarArriveClusterTmem(leaderBars + 8u * (2u * uint32_t(kMaxStages) + 2u + uint32_t(a0 + b)));
         }
         if (!ok) return false;
 #pragma unroll

@@ -24,6 +24,7 @@ constexpr int kABytes = kBM * kBK * 2;
 constexpr int kAccRows = 256;                   // rows of W per accumulator of a pair; a tile has one or two of them
 constexpr int kMaxStages = 8, kRingBytes = 192 * 1024;
 constexpr int kXBox = 32;                       // rows of one X load
+constexpr int kNarrowCols = 64;                 // columns of a tile that leave room for a fifth stage
 }  // namespace ragged
 
 namespace route {
@@ -171,17 +172,16 @@ inline RaggedPlan raggedPlan(int M, int N, int K, bool swiglu, const int (&clust
 }
 
 struct RaggedCut {
-  int tileAccs, colTiles, maxCols, parts, stages;
-  uint32_t stageBytes;
+  int tileAccs, colTiles, maxCols, parts, stages, narrowStages;
+  uint32_t stageBytes, narrowStageBytes;
   int grid;        // CTAs
   bool apart;      // not set up while the kernel before it runs
 };
 // plan: of a GEMM of M rows; null: grouped, the tiles of each expert are known on the device. pairs: that the device holds.
-inline RaggedCut raggedCut(int M, int K, const RaggedPlan* plan, int likelyRows, int pairs, int sms) {
+inline RaggedCut raggedCut(int M, int K, const RaggedPlan* plan, int pairs, int sms) {
   RaggedCut c{};
   c.tileAccs = 2; c.colTiles = 1; c.parts = 1;
-  // (groups of a few dozen rows: narrow tiles leave room for a fifth stage)
-  c.maxCols = !plan && likelyRows <= 40 ? 64 : ragged::kMaxCols;
+  c.maxCols = ragged::kMaxCols;
   int items = INT32_MAX;
   if (plan) {
     c.tileAccs = plan->tileAccs; c.colTiles = plan->colTiles; c.parts = plan->parts;
@@ -189,6 +189,8 @@ inline RaggedCut raggedCut(int M, int K, const RaggedPlan* plan, int likelyRows,
     items = plan->parts > 1 ? plan->tiles : plan->tileAccs * plan->tiles;      // (the tiles of a small last wave are issued as halves)
   }
   c.stages = raggedStages(c.tileAccs, c.maxCols, c.stageBytes);
+  // (grouped, the kernel decides between wide and narrow tiles: it knows the counts)
+  c.narrowStages = raggedStages(c.tileAccs, std::min(c.maxCols, ragged::kNarrowCols), c.narrowStageBytes);
   c.grid = (c.parts > 1 ? items : std::min(pairs, items)) * 2 * c.parts;
   // (fewer tiles than pairs: the pairs without one leave at once; 2066 x 3144 x 4264, 63 tiles: 49.7 us apart, 58.0 overlapped)
   c.apart = betterApart(c.parts > 1 ? c.grid : items, K, sms);

@@ -920,8 +920,9 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   ragged::Params p{};
   p.N = N; p.K = K; p.tokens = M; p.counts = g.counts; p.experts = g.experts; p.C = static_cast<__nv_bfloat16*>(C); p.ldc = outCols;
   p.status = status; p.timeoutNs = g.timeoutNs;
-  const route::RaggedCut cut = route::raggedCut(M, K, plan, g.likelyRows, pairs, smCount());
+  const route::RaggedCut cut = route::raggedCut(M, K, plan, pairs, smCount());
   p.tileAccs = cut.tileAccs; p.colTiles = cut.colTiles; p.maxCols = cut.maxCols; p.parts = cut.parts; p.stages = cut.stages; p.stageBytes = cut.stageBytes;
+  p.narrowStages = cut.narrowStages; p.narrowStageBytes = cut.narrowStageBytes;
   ragged::Maps maps{};
   if (!cache.get(maps.w, B, uint64_t(N) * uint64_t(g.experts), uint64_t(K), ragged::kBM) ||
       !cache.get(maps.x, A, uint64_t(M), uint64_t(K), uint32_t(ragged::kXBox))) return 1;

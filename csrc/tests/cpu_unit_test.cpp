@@ -184,6 +184,12 @@ static void testSkinnyCut() {
   CHECK(route::skinnyCut(1, 8192, 3584, 1, 0, 148).ahead > 0, "few-rows GEMM: a lap of W is asked for while the kernel before drains");
 }
 
+static void testRaggedCut() {
+  const route::RaggedCut c = route::raggedCut(10240, 7168, nullptr, 74, 148);
+  CHECK(c.maxCols == ragged::kMaxCols && c.stages == 4, "grouped GEMM: an expert of many rows gets tiles of 256 columns, whatever the average is");
+  CHECK(c.narrowStages == 5 && c.narrowStages * int(c.narrowStageBytes) <= ragged::kRingBytes, "grouped GEMM: five stages where every expert has few rows");
+}
+
 int main() {
   testStaticFor();
   testPipelineDepth<1>();
@@ -193,6 +199,7 @@ int main() {
   testPipelineOrder();
   testPartition();
   testSkinnyCut();
+  testRaggedCut();
   std::printf("%s: %d failure(s)\n", g_failures ? "FAILED" : "PASSED", g_failures);
   return g_failures ? 1 : 0;
 }

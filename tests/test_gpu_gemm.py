@@ -326,3 +326,25 @@ def test_grouped_gemm_with_a_k_shorter_than_the_lead_of_an_accumulator(k, counts
     for e, c in enumerate(counts):
         assert torch.equal(out[at:at + c].float(), (a[at:at + c].float() @ w[e].float().t()).to(torch.bfloat16).float())
         at += c
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("counts", [[64, 1, 0, 64, 33, 32, 64], [64, 65, 64, 0, 1], [0, 0, 300, 1, 64], [257] + [31] * 40, [640] + [20] * 31, [16] * 70, [0, 0]])
+def test_grouped_gemm_of_few_rows_an_expert_and_of_one_that_has_many(counts, swiglu):
+    # tiles of 64 columns and a ring of more stages where that is few more tiles (an expert of 300 rows among many), of 256 otherwise
+    from purlin_b200.ops.gemm import grouped_gemm
+    n, k, rows = 1056, 1096, sum(counts) + 8
+    a, _ = _small_integers(rows, 8, k, 41)
+    w = torch.stack([_small_integers(8, n, k, 43 + e)[1] for e in range(len(counts))])
+    width = n // 2 if swiglu else n
+    out = torch.full((rows, width), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm(a, w, torch.tensor(counts, dtype=torch.int32, device="cuda"), 32, out, swiglu=swiglu)
+    at = 0
+    for e, c in enumerate(counts):
+        if swiglu:
+            ref = _swiglu_ref(a[at:at + c], w[e])
+            assert ((out[at:at + c].float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()      # one rounding to bf16
+        else:
+            assert torch.equal(out[at:at + c].float(), (a[at:at + c].float() @ w[e].float().t()).to(torch.bfloat16).float())
+        at += c
+    assert (out[at:] == 7).all()

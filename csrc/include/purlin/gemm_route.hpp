@@ -44,7 +44,7 @@ inline bool fewWeightRows(int M, int N, int K, bool swiglu) { return !swiglu && 
 inline bool useSkinny(int M, int N, int K, bool swiglu) {
   if (fewWeightRows(M, N, K, swiglu)) return true;
   // always up to 32 rows, up to 64 once k is long enough to be split: 64 x 4096 x 1024 7.9 / 8.3, 54 x 7648 x 1336 SwiGLU 14.3 / 17.2;
-  // but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4. Above, what the others would take decides (gemmRoute).
+  // but 64 x 104 x 144 5.6 / 3.8, 64 x 22968 x 72 9.2 / 6.4. Above, what the others would take decides (kernelOf).
   return M <= 64 && (M <= 32 || K >= (N <= 8192 ? 512 : 1024));
 }
 // Parts that the few-rows kernel cuts k into: while the CTAs have a place on the GPU at the same time and a part keeps at least four
@@ -125,8 +125,7 @@ inline int raggedStages(int accs, int cols, uint32_t& stageBytes) {
 //   the weights come through HBM once.
 // What it buys, us, one B200, before / now: 2048 x 14336 x 8192 SwiGLU 371 / 325 (ten column tiles, where eight left a fourth wave of two
 // tiles), 1000 x 14336 x 8192 SwiGLU 205 / 168, 1000 x 8192 x 7168 97 / 85, 384 x 14336 x 8192 SwiGLU 121 / 78, 700 x 8192 x 28672 428 / 250;
-// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58. Over 750 random
-// shapes the geometric mean is 1.09; 22 are slower by more than 3 %, the worst by 18 % (2006 x 64 x 1320 11.6 / 14.2).
+// with k split over two pairs 512 x 8192 x 28672 297 / 174, 384 x 8192 x 28672 224 / 142, 200 x 14336 x 8192 SwiGLU 70 / 58.
 struct RaggedPlan { int tileAccs = 2, colTiles = 1, tiles = 1, parts = 1; double cycles = 0; };
 inline RaggedPlan raggedPlan(int M, int N, int K, bool swiglu, const int (&clusters)[3]) {
   const int kBlocks = (K + ragged::kBK - 1) / ragged::kBK, units = (M + 31) / 32, fewest = (units + 7) / 8;
@@ -159,7 +158,8 @@ inline RaggedPlan raggedPlan(int M, int N, int K, bool swiglu, const int (&clust
       for (int parts = 1; parts <= kMaxParts; parts *= 2) {
         if (!clusters[parts / 2] || kBlocks < 8 * parts || (parts > 1 && tiles > clusters[parts / 2])) break;
         // Among cuts: a pair with few tiles has the widest among them, and narrow tiles move more bytes per operation, which costs power
-        // (2072 x 4800 x 5016 SwiGLU: 11 tiles of 192 88.7 us, 14 of 128 and 160 97.2).
+        // (2072 x 4800 x 5016 SwiGLU: 11 tiles of 192 88.7 us, 14 of 128 and 160 97.2). Between kernels the plain number of cycles chooses better
+        // (one factor for all K off a cache line, 914 shapes: 2.2 % above the best kernel of each; with this factor 2.5 %).
         const double key = cyclesOf(accs, average + (widest - average) * clusters[0] / std::max<int64_t>(tiles, clusters[0]), tiles, parts) * (0.95 + 12.8 / average);
         if (bestKey == 0 || key < bestKey) {
           bestKey = key;
@@ -203,18 +203,39 @@ inline double plainCycles(const PlainTiles& t, int M, int N, int K, bool swiglu,
   const double tiles = double(t.tilesM) * t.tilesN, places = t.ctas == 2 ? sms / 2 : sms;
   const double block = t.accs == 2 ? std::max(4. * t.bn, 900.) : std::max({2. * t.bn + 184., (ragged::kABytes + t.bn / t.ctas * 128) / 58., 700.});
   const double drain = t.accs == 2 ? (swiglu ? 9000. : 6000.) * t.bn / 256 : 0.;
-  const double waves = std::ceil(tiles / places), ragged = K % ragged::kBK ? 1.25 : 1.;      // rows of K that do not begin on a cache line
-  return std::max(waves * ((K + ragged::kBK - 1) / ragged::kBK * block * ragged + drain) + 3000., (2. * N * K + 2. * M * K) / 3300. * ragged);
+  const double waves = std::ceil(tiles / places);
+  // rows of K that do not begin on a cache line; or not even on a sector of 32 bytes, which costs least where W has few rows to load
+  const double unaligned = K % ragged::kBK == 0 ? 1. : K % 16 == 0 ? 1.1 : N > 128 ? 1.55 : 1.15;
+  return std::max(waves * ((K + ragged::kBK - 1) / ragged::kBK * block * unaligned + drain) + 3000., (2. * N * K + 2. * M * K) / 3300. * unaligned);
 }
 
-// ... and the few-rows kernel: its CTAs' round trips (per k-block 450 cycles and 3.5 per row, measured with L2-sized weights) or the
-// weights, and a fixed part that grows with the rows (the partial tiles through distributed shared memory).
+// ... and the few-rows kernel: its CTAs' round trips (per k-block 450 cycles and 3.5 per column, measured with L2-sized weights) and what
+// each CTA adds at its end, which grows with the rows (the partial tiles through distributed shared memory), or the weights. CTAs beyond
+// those that the device holds are a second wave: at one CTA an SM 33 clusters of four and 15 of eight fit (151 x 4568 x 2256, 36
+// clusters of four: 25 us, the ragged kernel 16).
 inline double skinnyCycles(int M, int N, int K, bool swiglu, int sms) {
   if (M > skinny::kMaxTokens || N > 16384) return 1e30;
-  const long tiles = (N + skinny::kRows - 1) / skinny::kRows, slots = long(sms) * (M <= 128 ? 2 : 1);
-  const int kBlocks = (K + skinny::kK - 1) / skinny::kK, split = skinnySplit(tiles, kBlocks, slots);
-  const double waves = std::ceil(double(tiles * split) / slots), block = (450. + 3.5 * M / skinnyGroups(M, tiles, split, kBlocks, sms)) * (tiles * split > sms ? 1.3 : 1.);
-  return std::max(waves * kBlocks / split * block, 1.15 * (2. * N * K + 2. * M * K) / 3300.) + 7000. + (swiglu ? 105. : 45.) * M;
+  const long tiles = (N + skinny::kRows - 1) / skinny::kRows;
+  const SkinnyCut c = skinnyCut(M, N, K, 1, 0, sms);
+  const int kBlocks = (K + skinny::kK - 1) / skinny::kK, width = (M + c.columnGroups - 1) / c.columnGroups;
+  const long places = long(c.split == 8 ? std::min(sms, 120) : c.split == 4 ? std::min(sms, 132) : sms) * (M <= 128 ? 2 : 1);
+  const double waves = std::ceil(double(tiles * c.split) / places), block = (450. + 3.5 * ((width + 31) / 32 * 32)) * (tiles * c.split > sms ? 1.3 : 1.);
+  const double end = (swiglu ? 105. : 45.) * M;
+  return std::max(waves * (double(kBlocks) / c.split * block + end), 1.15 * (2. * N * K + 2. * M * K) / 3300. + end) + 7000.;
+}
+
+// The least expected time. The ragged kernel was 3 % ahead of the plain tiles at 4096 x 8192 x 7168 (326 / 351 us) and 8192 x 2048 x 1024
+// (28.8 / 30.7), behind at 2048 x 4096 x 512 (13.8 / 12.1) and 1000 x 4096 x 4096 (36 / 33, one wave of narrower tiles); the few-rows
+// kernel ahead at 128 x 8192 x 8192 (33.6, ragged 37.5, plain 42.2), behind at 128 x 8192 x 2048 (18.2, plain 13.9) and 160 x 8192 x
+// 8192 (38.6, ragged 36.6). The models are not good to a few per cent, and for tiles of one accumulator the ragged one is more hopeful than
+// the plain one (by 8 % in the medians of measured over expected), so such a cut has to be expected ahead by 5 %. Of 914 random shapes, every
+// kernel timed on each, the choice then takes 1.6 % longer than the best kernel on average, and 14 are more than 3 % slower than by the
+// tile counts that decided before there was a model. Without that margin, with one factor for all K off a cache line and without the second
+// waves of the few-rows kernel it was 2.4 % and 41 (2006 x 64 x 1320 plain 12.4 us, ragged 16.5; 151 x 4568 x 2256 ragged 16, few rows 25).
+enum { kPlain = 0, kSkinny = 1, kRagged = 2 };
+inline int kernelOf(double plain, double skinny, double ragged, int tileAccs) {
+  if (tileAccs == 1) ragged *= 1.05;
+  return skinny < std::min(plain, ragged) ? kSkinny : ragged < plain ? kRagged : kPlain;
 }
 
 }  // namespace route

@@ -937,16 +937,12 @@ int launchRagged(MapCache& cache, const void* A, const void* B, void* C, int M, 
   return 0;
 }
 
-// Which kernel a GEMM takes, and its cut if it is the ragged one: the least expected time. The ragged kernel was 3 % ahead of the plain
-// tiles at 4096 x 8192 x 7168 (326 / 351 us) and 8192 x 2048 x 1024 (28.8 / 30.7), behind at 2048 x 4096 x 512 (13.8 / 12.1) and 1000 x 4096
-// x 4096 (36 / 33, one wave of narrower tiles); the few-rows kernel ahead at 128 x 8192 x 8192 (33.6, ragged 37.5, plain 42.2), behind at
-// 128 x 8192 x 2048 (18.2, plain 13.9) and 160 x 8192 x 8192 (38.6, ragged 36.6).
-enum { kRoutePlain = 0, kRouteSkinny = 1, kRouteRagged = 2 };
-struct Route { int M = 0, N = 0, K = 0, epilogue = 0, device = -1, kernel = kRoutePlain; route::RaggedPlan cut; };
+// Which kernel a GEMM takes, and its cut if it is the ragged one: gemm_route.hpp.
+struct Route { int M = 0, N = 0, K = 0, epilogue = 0, device = -1, kernel = route::kPlain; route::RaggedPlan cut; };
 Route findRoute(const Params& p, const Shape& sh, int epilogue) {
   Route r;
   const bool swiglu = epilogue == kEpiSwiglu;
-  if (route::useSkinny(p.M, p.N, p.K, swiglu)) { r.kernel = kRouteSkinny; return r; }
+  if (route::useSkinny(p.M, p.N, p.K, swiglu)) { r.kernel = route::kSkinny; return r; }
   const double plain = route::plainCycles(route::PlainTiles{p.tilesM, p.tilesN, p.bn, sh.ctas, sh.accs}, p.M, p.N, p.K, swiglu, smCount());
   const double skinny = p.M > 64 ? route::skinnyCycles(p.M, p.N, p.K, swiglu, smCount()) : 1e30;
   double ragged = 1e30;
@@ -954,7 +950,7 @@ Route findRoute(const Params& p, const Shape& sh, int epilogue) {
     const int clusters[3] = {raggedClusters(epilogue, 1), raggedClusters(epilogue, 2), raggedClusters(epilogue, 4)};
     if (clusters[0]) { r.cut = route::raggedPlan(p.M, p.N, p.K, swiglu, clusters); ragged = r.cut.cycles; }
   }
-  r.kernel = skinny < std::min(plain, ragged) ? kRouteSkinny : ragged < plain ? kRouteRagged : kRoutePlain;
+  r.kernel = route::kernelOf(plain, skinny, ragged, r.cut.tileAccs);
   return r;
 }
 // A function of the sizes (and of the device's cluster counts): each thread keeps those of its recent sizes, a microsecond of host time.
@@ -1011,9 +1007,9 @@ int purlin_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   if (!fillShape(p, sh, M, N, K, epilogue, bn, M)) return 1;
   static thread_local MapCache cache;
   if (bn == 0) {
-    const Route& route = gemmRoute(p, sh, epilogue);
-    if (route.kernel == kRouteSkinny) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
-    if (route.kernel == kRouteRagged) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, &route.cut, status, static_cast<cudaStream_t>(stream));
+    const Route& r = gemmRoute(p, sh, epilogue);
+    if (r.kernel == route::kSkinny) return launchSkinny(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, status, static_cast<cudaStream_t>(stream));
+    if (r.kernel == route::kRagged) return launchRagged(cache, A, B, C, M, N, K, epilogue, GroupedArgs{}, &r.cut, status, static_cast<cudaStream_t>(stream));
   }
   Maps maps{};
   if (!cache.get(maps.a, A, uint64_t(M), uint64_t(K), kBM) || !cache.get(maps.b, B, uint64_t(N), uint64_t(K), uint32_t(p.bn / sh.ctas)) ||

@@ -190,6 +190,21 @@ static void testRaggedCut() {
   CHECK(c.narrowStages == 5 && c.narrowStages * int(c.narrowStageBytes) <= ragged::kRingBytes, "grouped GEMM: five stages where every expert has few rows");
 }
 
+static void testKernelChoice() {
+  const int clusters[3] = {74, 33, 15};
+  auto choice = [&](int m, int n, int k, const route::PlainTiles& t) {
+    const route::RaggedPlan cut = route::raggedPlan(m, n, k, false, clusters);
+    return route::kernelOf(route::plainCycles(t, m, n, k, false, 148), route::skinnyCycles(m, n, k, false, 148), cut.cycles, cut.tileAccs);
+  };
+  // expected times closer than the models are to the truth
+  CHECK(choice(2006, 64, 1320, {16, 1, 256, 1, 1}) == route::kPlain && choice(5191, 88, 1696, {41, 1, 256, 1, 1}) == route::kPlain &&
+        choice(2533, 352, 1696, {20, 2, 256, 1, 1}) == route::kPlain, "the plain tiles stay where the ragged kernel is not expected ahead by the model's own error");
+  CHECK(choice(151, 4568, 2256, {2, 18, 256, 1, 1}) != route::kSkinny && choice(200, 4592, 3264, {2, 18, 256, 1, 1}) != route::kSkinny,
+        "few-rows GEMM: clusters that the device does not hold at once are a second wave");
+  CHECK(choice(1000, 14336, 8192, {8, 56, 256, 1, 1}) == route::kRagged && choice(128, 8192, 8192, {1, 32, 256, 1, 1}) == route::kSkinny,
+        "large differences decide as before");
+}
+
 int main() {
   testStaticFor();
   testPipelineDepth<1>();
@@ -200,6 +215,7 @@ int main() {
   testPartition();
   testSkinnyCut();
   testRaggedCut();
+  testKernelChoice();
   std::printf("%s: %d failure(s)\n", g_failures ? "FAILED" : "PASSED", g_failures);
   return g_failures ? 1 : 0;
 }

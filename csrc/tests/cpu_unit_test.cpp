@@ -187,6 +187,13 @@ static void testSkinnyCut() {
 static void testRaggedCut() {
   const route::RaggedCut c = route::raggedCut(10240, 7168, nullptr, 74, 148);
   CHECK(c.maxCols == ragged::kMaxCols && c.stages == 4, "grouped GEMM: an expert of many rows gets tiles of 256 columns, whatever the average is");
+  bool oneAccOverlapped = true, twoAccsByBusyCtas = true;
+  for (int tiles = 1; tiles <= 200; ++tiles) {
+    const route::RaggedPlan one{1, 1, tiles, 1, 0}, two{2, 1, tiles, 1, 0};
+    oneAccOverlapped = oneAccOverlapped && !route::raggedCut(256, 4096, &one, 74, 148).apart;
+    twoAccsByBusyCtas = twoAccsByBusyCtas && route::raggedCut(256, 4096, &two, 74, 148).apart == (2 * tiles > 74 && 2 * tiles < 127);
+  }
+  CHECK(oneAccOverlapped && twoAccsByBusyCtas, "ragged GEMM: launched apart by the CTAs that have a tile, with two accumulators alone");
   CHECK(c.narrowStages == 5 && c.narrowStages * int(c.narrowStageBytes) <= ragged::kRingBytes, "grouped GEMM: five stages where every expert has few rows");
 }
 

@@ -15,6 +15,7 @@
 #include "purlin/pipeline.hpp"
 #include "purlin/plan.hpp"
 #include "purlin/static_for.hpp"
+#include "purlin/tuning.hpp"
 
 using namespace purlin;
 
@@ -212,6 +213,31 @@ static void testKernelChoice() {
         "large differences decide as before");
 }
 
+// ---- the grid of a collective whose ranks share one GPU ----
+static CollectiveSpec allReduceSpec(int world, size_t bytes) {
+  CollectiveSpec s;
+  s.op = ConsumeOp::reduce;
+  s.world = world;
+  s.bytes = bytes;
+  return s;
+}
+static void testFitEmulated() {
+  // a ring of seven tiles and more leaves an SM one CTA, so the ranks' CTAs may not be more than the SMs
+  bool fits = true;
+  for (int world = 2; world <= 8; ++world)
+    for (int depth : {0, 2, 7, 8}) {
+      const CollectiveSpec s = allReduceSpec(world, 32 << 20);
+      const WorkspaceLayout ws = workspaceLayout(world, 64 << 20);
+      Policy p = defaultPolicy(s, ws);
+      p.stageDepth = depth;
+      fitEmulated(p, s, 148);
+      Plan plan;
+      std::string err;
+      fits = fits && buildPlan(s, p, ws, plan, err) && plan.blocks * world <= 148 * (depth == 0 && world > 4 ? 2 : 1);
+    }
+  CHECK(fits, "emulated grids: one CTA per SM where the bulk ring does not leave room for two");
+}
+
 int main() {
   testStaticFor();
   testPipelineDepth<1>();
@@ -223,6 +249,7 @@ int main() {
   testSkinnyCut();
   testRaggedCut();
   testKernelChoice();
+  testFitEmulated();
   std::printf("%s: %d failure(s)\n", g_failures ? "FAILED" : "PASSED", g_failures);
   return g_failures ? 1 : 0;
 }

@@ -138,6 +138,21 @@ def test_default_grids_fit_and_ranks_travel_with_the_launch(worlds, world):
         run_case(ew, A2AV, sizes=[_sizes(world, 60 + r, scale=scale, zero_every=4) for r in range(world)], dtype=0, pol=None)
 
 
+@pytest.mark.parametrize("world", [5, 7, 8])
+def test_a_measured_band_with_a_deep_ring_fits_on_one_gpu(worlds, world):
+    # a ring of eight tiles is 128 KiB of shared memory: one CTA per SM, where the built-in policy of so many ranks counts on two
+    import ctypes
+    from purlin_b200 import _native
+    lib = _native.cuda()
+    band = policy(arPath=1, stageDepth=8, chunkBytes=0)
+    lib.purlin_tuning_clear()
+    try:
+        _native.check(lib, lib.purlin_tuning_add(AR, world, 64 << 20, ctypes.byref(band)))
+        run_case(worlds(world, 4 << 20), AR, nbytes=3 << 20, dtype=0, pol=None)
+    finally:
+        lib.purlin_tuning_clear()
+
+
 def test_absent_rank_times_out_and_context_recovers():
     # A rank that never launches: the others' bounded waits give up, the host reads a status, and after
     # clearing it the same contexts run a correct collective. Nothing traps, faults or spins forever.

@@ -184,7 +184,7 @@ inline Policy selectPolicy(const CollectiveSpec& s, const WorkspaceLayout& ws) {
 // reducer has half of a copier's (8 x 16 against 8 x 32 bytes a thread), so its bytes count twice: 64 MiB by 4 ranks 352 -> 261 us, reduce-
 // scatter 4 x 16 MiB 205 -> 162. Where the streams alone take most CTAs of a rank (8 ranks: 15 of 18), CTAs of 128 threads, two on an SM,
 // leave the reducers their part: all-reduce of 64 MiB by 8 ranks 827 -> 485, reduce-scatter 8 x 8 MiB 394 -> 322.
-inline void fitEmulated(Policy& p, const CollectiveSpec& s, int sms) {
+inline void fitEmulated(Policy& p, const CollectiveSpec& s, const WorkspaceLayout& ws, int sms) {
   const int W = s.world;
   // (a bulk ring of seven tiles or more leaves an SM one CTA: measured bands with a ring keep one)
   const bool small = s.op == ConsumeOp::reduce && W > 4 && W <= 8 && p.regime == int32_t(Regime::throughput) && p.stageDepth == 0;
@@ -213,8 +213,12 @@ inline void fitEmulated(Policy& p, const CollectiveSpec& s, int sms) {
     const int uneven = n[0] % least[0];
     n[0] -= uneven; n[2] += uneven;
   }
-  // few and large chunks once there are enough of them: a chunk costs every stream a barrier and a flag
-  if (composed && p.chunkBytes && s.bytes >= (12ull << 20)) p.chunkBytes = std::max<uint64_t>(p.chunkBytes, 4ull << 20);
+  // Few and large chunks once there are enough of them: a chunk costs every stream a barrier and a flag. A payload larger than the staging
+  // half streams through windows of it, where a large chunk must leave room for others in flight (48 MiB, us, large / as chosen: 4 ranks, one in a window
+  // 491 / 331, two 303 / 328; 8 ranks, one 814 / 419, two 503 / 466, three 431 / 437; 3 ranks, two 264 / 273, 5 ranks, four 324 / 382). One that no
+  // window holds is cut into quarters of a window by the plan (3 ranks, staging of 4 MiB: 299 / 521).
+  const uint64_t large = 4ull << 20, inWindow = roundDown(ws.stagingTRSize / uint64_t(W), uint64_t(kAccessAlign)) / roundUp(large / uint64_t(W), uint64_t(kAccessAlign));
+  if (composed && p.chunkBytes && s.bytes >= (12ull << 20) && (s.bytes <= ws.stagingTRSize || inWindow == 0 || inWindow >= (W <= 4 ? 2u : 3u))) p.chunkBytes = std::max<uint64_t>(p.chunkBytes, large);
   p.putBlocks = n[0]; p.localBlocks = std::max(n[1], 1); p.consumeBlocks = n[2]; p.gatherBlocks = std::max(n[3], 1);
 }
 

@@ -445,7 +445,7 @@ int purlin_emu_collective(PurlinHostContext* const* ctxs, int world, int collect
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctxs[r]->device);
       fitted = selectPolicy(spec, ctxs[r]->ws);
-      fitEmulated(fitted, spec, sms);
+      fitEmulated(fitted, spec, ctxs[r]->ws, sms);
       use = &fitted;
     }
     if (!planFor(spec, ctxs[r]->ws, use, host[r].plan, nullptr)) return 1;

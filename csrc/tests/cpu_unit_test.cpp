@@ -230,11 +230,28 @@ static void testFitEmulated() {
       const WorkspaceLayout ws = workspaceLayout(world, 64 << 20);
       Policy p = defaultPolicy(s, ws);
       p.stageDepth = depth;
-      fitEmulated(p, s, 148);
+      fitEmulated(p, s, ws, 148);
       Plan plan;
       std::string err;
       fits = fits && buildPlan(s, p, ws, plan, err) && plan.blocks * world <= 148 * (depth == 0 && world > 4 ? 2 : 1);
     }
+  // an all-reduce larger than its staging streams through windows of it: chunks made larger may not fill a window, or nothing overlaps
+  bool pipelined = true, large = true;
+  for (int world : {3, 4, 5, 8})
+    for (int mib : {1, 2, 3, 4, 6, 7, 8, 12, 16, 24, 64}) {
+      const CollectiveSpec s = allReduceSpec(world, 48 << 20);
+      const WorkspaceLayout ws = workspaceLayout(world, size_t(mib) << 20);
+      Policy p = defaultPolicy(s, ws);
+      const uint64_t chosen = p.chunkBytes;
+      fitEmulated(p, s, ws, 148);
+      Plan plan;
+      std::string err;
+      uint32_t slots = buildPlan(s, p, ws, plan, err) ? ~0u : 0u;
+      for (int i = 0; i < plan.nSteps; ++i) if (plan.steps[i].chunks > 1) slots = std::min(slots, plan.steps[i].slots);
+      pipelined = pipelined && (p.chunkBytes == chosen || slots >= 2);
+      if (mib == 64) large = large && p.chunkBytes >= (4ull << 20);
+    }
+  CHECK(pipelined && large, "emulated all-reduce: chunks are made larger only where others stay in flight beside them");
   CHECK(fits, "emulated grids: one CTA per SM where the bulk ring does not leave room for two");
 }
 

@@ -138,6 +138,15 @@ def test_default_grids_fit_and_ranks_travel_with_the_launch(worlds, world):
         run_case(ew, A2AV, sizes=[_sizes(world, 60 + r, scale=scale, zero_every=4) for r in range(world)], dtype=0, pol=None)
 
 
+@pytest.mark.parametrize("world", [3, 4, 5, 7, 8])
+def test_default_reductions_of_uneven_worlds_and_of_large_payloads(worlds, world):
+    # an odd number of 32-byte units, resident (one flag a stream, chunks) and through windows of the staging half
+    for staging, n in ((16 << 20, 5 * (1 << 20) + 32), (16 << 20, 13 * (1 << 20) + 32), (4 << 20, 13 * (1 << 20) + 32)):
+        run_case(worlds(world, staging), AR, nbytes=n, dtype=0, pol=None)
+    for n in (1 << 20, 3 * (1 << 20) + 32):
+        run_case(worlds(world, 32 << 20), RS, nbytes=n, dtype=4, pol=None, reps=1)
+
+
 @pytest.mark.parametrize("world", [5, 7, 8])
 def test_a_measured_band_with_a_deep_ring_fits_on_one_gpu(worlds, world):
     # a ring of eight tiles is 128 KiB of shared memory: one CTA per SM, where the built-in policy of so many ranks counts on two

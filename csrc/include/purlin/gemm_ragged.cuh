@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) raggedGemmKernel(const __grid_con
   }
   if (SPLIT && warp < 2) { agree(*abortWord == 0); __syncwarp(); tc::clusterSync(); }      // the two barriers of the exchange
 
-  if (*abortWord) __nanosleep(20000);   // let copies already in flight land before shared memory and TMEM go away
+  if (*abortWord) tc::landingPause();   // copies already in flight land before shared memory and TMEM go away
   __syncwarp();
   tc::fenceBeforeThreadSync();
   tc::clusterSync();                    // neither CTA frees TMEM the pair's MMA still writes

@@ -61,6 +61,13 @@ PURLIN_D void mbarDrain(uint32_t bar, uint32_t parity) {
   while (!mbarTryWait(bar, parity) && sig::globalTimerNs() - start < 1000ull * 1000 * 1000) {}
 }
 
+// The same where copies are credited to the other CTA's barriers, whose phases they need not complete: a pause far longer than a copy or an
+// MMA takes (a few microseconds). By the clock, because a sleep may end at once.
+PURLIN_D void landingPause() {
+  const uint64_t start = sig::globalTimerNs();
+  while (sig::globalTimerNs() - start < 200ull * 1000) __nanosleep(2000);
+}
+
 // ---- TMA (tile mode, this CTA only) ----
 PURLIN_D void tmaLoad2d(uint32_t smemDst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -609,7 +609,7 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
   }
 
   // ------------------------------- teardown -------------------------------
-  if (*abortWord) __nanosleep(20000);   // let copies already in flight land before shared memory and TMEM go away
+  if (*abortWord) tc::landingPause();   // copies already in flight land before shared memory and TMEM go away
   tc::fenceBeforeThreadSync();
   if constexpr (CTAS == 2) tc::clusterSync(); else __syncthreads();   // neither CTA frees TMEM the pair's MMA still writes
   if (warp == 1) {

@@ -216,6 +216,28 @@ def test_a_wait_that_runs_out_reports_and_leaves_no_half_sums(swiglu):
     assert status[0].item() == 0 and torch.equal(out.float(), ref)
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_a_wait_that_runs_out_in_the_kernel_of_many_rows_an_expert_reports(swiglu):
+    # the same on CTA pairs (more than a dozen rows an expert): a row is the product or untouched, and the next call is whole
+    from purlin_b200.ops.gemm import grouped_gemm
+    rows, n, k = 16, 64, 1 << 21
+    a = torch.zeros(rows, k, device="cuda", dtype=torch.bfloat16)
+    a[:, ::4096] = 1
+    w = torch.full((1, n, k), 0.125, device="cuda", dtype=torch.bfloat16)
+    counts = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    width = n // 2 if swiglu else n
+    ref = torch.full((rows, width), 64.0 * 64.0 if swiglu else 64.0, device="cuda")      # 512 ones x 0.125; silu(64) = 64 in fp32
+    out = torch.full((rows, width), 7.0, device="cuda", dtype=torch.bfloat16)
+    grouped_gemm(a, w, counts, rows, out, swiglu=swiglu, status_ptr=status.data_ptr(), timeout_ns=1)
+    torch.cuda.synchronize()
+    assert status[0].item() == 5 and status[1].item() in (1, 2, 3, 5)
+    assert ((out == 7) | (out.float() == ref)).all()
+    status.zero_()
+    grouped_gemm(a, w, counts, rows, out, swiglu=swiglu, status_ptr=status.data_ptr())
+    assert status[0].item() == 0 and torch.equal(out.float(), ref)
+
+
 def _swiglu_ref(a, w):
     v = (a.float() @ w.float().t()).view(a.shape[0], w.shape[0] // 32, 2, 16)
     return (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(a.shape[0], w.shape[0] // 2)

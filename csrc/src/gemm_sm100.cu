@@ -560,7 +560,8 @@ gemmKernel(const __grid_constant__ Maps maps, const __grid_constant__ Params p) 
       tc::fenceBeforeThreadSync();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (CTAS == 2) tc::mbarArriveCluster(leaderBars + 8u * (2 * p.stages + 2 + a));
+        if constexpr (CTAS == 2 && COMM == kCommNone) tc::mbarArriveClusterTmem(leaderBars + 8u * (2 * p.stages + 2 + a));
+        else if constexpr (CTAS == 2) tc::mbarArriveCluster(leaderBars + 8u * (2 * p.stages + 2 + a));
         else tc::mbarArrive(tmemEmptyBar(a));
       }
       if constexpr (COMM == kCommRS) {

@@ -19,8 +19,9 @@
 //     every tile, and the release then waited about 2000 more for the stores; now 800 (plain) and 2500 (SwiGLU, bound by its
 //     exponentials and divisions) per accumulator. The main loop runs at the tensor pipe's rate, 1024 cycles per k-block;
 //   * what is left of the epilogue is hidden by moving the accumulators against each other (kLead).
-// One B200, before / now in turn, us (all of it under the power cap): 32 experts of 1024 rows, 4096 x 7168 SwiGLU 1623 / 1494,
-// 7168 x 2048 944 / 752; 8190 x 7168 x 2048 212 / 172, 1000 x 14336 x 8192 SwiGLU 209 / 203.
+// One B200, us, with the epilogue before this one / with it, and the cut unchanged (all of it under the power cap): 32 experts of 1024 rows, 4096 x 7168 SwiGLU 1623 / 1494,
+// 7168 x 2048 944 / 752; 8190 x 7168 x 2048 212 / 172,
+// 1000 x 14336 x 8192 SwiGLU 209 / 203 (168 with the cuts of gemm_route.hpp).
 #pragma once
 #include "gemm_skinny.cuh"
 

@@ -32,7 +32,7 @@ struct Params {
   int columnGroups;        // without counts: this many CTAs share a tile's columns, a pass each (blockIdx.y)
   int tokenBox;            // rows of one X load: 16 or 32
   int stages, tmemCols;
-  int ahead;               // k-blocks of W that are asked into L2 while the kernel before this one drains (0 where it has ended)
+  int ahead;               // k-blocks of W that are asked into L2 while the kernel before this one drains (0 where it has ended, and with counts)
   const int32_t* counts;   // rows per expert, or null: one group of `tokens` rows
   __nv_bfloat16* C;
   int ldc;
